@@ -31,6 +31,7 @@ struct tcv_ctx {
     void* c_scratch = nullptr;
     tcv_plan* plan = nullptr;
     tcv_tuning tuning{16, 32, 0, 0};
+    bool tuned = false;  // a tuning was set: without one the plan picks its work units itself
     bool initialized = false;
     std::string err;
 };
@@ -135,7 +136,9 @@ tcv_status rebuild_plan(tcv_ctx* c)
         tcv_plan_destroy(c->plan);
         c->plan = nullptr;
     }
-    const size_t need = tcv_plan_workspace_bytes_tuned(c->n_data, c->support, c->cfg.g_size, c->c_len, &c->tuning);
+    const tcv_tuning* tuning = c->tuned ? &c->tuning : nullptr;
+    const size_t need = tuning ? tcv_plan_workspace_bytes_tuned(c->n_data, c->support, c->cfg.g_size, c->c_len, tuning)
+                               : tcv_plan_workspace_bytes(c->n_data, c->support, c->cfg.g_size, c->c_len);
     if (need > c->work_bytes) {
         CTX_CUDA(c, cudaStreamSynchronize(c->stream));
         cudaFree(c->work);
@@ -145,7 +148,8 @@ tcv_status rebuild_plan(tcv_ctx* c)
         c->work_bytes = need;
     }
     CTX_TRY(c, tcv_plan_build_tuned(&c->plan, c->iu, c->iv, c->coff, c->n_data, c->support, c->cfg.g_size,
-                                    c->c_len, &c->tuning, c->work, c->work_bytes, c->stream));
+                                    c->c_len, tuning, c->work, c->work_bytes, c->stream));
+    if (!tuning) CTX_TRY(c, tcv_plan_tuning(c->plan, &c->tuning));
     int64_t rej = 0;
     CTX_TRY(c, tcv_plan_rejected(c->plan, &rej, c->stream));
     if (rej > 0) {
@@ -335,12 +339,15 @@ tcv_status tcv_set_tuning(tcv_ctx* c, const tcv_tuning* t)
         nt.degrid_split < 0 || nt.kernel < 0 || nt.kernel > 3 || (nt.kernel != 0 && nt.tile_rows != 8))
         return TCV_ERR_ARG;
     const tcv_tuning prev = c->tuning;
+    const bool was_tuned = c->tuned;
     c->tuning = nt;
+    c->tuned = true;
     if (!c->initialized) return TCV_OK;
     tcv_status s = ensure_tables(c);
     if (s == TCV_OK) s = rebuild_plan(c);
     if (s != TCV_OK && s != TCV_ERR_BOUNDS) {
         c->tuning = prev;
+        c->tuned = was_tuned;
         rebuild_plan(c);
     }
     return s;

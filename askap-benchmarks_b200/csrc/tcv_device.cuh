@@ -456,13 +456,17 @@ degrid_tile_kernel(const typename Tab::elem* __restrict__ ctab,
 // that were not split are skipped.
 template <int kR>
 __global__ void __launch_bounds__(kTileThreads)
-fold_kernel(const u32* __restrict__ items, const u32* __restrict__ group_start, const u32* __restrict__ nunits,
-            const u32* __restrict__ pstart, GridArgs a)
+fold_kernel(const u32* __restrict__ items, const u32* __restrict__ group_start,
+            const u32* __restrict__ group_ustart, const u32* __restrict__ nunits, const u32* __restrict__ pstart,
+            GridArgs a)
 {
     constexpr int kTH = tile_height(kR);
     constexpr int kPoints = kTileW * kTH;
     constexpr u32 kSlices = kPoints / kTileThreads;
     const u32 i0 = group_start[a.group], i1 = group_start[a.group + 1];
+    // as many units as non-empty cells: no cell of the group was split, so nothing is walked
+    // (60 k samples of a 129^2 footprint, 8 groups, none split: 10 us a launch walking the cells)
+    if (group_ustart[a.group + 1] - group_ustart[a.group] == i1 - i0) return;
     for (u32 w = blockIdx.x; w < (i1 - i0) * kSlices; w += gridDim.x) {
         const u32 k = i0 + w / kSlices;
         const u32 nu = nunits[k];

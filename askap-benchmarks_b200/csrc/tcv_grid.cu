@@ -70,7 +70,8 @@ tcv_status launch(const tcv_plan* p, const float2* data, const void* c, float c_
         TCV_CUDA(cudaLaunchKernel(kernel, dim3(ctas), dim3(kTileThreads), args, 0, st));
         if (g.split) {
             // the split cells' partial tiles into the grid, before the next group touches it
-            fold_kernel<kR><<<fold_ctas(), kTileThreads, 0, st>>>(p->items, p->group_start, p->nunits, p->pstart, a);
+            fold_kernel<kR><<<fold_ctas(), kTileThreads, 0, st>>>(p->items, p->group_start, p->group_ustart, p->nunits,
+                                                                  p->pstart, a);
             TCV_CUDA(cudaGetLastError());
         }
     }
@@ -107,7 +108,8 @@ tcv_status launch_adjoint(const tcv_plan* p, const float2* grid, const void* c, 
 
 tcv_status launch_fold8(const tcv_plan* p, const GridArgs& a, cudaStream_t st)
 {
-    fold_kernel<8><<<fold_ctas(), kTileThreads, 0, st>>>(p->items, p->group_start, p->nunits, p->pstart, a);
+    fold_kernel<8><<<fold_ctas(), kTileThreads, 0, st>>>(p->items, p->group_start, p->group_ustart, p->nunits,
+                                                         p->pstart, a);
     TCV_CUDA(cudaGetLastError());
     return TCV_OK;
 }

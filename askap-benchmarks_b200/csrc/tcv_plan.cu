@@ -779,6 +779,8 @@ bool geom_supported(const PlanGeom& g)
 // Degridding anchor tiles are the largest ta whose staged region (ta + sSize - 1)^2 complex
 // points fits in shared memory next to the partial sums; beyond that the direct kernel reads
 // the grid from global memory.
+void default_units(PlanGeom& g);
+
 PlanGeom make_geom(int64_t n, int support, const int* g_sizes, int n_jobs, int64_t c_len, const tcv_tuning* t,
                    bool anchors)
 {
@@ -847,7 +849,37 @@ PlanGeom make_geom(int64_t n, int support, const int* g_sizes, int n_jobs, int64
         g.akey_bits = g.atile_bits + 1;
     }
     g.key64 = g.key_bits > 32 || (g.anchors && g.akey_bits > 32);
+    if (!t && g.anchors) default_units(g);
     return g;
+}
+
+// Work units of a plan without a tuning.  Where the samples lie is not known on the host, and
+// samples that crowd into a few tiles leave most SMs idle with cells whole (16 k samples of a 45^2
+// footprint meet ~25 tiles of 64 x 64: gridding 0.71 ms whole, 0.074-0.080 ms in units of 32-64
+// samples; 60 k samples of 29^2 within 150^2 points: 7.2 and 0.12 ms), while samples spread over
+// many tiles are not split by a rule that aims at the device: about four units per SM slot of four
+// CTAs (2368), in whole powers of two.  Below 32 samples a unit's tile write costs more than its
+// work; above 512 no measured problem gained.  Degridding units need no partial tile, so they are
+// half as large (37 k samples of 65^2: 0.147 ms with 64, 0.140 ms with 32, 0.82 ms whole).
+// The partial tiles never push a plan past kUnitsBytes that would fit without them: that is the
+// scratch of the allocation-free entry, which takes every problem it took with cells whole.
+void default_units(PlanGeom& g)
+{
+    constexpr size_t kUnitsBytes = size_t(64) << 20;
+    const double reach = (double(g.s + g.tw - 1) / g.tw) * (double(g.s + g.th - 1) / g.th);
+    const double pairs = double(g.n) * reach;  // mean tiles of a footprint
+    auto size = [&](double units, int most) {
+        int u = 32;
+        while (u < most && double(u) * units < pairs) u *= 2;
+        return u;
+    };
+    const bool small = plan_bytes(g, nullptr) <= kUnitsBytes;
+    auto fits = [&] { return !small || plan_bytes(g, nullptr) <= kUnitsBytes; };
+    g.dsplit = size(2 * 2368.0, 128);
+    if (!fits()) g.dsplit = 0;
+    for (g.split = size(2368.0, 512); g.split <= 512; g.split *= 2)
+        if (fits()) return;
+    g.split = 0;
 }
 
 size_t plan_bytes(const PlanGeom& g, size_t* cub_bytes_out)
