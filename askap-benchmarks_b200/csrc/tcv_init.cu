@@ -41,18 +41,22 @@ struct CParams {
     int64_t n;
 };
 
-// One thread per table entry: Benchmark.cc:236-258 in FP64, stored as float (imaginary part 0).
+// Benchmark.cc:236-258 in FP64, stored as float (imaginary part 0).  One thread per entry of the
+// planes w >= 0: plane -w has the same |w|, so the same values, and the thread stores them there
+// too (half the double-precision cosines, which bound this kernel: 378 -> 204 us at 33 planes of
+// 64 x 129^2 entries).
 __global__ void init_c_kernel(CParams p, float2* c)
 {
+    const int64_t per_plane = int64_t(p.s) * p.s * p.os * p.os;
     const int64_t cind = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (cind >= p.n) return;
+    if (cind >= per_plane * (p.w_size / 2 + 1)) return;
     int64_t t = cind;
     const int i = int(t % p.s); t /= p.s;
     const int j = int(t % p.s); t /= p.s;
     const int osi = int(t % p.os); t /= p.os;
     const int osj = int(t % p.os); t /= p.os;
-    const int k = int(t);
-    const double w = (double)(k - p.w_size / 2);
+    const int above = p.w_size / 2 + int(t), below = p.w_size / 2 - int(t);
+    const double w = (double)int(t);
     const double f_scale = __ddiv_rn(sqrt(__dmul_rn(__dmul_rn(fabs(w), p.w_cell_size), p.freq0)), p.cell_size);
     const double os = (double)p.os;
     const double dj = __dadd_rn((double)(j - p.c_center), __ddiv_rn((double)osj, os));
@@ -60,10 +64,13 @@ __global__ void init_c_kernel(CParams p, float2* c)
     const double r2 = __dadd_rn(__dmul_rn(dj, dj), __dmul_rn(di, di));
     double val;
     if (w != 0.0)
-        val = cos(__ddiv_rn(r2, __dmul_rn(w, f_scale)));
+        val = cos(__ddiv_rn(r2, __dmul_rn(w, f_scale)));  // cos is even: also plane -w's value
     else
         val = exp(-r2);
-    c[cind] = make_float2((float)val, 0.0f);
+    const int64_t in_plane = cind - t * per_plane;
+    const float2 z = make_float2((float)val, 0.0f);
+    if (above < p.w_size) c[above * per_plane + in_plane] = z;
+    if (below != above) c[below * per_plane + in_plane] = z;
 }
 
 __device__ __forceinline__ float cabs_ref(float2 z)
@@ -72,33 +79,252 @@ __device__ __forceinline__ float cabs_ref(float2 z)
     return z.y == 0.0f ? fabsf(z.x) : hypotf(z.x, z.y);
 }
 
+// ------------------------------------------------------------------------------------------
 // The reference normalises with a sequential float sum of |C| over the flat table
-// (Benchmark.cc:261-265).  The order of a float sum decides its value (it saturates at 2^24
-// for the default 35 M entry table), so one thread adds the values in index order while the
-// rest of the block stages the next chunk in shared memory.
-constexpr int kSumChunk = 4096;
-__global__ void __launch_bounds__(1024) sum_abs_seq_kernel(const float2* c, int64_t n, float* out)
+// (Benchmark.cc:261-265).  The order of a float sum decides its value (it saturates at 2^24 for
+// the default 35 M entry table), and one thread adding in that order took 117.6 ms there.  The
+// same value in parallel: while the sum s = m * u stays in one binade (u its last place, m in
+// [2^23, 2^24)), adding x >= 0 takes m to m + round(x / u) whatever m is, except that a tie is
+// rounded by the parity of m + floor(x / u).  So an entry is a pair of whole-number increments,
+// for an even and an odd m (Inc2), a run of entries composes into one such pair, and composition
+// is associative: it can be summed in any grouping.  Where m would reach 2^24 the binade ends:
+// the entries around that place are added one by one in float, and the sum goes on with the next
+// binade's u.
+//   sum_blocks_kernel   per block of entries, its sum in double (an estimate of where s stands)
+//   sum_incs_kernel     per block, its increments for the two binades s may be in there
+//   sum_walk_kernel     one CTA walks the blocks, 1024 composed at a time; a block in which the
+//                       binade ends, or whose two binades do not hold s, is walked entry by entry
+// Both block kernels read the table once (281 MB at the default size: bandwidth); the walk is a
+// chain of ~25 binades of a few microseconds.  117.6 -> 0.25 ms at the default size.
+// ------------------------------------------------------------------------------------------
+constexpr int kSumChunk = 4096;       // entries a CTA of the block kernels handles per round
+constexpr int kSumMaxBlocks = 4096;
+constexpr unsigned kIncCap = 1u << 26;  // increments from 2^24 on only say "the binade ends"
+
+struct Inc2 {
+    unsigned even, odd;  // increment of m from an even and from an odd m
+};
+
+struct SumBlocks {
+    int64_t n, per;  // entries, entries per block (a multiple of kSumChunk)
+    int nb;
+    double* sum;     // per block
+    Inc2* incs;      // per block: increments at exponent exps[b], then at exps[b] + 1
+    int* exps;
+};
+
+__device__ __forceinline__ Inc2 inc_then(const Inc2 a, const Inc2 b)  // a's entries, then b's
 {
-    __shared__ float buf[2][kSumChunk];
-    const int64_t nchunks = (n + kSumChunk - 1) / kSumChunk;
-    for (int i = threadIdx.x; i < kSumChunk && i < n; i += blockDim.x) buf[0][i] = cabs_ref(c[i]);
+    return Inc2{min(kIncCap, a.even + ((a.even & 1u) ? b.odd : b.even)),
+                min(kIncCap, a.odd + ((a.odd & 1u) ? b.even : b.odd))};
+}
+
+__device__ __forceinline__ Inc2 inc_of(float x, float per_u)  // per_u = 1 / u, a power of two
+{
+    const float q = fminf(x * per_u, float(kIncCap)), f = floorf(q), r = q - f;
+    const unsigned n = unsigned(f);
+    const unsigned up = r > 0.5f, tie = r == 0.5f;
+    return Inc2{n + (up | (tie & n)), n + (up | (tie & ~n & 1u))};
+}
+
+__device__ __forceinline__ int exponent_of(float s) { return int((__float_as_uint(s) >> 23) & 0xffu) - 127; }
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float(unsigned(e + 127) << 23); }
+
+// inclusive scan over the warp's lanes in lane order
+__device__ __forceinline__ Inc2 inc_warp_scan(Inc2 v, int lane)
+{
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const Inc2 o{__shfl_up_sync(0xffffffffu, v.even, d), __shfl_up_sync(0xffffffffu, v.odd, d)};
+        if (lane >= d) v = inc_then(o, v);
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(256) sum_blocks_kernel(const float2* __restrict__ c, SumBlocks b)
+{
+    __shared__ double ws[8];
+    const int64_t lo = b.per * blockIdx.x, hi = min(b.n, lo + b.per);
+    double s = 0.0;
+    for (int64_t i = lo + threadIdx.x; i < hi; i += 256) s += double(cabs_ref(c[i]));
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
-    float sum = 0.0f;
-    for (int64_t ch = 0; ch < nchunks; ++ch) {
-        const int cur = int(ch & 1);
-        if (threadIdx.x >= 32) {
-            const int64_t base = (ch + 1) * kSumChunk;
-            for (int i = threadIdx.x - 32; i < kSumChunk && base + i < n; i += blockDim.x - 32)
-                buf[cur ^ 1][i] = cabs_ref(c[base + i]);
-        } else if (threadIdx.x == 0) {
-            const int64_t base = ch * kSumChunk;
-            const int len = int(n - base < kSumChunk ? n - base : kSumChunk);
-            const float* b = buf[cur];
-            for (int i = 0; i < len; ++i) sum = __fadd_rn(sum, b[i]);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) s += ws[w];
+        b.sum[blockIdx.x] = s;
+    }
+}
+
+__global__ void __launch_bounds__(256) sum_incs_kernel(const float2* __restrict__ c, SumBlocks b)
+{
+    __shared__ double ws[8];
+    __shared__ Inc2 wi[2][8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the sum before this block, as the double sums have it; the float sum lags or leads it by its
+    // accumulated roundings, so the binade is taken from a little below
+    double s = 0.0;
+    for (int k = threadIdx.x; k < int(blockIdx.x); k += 256) s += b.sum[k];
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) ws[warp] = s;
+    __syncthreads();
+    s = 0.0;
+    for (int w = 0; w < 8; ++w) s += ws[w];
+    const int e = max(-64, min(100, exponent_of(float(0.9 * s))));
+    const float q0 = pow2f(23 - e), q1 = pow2f(22 - e);
+    Inc2 t0{0, 0}, t1{0, 0};  // thread 0: of the block so far
+    const int64_t lo = b.per * blockIdx.x, hi = min(b.n, lo + b.per);
+    for (int64_t base = lo; base < hi; base += kSumChunk) {
+        constexpr int kPer = kSumChunk / 256;  // consecutive entries per thread
+        const int64_t at = base + int64_t(threadIdx.x) * kPer;
+        Inc2 v0{0, 0}, v1{0, 0};
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (at + k >= hi) break;
+            const float x = cabs_ref(c[at + k]);
+            v0 = inc_then(v0, inc_of(x, q0));
+            v1 = inc_then(v1, inc_of(x, q1));
+        }
+        v0 = inc_warp_scan(v0, lane);
+        v1 = inc_warp_scan(v1, lane);
+        __syncthreads();  // thread 0 is done with the last round's warps
+        if (lane == 31) {
+            wi[0][warp] = v0;
+            wi[1][warp] = v1;
         }
         __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < 8; ++w) {
+                t0 = inc_then(t0, wi[0][w]);
+                t1 = inc_then(t1, wi[1][w]);
+            }
     }
-    if (threadIdx.x == 0) out[0] = sum;
+    if (threadIdx.x == 0) {
+        b.exps[blockIdx.x] = e;
+        b.incs[2 * blockIdx.x] = t0;
+        b.incs[2 * blockIdx.x + 1] = t1;
+    }
+}
+
+constexpr int kWalkThreads = 1024;
+constexpr float kSumTiny = 1e-18f;  // below this the entries are added one by one
+
+struct WalkShared {
+    Inc2 warp[kWalkThreads / 32];
+    unsigned first;  // first thread whose part the binade ends in
+    float s;         // the sum so far
+};
+
+// Add the threads' parts (inc each, in thread order) to sh.s as far as the binade reaches: returns
+// the first thread whose part was not added (kWalkThreads: none), and with m_out that thread's m
+// at its part's start (all threads get their own).
+__device__ unsigned walk_parts(WalkShared& sh, Inc2 inc, bool stop, unsigned m, float u, unsigned& m_out)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Inc2 in = inc_warp_scan(inc, lane);
+    if (lane == 31) sh.warp[warp] = in;
+    if (threadIdx.x == 0) sh.first = kWalkThreads;
+    __syncthreads();
+    Inc2 pre{0, 0};
+    if (warp == 0) {
+        const Inc2 w = inc_warp_scan(sh.warp[lane], lane);
+        __syncwarp();
+        sh.warp[lane] = w;
+    }
+    __syncthreads();
+    if (warp) pre = sh.warp[warp - 1];
+    Inc2 before{__shfl_up_sync(0xffffffffu, in.even, 1), __shfl_up_sync(0xffffffffu, in.odd, 1)};
+    if (lane == 0) before = Inc2{0, 0};
+    before = inc_then(pre, before);
+    const Inc2 after = inc_then(before, inc);
+    const unsigned m0 = m + ((m & 1u) ? before.odd : before.even), m1 = m + ((m & 1u) ? after.odd : after.even);
+    if (stop || m1 >= (1u << 24)) atomicMin(&sh.first, threadIdx.x);
+    m_out = m0;
+    __syncthreads();
+    const unsigned first = sh.first;
+    if (first == kWalkThreads && threadIdx.x == kWalkThreads - 1) sh.s = float(m1) * u;
+    return first;
+}
+
+// The entries [lo, hi) added to sh.s.
+__device__ void walk_entries(WalkShared& sh, const float2* __restrict__ c, int64_t lo, int64_t hi)
+{
+    constexpr int kPer = 4;
+    while (lo < hi) {
+        __syncthreads();
+        const float s = sh.s;
+        const int64_t at = lo + int64_t(threadIdx.x) * kPer;
+        float x[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) x[k] = at + k < hi ? cabs_ref(c[at + k]) : 0.f;
+        unsigned first, m0 = 0;
+        float u = 1.f;
+        if (s < kSumTiny) {  // no binade yet: on to the first entries that are not zero
+            const bool any = x[0] != 0.f || x[1] != 0.f || x[2] != 0.f || x[3] != 0.f;
+            first = walk_parts(sh, Inc2{0, 0}, any, 0u, 0.f, m0);
+            if (first == kWalkThreads) {
+                __syncthreads();
+                if (threadIdx.x == 0) sh.s = s;
+            } else if (threadIdx.x == first) {
+                float t = s;
+#pragma unroll
+                for (int k = 0; k < kPer; ++k) t = __fadd_rn(t, x[k]);
+                sh.s = t;
+            }
+        } else {
+            const int e = exponent_of(s);
+            u = pow2f(e - 23);
+            const float per_u = pow2f(23 - e);
+            Inc2 inc{0, 0};
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) inc = inc_then(inc, inc_of(x[k], per_u));
+            first = walk_parts(sh, inc, false, unsigned(s * per_u), u, m0);
+            if (threadIdx.x == first) {
+                float t = float(m0) * u;
+#pragma unroll
+                for (int k = 0; k < kPer; ++k) t = __fadd_rn(t, x[k]);
+                sh.s = t;
+            }
+        }
+        lo += first == kWalkThreads ? int64_t(kWalkThreads) * kPer : (int64_t(first) + 1) * kPer;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kWalkThreads) sum_walk_kernel(const float2* __restrict__ c, SumBlocks b, float* out)
+{
+    __shared__ WalkShared sh;
+    if (threadIdx.x == 0) sh.s = 0.f;
+    walk_entries(sh, c, 0, min(b.n, b.per));  // the first binades are short
+    int k = 1;
+    while (k < b.nb) {
+        const float s = sh.s;
+        const int mine = k + int(threadIdx.x);
+        unsigned first = 0, m0 = 0;
+        if (s >= kSumTiny) {
+            const int e = exponent_of(s);
+            Inc2 inc{0, 0};
+            bool stop = false;
+            if (mine < b.nb) {
+                const int d = e - b.exps[mine];
+                stop = d < 0 || d > 1;
+                if (!stop) inc = b.incs[2 * mine + d];
+            }
+            const float u = pow2f(e - 23);
+            first = walk_parts(sh, inc, stop, unsigned(s * pow2f(23 - e)), u, m0);
+            if (threadIdx.x == first) sh.s = float(m0) * u;
+        }
+        if (first == kWalkThreads) {
+            k += kWalkThreads;
+            __syncthreads();
+            continue;
+        }
+        k += int(first);
+        __syncthreads();  // the sum before block k
+        walk_entries(sh, c, int64_t(k) * b.per, min(b.n, (int64_t(k) + 1) * b.per));
+        ++k;
+    }
+    if (threadIdx.x == 0) out[0] = sh.s;
 }
 
 // C *= float(wSize*os*os) / sumC, as a complex multiply by (scale, 0) (Benchmark.cc:267-269).
@@ -147,30 +373,27 @@ __global__ void offsets_kernel(OffParams p, const double* u, const double* v, co
 }
 
 // ---- table storage conversions ----
-__global__ void absmax_imag_kernel(const float2* c, int64_t n, unsigned int* absmax_bits,
-                                   unsigned long long* imag_nonzero)
+__global__ void absmax_kernel(const float2* c, int64_t n, unsigned int* absmax_bits)
 {
     float m = 0.f;
-    unsigned long long nz = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 z = c[i];
         m = fmaxf(m, fmaxf(fabsf(z.x), fabsf(z.y)));
-        nz += (z.y != 0.f);
     }
-    for (int o = 16; o; o >>= 1) {
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        nz += __shfl_xor_sync(0xffffffffu, nz, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
-        if (nz) atomicAdd(imag_nonzero, nz);
-    }
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
 }
 
-__global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre_scale, void* out)
+// One entry per thread and step; counts the entries with an imaginary part as it goes (for the
+// forms without a scale this is the only pass over the table: 35 M entries to r32 in 175 us with a
+// counting pass before it, 85 us in one).
+__global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre_scale, void* out,
+                               unsigned long long* imag_nonzero)
 {
+    unsigned long long nz = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 z = c[i];
+        nz += (z.y != 0.f);
         switch (c_type) {
             case TCV_C_R32: static_cast<float*>(out)[i] = z.x; break;
             case TCV_C_CBF16: {
@@ -187,6 +410,8 @@ __global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre
             default: break;
         }
     }
+    for (int o = 16; o; o >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, o);
+    if ((threadIdx.x & 31) == 0 && nz) atomicAdd(imag_nonzero, nz);
 }
 
 inline int grid_blocks(int64_t n, int threads)
@@ -218,7 +443,11 @@ tcv_status tcv_c_geometry(double freq0, double cell_size, int baseline, int w_si
     return TCV_OK;
 }
 
-size_t tcv_init_c_scratch_bytes(void) { return 256; }
+// the sum, then the per-block sums, increments and exponents of the parallel sum
+size_t tcv_init_c_scratch_bytes(void)
+{
+    return 256 + size_t(kSumMaxBlocks) * (sizeof(double) + 2 * sizeof(Inc2) + sizeof(int));
+}
 
 tcv_status tcv_init_c_raw(double freq0, double cell_size, int baseline, int w_size, float* d_c,
                           void* d_scratch, float* sum_c_out, void* stream)
@@ -232,10 +461,24 @@ tcv_status tcv_init_c_raw(double freq0, double cell_size, int baseline, int w_si
     if (n > INT_MAX) return TCV_ERR_UNSUPPORTED;  // cOffset is a 32-bit int in the reference
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CParams p{2 * support + 1, os, w_size, support, wcs, freq0, cell_size, n};
-    init_c_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(p, reinterpret_cast<float2*>(d_c));
+    const int64_t half = n / w_size * (w_size / 2 + 1);  // entries of the planes w >= 0
+    init_c_kernel<<<unsigned((half + 255) / 256), 256, 0, s>>>(p, reinterpret_cast<float2*>(d_c));
     TCV_CUDA(cudaGetLastError());
     float* d_sum = static_cast<float*>(d_scratch);
-    sum_abs_seq_kernel<<<1, 1024, 0, s>>>(reinterpret_cast<const float2*>(d_c), n, d_sum);
+    SumBlocks sb{};
+    sb.n = n;
+    const int64_t chunks = (n + kSumChunk - 1) / kSumChunk;
+    sb.per = (chunks + kSumMaxBlocks - 1) / kSumMaxBlocks * kSumChunk;
+    sb.nb = int((n + sb.per - 1) / sb.per);
+    sb.sum = reinterpret_cast<double*>(static_cast<char*>(d_scratch) + 256);
+    sb.incs = reinterpret_cast<Inc2*>(sb.sum + kSumMaxBlocks);
+    sb.exps = reinterpret_cast<int*>(sb.incs + 2 * kSumMaxBlocks);
+    const float2* table = reinterpret_cast<const float2*>(d_c);
+    sum_blocks_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
+    TCV_CUDA(cudaGetLastError());
+    sum_incs_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
+    TCV_CUDA(cudaGetLastError());
+    sum_walk_kernel<<<1, kWalkThreads, 0, s>>>(table, sb, d_sum);
     TCV_CUDA(cudaGetLastError());
     scale_c_kernel<<<grid_blocks(n, 256), 256, 0, s>>>(reinterpret_cast<float2*>(d_c), n,
                                                        float(w_size * os * os), d_sum);
@@ -282,21 +525,15 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
     unsigned int* d_max = static_cast<unsigned int*>(scratch);
     unsigned long long* d_nz = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 8);
     cudaError_t e = cudaMemsetAsync(scratch, 0, 16, s);
-    if (e == cudaSuccess) {
-        absmax_imag_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, d_max, d_nz);
-        e = cudaGetLastError();
-    }
-    unsigned int hmax = 0;
-    unsigned long long hnz = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hmax, d_max, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hnz, d_nz, 8, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(scratch);
-    TCV_CUDA(e);
     float pre = 1.0f, post = 1.0f;
-    if (c_type == TCV_C_CF16 || c_type == TCV_C_RF16) {
+    if (e == cudaSuccess && (c_type == TCV_C_CF16 || c_type == TCV_C_RF16)) {
         // power-of-two scale putting max |C| in [2^14, 2^15): the table keeps FP16's full
         // precision without approaching its 65504 limit; kernels undo it exactly with c_scale.
+        unsigned int hmax = 0;
+        absmax_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, d_max);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&hmax, d_max, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         const float amax = __builtin_bit_cast(float, hmax);
         int ex = 0;
         if (amax > 0.f) {
@@ -306,8 +543,15 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
             post = std::ldexp(1.0f, -shift);
         }
     }
-    convert_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, c_type, pre, d_out);
-    TCV_CUDA(cudaGetLastError());
+    unsigned long long hnz = 0;
+    if (e == cudaSuccess) {
+        convert_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, c_type, pre, d_out, d_nz);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hnz, d_nz, 8, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFree(scratch);
+    TCV_CUDA(e);
     if (c_scale_out) *c_scale_out = post;
     if (imag_nonzero_out) *imag_nonzero_out = int64_t(hnz);
     return TCV_OK;
