@@ -13,14 +13,43 @@
 // HogbomGolden.cc:108); that is kept.  Where it points outside the PSF (only when the PSF peak is
 // off the diagonal) the reference reads out of bounds; here those rows are skipped and counted.
 //
-// B200 layout: one launch per iteration, no host round trip.  A launch subtracts the PSF over its
-// blocks' slices of the image and scans the updated values for the next peak in the same pass, so
-// an iteration reads the residual once, reads the PSF's overlap once and writes the overlap once.
-// Each block leaves one candidate, a 64-bit key (|value| bits << 32 | ~index: the largest key is
-// the largest magnitude at the smallest index) with its signed value; the last block to finish
-// (an atomic ticket, no waiting) reduces the candidates to the winner that the next launch reads.
-// The stop test (|peak| < threshold) is taken on the device: later launches see the flag and return.
+// Three forms, chosen by size (tcv_hogbom_deconvolve); all give the same bits.
+//
+// Up to 2048 x 2048 (hog_resident_kernel): the residual stays in registers, one cooperative launch.
+//
+// Larger images: updates are put off.  The image is cut into blocks of at least 32 x 32 pixels, and
+// a block's updates wait until the block could hold the next peak:
+//   * per block, a bound on its |residual|: its largest |value| when last brought up to date, plus
+//     |t| x the largest |psf| over the part of the PSF each update since has laid on it (from a table
+//     of the PSF's block maxima), rounded up;
+//   * the updated value at the peak itself, |peak - t psf(peak)|, is a lower limit of the next peak:
+//     blocks whose bound is below it cannot hold that and are left alone; the others ("hot", ~25 per
+//     iteration around the brightest pixels, of 16384 at 4096^2) apply their pending updates in
+//     order and give their largest value, which is exact.
+// hog_lead_kernel runs kLeadIters iterations in one cluster, whose CTAs share out the blocks and
+// exchange candidates through distributed shared memory: an iteration is a chain of latencies
+// (bounds, the hot blocks' loads, the exchange: 5 us at 4096^2), not a pass over the image.
+// hog_apply_kernel follows on the whole device: it brings blocks near the peak up to date, and
+// every kRing iterations and at the end all blocks (9 us an iteration at 4096^2, most of it the PSF
+// windows from L2).  A pixel's updates are applied in iteration order with the reference's
+// roundings whenever they are applied, so the bits do not depend on the schedule.
+//
+// Beyond the block table's size (or with TCV_HOGBOM_PER_LAUNCH): a launch per iteration, which
+// subtracts the PSF over its blocks' slices of the image and scans the updated values for the
+// next peak in the same pass, so an iteration reads the residual once, reads the PSF's overlap
+// once and writes the overlap once.  Each block leaves one candidate, a 64-bit key (|value| bits
+// << 32 | ~index: the largest key is the largest magnitude at the smallest index) with its signed
+// value; the last block to finish (an atomic ticket, no waiting) reduces the candidates to the
+// winner that the next launch reads.  The stop test (|peak| < threshold) is taken on the device:
+// later launches see the flag and return.
+//
+// Measured on one B200, us an iteration, and in brackets with one pass over the image per iteration
+// (in one cooperative launch up to 48 MiB of images, all CTAs waiting on one counter; a launch
+// each beyond): 223^2 1.8 (8.0), 1024^2 3.4 (4.64), 1884^2 6.8 (8.2), 4096^2 16.5 (27.0).
 #include "tcv_internal.cuh"
+
+#include <cooperative_groups.h>
+#include <cuda_pipeline.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -35,13 +64,14 @@ constexpr int kHogMaxBlocks = 592;  // 4 x 148: one wave of four 256-thread CTAs
 struct HogState {
     unsigned long long win_key[3];  // winners: [0], [1] by iteration parity, [2] the PSF's
     float win_val[3];
-    unsigned int arrived;           // blocks finished in the current launch (persistent loop: in all
-                                    // iterations so far)
+    unsigned int arrived;           // blocks finished in the current launch
     int stopped;                    // 1 + the iteration whose |peak| fell below the threshold; 0 = running
     int done;                       // iterations carried out
     unsigned int psf_pos;           // PSF peak index
     unsigned long long skipped_rows;  // PSF rows outside the PSF (reference out-of-bounds reads)
-    int error;                        // persistent kernel: a barrier wait gave up
+    int error;                        // a wait for other CTAs gave up
+    int batch, used;                  // put-off updates: the ring's last batch and its PSF windows
+    unsigned int nwarm;               // and the blocks of the list for hog_apply_kernel
 };
 
 struct HogArgs {
@@ -50,16 +80,12 @@ struct HogArgs {
     float* model;
     unsigned long long* keys;  // one candidate per block
     float* vals;
-    unsigned long long* keys2;  // persistent loop: the candidates of odd iterations
-    float* vals2;
     HogState* state;
     float* hist_val;         // per iteration: peak value (may be null)
     unsigned int* hist_pos;  // per iteration: peak index (may be null)
     int width, psf_width, nblocks;
     long long n;  // width * width
     float gain, threshold;
-    unsigned long long wait_ns;  // persistent loop: limit of one grid-barrier wait
-    unsigned int withheld;       // persistent loop: arrivals the barrier counts that never come (test hook)
 };
 
 __device__ __forceinline__ unsigned int key_index(unsigned long long k) { return ~static_cast<unsigned int>(k); }
@@ -321,81 +347,818 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// All iterations in one cooperative launch (every CTA resident).  Per iteration each CTA leaves its
-// candidate in the buffer of the iteration's parity and adds one to a monotonic arrival count;
-// once the count reaches the iteration's target every CTA reads all candidates itself and reduces
-// them in the same order (so every CTA holds the same winner), with no second round trip through a
-// published winner.  Waits are bounded by an iteration count and 2 s of %globaltimer, after which
-// the CTA flags the error and returns (the host reports TCV_ERR_TIMEOUT).  Two candidate buffers
-// suffice: a CTA cannot write iteration it + 1's candidates before every CTA has arrived at barrier
-// it, i.e. has read iteration it - 1's.
-template <bool kVec>
-__global__ void __launch_bounds__(kHogThreads, 2) hog_persist_kernel(HogArgs a, int niters)
+constexpr int kLeadThreads = 512;
+constexpr int kLeadWarps = kLeadThreads / 32;
+constexpr int kLeadCtas = 16;        // CTAs of the leading cluster (8 where 16 do not fit)
+constexpr int kBlkSide = 128;        // image and PSF blocks per side, at most
+constexpr int kBlkMax = kBlkSide * kBlkSide;
+constexpr int kDeferMaxWidth = 128 * kBlkSide;  // blocks of up to 128 x 128 pixels
+constexpr int kOwned = kBlkMax / 8;  // blocks per CTA of the cluster, at most
+constexpr int kLeadIters = 16;       // iterations per launch of the cluster (even)
+constexpr int kRing = 128;           // iterations whose updates may be pending (a multiple of kLeadIters)
+constexpr int kApplyThreads = 128;
+constexpr int kApplyRows = 4;        // rows per warp: a CTA works on 32 x 16 pixels at a time
+constexpr int kSlots = 48;           // PSF windows of that size an applying CTA holds
+constexpr int kStrips = 32 / (kApplyThreads / 32 * kApplyRows);  // parts of 32 columns a 32 x 32 square is worked on in
+constexpr int kWindow = kApplyThreads * kApplyRows;  // pixels of a window
+
+// A candidate as one word: larger |value| first, then the smaller index (row << 16 | column, so that
+// no division is needed to get at them); the sign last.
+__device__ __forceinline__ unsigned long long cand_key(float v, int x, int y)
 {
-    HogState* st = a.state;
-    const unsigned int psf_pos = st->psf_pos;
-    __shared__ int ok;
-    unsigned int ppos = key_index(__ldcg(&st->win_key[0]));  // the dirty image's scan
-    float peak = __ldcg(&st->win_val[0]);
+    const unsigned int b = __float_as_uint(v), idx = unsigned(y) << 16 | unsigned(x);
+    return (static_cast<unsigned long long>(b & 0x7fffffffu) << 33) | (static_cast<unsigned long long>(~idx) << 1) | (b >> 31);
+}
+__device__ __forceinline__ float cand_abs(unsigned long long k) { return __uint_as_float(unsigned(k >> 33)); }
+__device__ __forceinline__ float cand_value(unsigned long long k)
+{
+    return __uint_as_float(unsigned(k >> 33) | (unsigned(k & 1u) << 31));
+}
+__device__ __forceinline__ unsigned int cand_index(unsigned long long k) { return ~unsigned(k >> 1); }
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
+{
+    const unsigned int hi = unsigned(k >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned int lo = __reduce_max_sync(0xffffffffu, hi == top ? unsigned(k) : 0u);
+    return (static_cast<unsigned long long>(top) << 32) | lo;
+}
+
+// ------------------------------------------------------------------------------------------
+// Images that fit the register files: the residual stays in registers for all iterations.  Each CTA
+// owns whole rows, a thread up to kRowsT x kChunks pixels of them; an iteration loads the PSF (from
+// L2), updates, and finds the CTA's candidate; the CTAs of a cluster send theirs to its first CTA
+// through distributed shared memory, the first CTAs exchange theirs through global memory (16-18
+// words instead of one per CTA: all CTAs polling all CTAs' words kept the few L2 lines they lie on
+// busy and took 4 us), and each hands the winner to its cluster.
+// ------------------------------------------------------------------------------------------
+constexpr int kResThreads = 512;
+constexpr int kResChunks = 4;       // columns per thread, at most: widths up to 2048
+constexpr int kResClusters = 32;    // clusters of a launch, at most
+
+struct ResArgs {
+    HogArgs h;
+    unsigned long long* post;  // [2][kResClusters][2]: the clusters' candidates, by iteration parity
+    int rows;                  // rows per CTA
+};
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
+
+// one candidate to CTA `cta` of the cluster, counted there by its barrier
+__device__ __forceinline__ void send_key(const unsigned long long* slot, const unsigned long long* bar, int cta,
+                                         unsigned long long key)
+{
+    unsigned dst, mb;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_addr(slot)), "r"(cta));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(mb) : "r"(smem_addr(bar)), "r"(cta));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(dst), "l"(key), "r"(mb)
+                 : "memory");
+}
+__device__ __forceinline__ void expect_bytes(const unsigned long long* bar, int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+// waits for the barrier's phase; false after wait_ns (or the iteration cap)
+__device__ __forceinline__ bool wait_phase(const unsigned long long* bar, unsigned phase, unsigned long long wait_ns)
+{
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0; spin < (1u << 24); ++spin) {
+        unsigned ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(smem_addr(bar)), "r"(phase) : "memory");
+        if (ok) return true;
+        if ((spin & 63u) == 63u) {
+            if (!t0)
+                t0 = global_ns();
+            else if (global_ns() - t0 >= wait_ns)
+                return false;
+        }
+    }
+    return false;
+}
+
+// rows whose PSF values are loaded into registers: 32 values a thread at most, beside up to 64 pixels
+__host__ __device__ constexpr int res_direct(int rows, int chunks) { return rows * chunks <= 32 ? rows : 32 / chunks; }
+
+template <int kRowsT, int kChunks>
+__global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a, int niters, unsigned long long wait_ns,
+                                                                      unsigned int withheld)
+{
+    constexpr int kDirect = res_direct(kRowsT, kChunks);
+    extern __shared__ __align__(16) float later[];  // [(kRowsT - kDirect) * kChunks][kResThreads]
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    __shared__ unsigned long long got[2][16], win[2];    // by iteration parity: the cluster's candidates; the winner
+    __shared__ unsigned long long bar_got[2], bar_win[2];
+    __shared__ unsigned long long key;
+    __shared__ unsigned wk[kResThreads / 32];
+    HogState* st = a.h.state;
+    const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int W = a.h.width, P = a.h.psf_width;
+    const int ctas = int(cluster.num_blocks()), rank = int(cluster.block_rank()), cl = int(blockIdx.x) / ctas;
+    const int ncl = int(gridDim.x) / ctas;
+    const int y0 = int(blockIdx.x) * a.rows, ye = min(W, y0 + a.rows);
+    if (tid == 0) {
+        for (int p = 0; p < 2; ++p) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar_got[p])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar_win[p])) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    float r[kRowsT][kChunks];
+#pragma unroll
+    for (int i = 0; i < kRowsT; ++i)
+#pragma unroll
+        for (int j = 0; j < kChunks; ++j) {
+            const int x = tid + j * kResThreads, y = y0 + i;
+            r[i][j] = x < W && y < ye ? a.h.residual[size_t(y) * W + x] : __int_as_float(0x7fffffff);  // never a peak
+        }
+    const int px = int(st->psf_pos % unsigned(P)), py = int(st->psf_pos / unsigned(P));
+    const unsigned int flat = key_index(st->win_key[0]);  // the dirty image's scan
+    int rx = int(flat % unsigned(W)), ry = int(flat / unsigned(W));
+    float peak = st->win_val[0];
+    // the model update of the last iteration, its load left in flight (one thread of the first CTA)
+    const bool models = blockIdx.x == 0 && tid == kResThreads - 1;
+    float m_old = 0.f, m_add = 0.f;
+    size_t m_pos = 0;
+    bool m_open = false;
+    unsigned long long skipped = 0;
+    cluster.sync();  // every CTA runs (its shared memory is written to)
     for (int it = 0; it < niters; ++it) {
-        if (fabsf(peak) < a.threshold) {  // every CTA holds the same winner: all stop here
-            if (blockIdx.x == 0 && threadIdx.x == 0) st->stopped = it + 1;
-            return;
+        const int par = it & 1;
+        const unsigned phase = unsigned(it >> 1) & 1u;
+        if (fabsf(peak) < a.h.threshold) {  // every CTA holds the same winner: all stop here (HogbomGolden.cc:86-89)
+            if (models) st->stopped = it + 1;
+            break;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            model_update(a, it, ppos, peak);
+        const int diffx = rx - px, diffy = ry - px;  // diffy uses px, as the reference does
+        const int startx = max(0, diffx), stopx = min(W - 1, rx + (P - px - 1));
+        const int starty = max(0, ry - py), stopy = min(W - 1, ry + (P - py - 1));
+        // rows whose PSF row lies inside the PSF (all of them unless its peak is off the diagonal)
+        const int ya = max(starty, diffy), yb = min(stopy, diffy + P - 1);
+        const float t = __fmul_rn(a.h.gain, peak);
+        if (tid == 0) {
+            if (rank == 0) expect_bytes(&bar_got[par], ctas * 8);
+            expect_bytes(&bar_win[par], 8);
+        }
+        if (models) {  // model[absPeakPos] += absPeakVal * g_gain (HogbomGolden.cc:93)
+            if (m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
+            m_pos = size_t(ry) * W + rx;
+            m_add = __fmul_rn(peak, a.h.gain);
+            m_old = *reinterpret_cast<volatile float*>(a.h.model + m_pos);
+            m_open = true;
+            if (a.h.hist_val) a.h.hist_val[it] = peak;
+            if (a.h.hist_pos) a.h.hist_pos[it] = unsigned(m_pos);
             st->done = it + 1;
+            skipped += (unsigned long long)(stopy - starty + 1 - max(0, yb - ya + 1));
         }
-        float bv;
-        unsigned long long skipped;
-        unsigned long long best = iter_body<kVec>(a, ppos, peak, psf_pos, bv, skipped);
-        if (skipped) atomicAdd(&st->skipped_rows, skipped);
-        best = block_max(best, bv);
-        unsigned long long* keys = (it & 1) ? a.keys2 : a.keys;
-        float* vals = (it & 1) ? a.vals2 : a.vals;
-        if (threadIdx.x == 0) {
-            keys[blockIdx.x] = best;
-            vals[blockIdx.x] = bv;
-            __threadfence();
-            atomicAdd(&st->arrived, 1u);
-            const unsigned int target = unsigned(it + 1) * unsigned(a.nblocks) + a.withheld;
-            ok = 0;
-            const unsigned long long t0 = global_ns();
-            for (unsigned int spin = 0; spin < (1u << 24); ++spin) {
-                if (*reinterpret_cast<volatile unsigned int*>(&st->arrived) >= target) {
-                    ok = 1;
-                    break;
-                }
-                if (*reinterpret_cast<volatile int*>(&st->error)) break;
-                __nanosleep(32);
-                if ((spin & 63u) == 63u && global_ns() - t0 >= a.wait_ns) break;
+        const float* __restrict__ p0 = a.h.psf + (ptrdiff_t(y0 - diffy) * P + (tid - diffx));
+        bool cols[kChunks];
+#pragma unroll
+        for (int j = 0; j < kChunks; ++j) cols[j] = tid + j * kResThreads >= startx && tid + j * kResThreads <= stopx;
+        const int ia = ya - y0, ib = min(yb, ye - 1) - y0;  // this CTA's rows that are updated
+        // the whole iteration's PSF values in flight at once: the later rows' by asynchronous copies to
+        // this thread's own places in shared memory, the first rows' in registers
+        // (2048^2: 7.6 us an iteration with half of them loaded after the other half, 6.35 so)
+#pragma unroll
+        for (int i = kDirect; i < kRowsT; ++i)
+            if (i >= ia && i <= ib) {
+                const float* __restrict__ q = p0 + ptrdiff_t(i) * P;
+#pragma unroll
+                for (int j = 0; j < kChunks; ++j)
+                    if (cols[j])
+                        __pipeline_memcpy_async(later + ((i - kDirect) * kChunks + j) * kResThreads + tid, q + j * kResThreads, 4);
             }
-            if (!ok) st->error = 1;
-            __threadfence();
+        if (kDirect < kRowsT) __pipeline_commit();
+        float pv[kDirect][kChunks], top = -1.f;  // only the largest |value| is kept here
+#pragma unroll
+        for (int i = 0; i < kDirect; ++i)
+            if (i >= ia && i <= ib) {
+                const float* __restrict__ q = p0 + ptrdiff_t(i) * P;
+#pragma unroll
+                for (int j = 0; j < kChunks; ++j)
+                    if (cols[j]) pv[i][j] = __ldg(q + j * kResThreads);
+            }
+#pragma unroll
+        for (int i = 0; i < kRowsT; ++i) {
+            if (i == kDirect) __pipeline_wait_prior(0);
+            if (i >= ia && i <= ib) {
+#pragma unroll
+                for (int j = 0; j < kChunks; ++j)
+                    if (cols[j])
+                        r[i][j] = __fsub_rn(r[i][j], __fmul_rn(t, i < kDirect ? pv[i < kDirect ? i : 0][j]
+                                                                              : later[((i - kDirect) * kChunks + j) * kResThreads + tid]));
+            }
+#pragma unroll
+            for (int j = 0; j < kChunks; ++j) top = fmaxf(top, fabsf(r[i][j]));  // (places past the image hold NaN)
+        }
+        // the CTA's largest |value|, then its first place (only threads that hold that value look)
+        const unsigned mine = top < 0.f ? 0u : __float_as_uint(top) + 1u;
+        const unsigned most = __reduce_max_sync(0xffffffffu, mine);
+        if (lane == 0) wk[warp] = most;
+        if (tid == 0) key = 0;
+        __syncthreads();
+        const unsigned all = __reduce_max_sync(0xffffffffu, lane < kResThreads / 32 ? wk[lane] : 0u);
+        if (mine == all && all) {
+            bool found = false;
+#pragma unroll
+            for (int i = 0; i < kRowsT; ++i)
+#pragma unroll
+                for (int j = 0; j < kChunks; ++j)
+                    if (!found && fabsf(r[i][j]) == top) {  // rows, then columns in order: the thread's first
+                        found = true;
+                        atomicMax(&key, cand_key(r[i][j], tid + j * kResThreads, y0 + i));
+                    }
         }
         __syncthreads();
-        if (!ok) return;
-        // every CTA: the winner of this iteration's candidates, in the same order everywhere
-        unsigned long long k = 0;
-        float v = 0.f;
-        for (int i = threadIdx.x; i < a.nblocks; i += kHogThreads) {
-            const unsigned long long ki = __ldcg(keys + i);
-            if (ki > k) {
-                k = ki;
-                v = __ldcg(vals + i);
+        unsigned long long c;
+        bool ok = true;
+        if (warp == 0) {
+            c = key;
+            if (lane == 0) send_key(&got[par][rank], &bar_got[par], 0, c);
+            if (rank == 0) {
+                ok = wait_phase(&bar_got[par], phase, wait_ns);
+                c = warp_max(lane < ctas ? got[par][lane] : 0ull);
+                volatile unsigned long long* w = a.post + size_t(par) * kResClusters * 2;
+                const unsigned long long tag = unsigned(it + 1);
+                // two words, each with the iteration: a reader takes them when both are there.  Two
+                // buffers suffice: a cluster posts iteration it + 2's after it has all of it + 1's.
+                if (lane == 0) {
+                    w[cl * 2] = (c & 0xffffffff00000000ull) | tag;
+                    w[cl * 2 + 1] = (c << 32) | tag;
+                }
+                c = 0;
+                if (lane < ncl + int(withheld)) {
+                    bool here = false;
+                    unsigned long long t0 = 0;
+                    for (unsigned spin = 0; spin < (1u << 26) && ok; ++spin) {
+                        const unsigned long long k0 = w[min(lane, ncl - 1) * 2], k1 = w[min(lane, ncl - 1) * 2 + 1];
+                        if (lane < ncl && unsigned(k0) == unsigned(tag) && unsigned(k1) == unsigned(tag)) {
+                            c = (k0 & 0xffffffff00000000ull) | (k1 >> 32);
+                            here = true;
+                            break;
+                        }
+                        if ((spin & 63u) == 63u) {
+                            if (*reinterpret_cast<volatile int*>(&st->error)) break;
+                            if (!t0) t0 = global_ns();
+                            if (global_ns() - t0 >= wait_ns) break;
+                        }
+                    }
+                    ok = here;
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                c = warp_max(c);
+                if (!ok) st->error = 1;
+                if (ok && lane < ctas) send_key(&win[par], &bar_win[par], lane, c);
             }
         }
-        k = block_max(k, v);
-        const bool zero = (k >> 32) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
-        ppos = zero ? 0u : key_index(k);
-        peak = zero ? 0.f : v;
+        if (ok) ok = wait_phase(&bar_win[par], phase, wait_ns);
+        if (!__syncthreads_and(ok)) {
+            st->error = 1;
+            break;
+        }
+        c = win[par];
+        const bool zero = (c >> 33) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
+        const unsigned int idx = zero ? 0u : cand_index(c);
+        rx = int(idx & 0xffffu);
+        ry = int(idx >> 16);
+        peak = zero ? 0.f : cand_value(c);
+    }
+#pragma unroll
+    for (int i = 0; i < kRowsT; ++i)
+#pragma unroll
+        for (int j = 0; j < kChunks; ++j) {
+            const int x = tid + j * kResThreads, y = y0 + i;
+            if (x < W && y < ye) a.h.residual[size_t(y) * W + x] = r[i][j];
+        }
+    if (models && m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
+    if (models && skipped) st->skipped_rows = skipped;
+    cluster.sync();  // no CTA leaves while another's store to it may be under way
+}
+
+// ------------------------------------------------------------------------------------------
+// Larger images: put-off updates (see the top of the file).
+// ------------------------------------------------------------------------------------------
+// One update as the blocks apply it: residual[y][x] -= t * psf[y * P + x + off] for the pixels
+// (x, y) of the image that the PSF's rows and columns cover.
+struct Update {
+    float t;
+    int off;
+    unsigned int xr, yr;  // first | last << 16
+};
+
+// How the applying CTAs share PSF windows among updates at one peak: the ring is walked in batches
+// of at most kSlots windows; an update's window is loaded unless an update of the batch already
+// has (prev: the last earlier update in the ring at the same place, or -1).
+struct UpdateSlot {
+    short prev, slot, batch, pad;  // batch: ring index its batch starts at
+};
+
+struct DeferArgs {
+    HogArgs h;
+    float* bound;           // per image block: limit of its |residual| as of the last update
+    int* applied;           // per image block: iterations whose updates it has
+    unsigned int* warm;     // st->nwarm blocks that hog_apply_kernel is to bring up to date
+    const float* pmax;      // per PSF block: its largest |value|
+    Update* ring;           // [kRing] updates of the iterations from base on
+    UpdateSlot* slots;      // [kRing]
+    int lb, nbx;            // log2 of the block side; blocks per image side
+    int lbp, npx;           // the same of the PSF
+};
+
+// An update's cover of the 32 columns from x0 and `rows` rows from y0: whole (2; they then lie
+// inside the image), in part (1) or none (0).
+__device__ __forceinline__ int cover_of(const Update& u, int x0, int y0, int rows)
+{
+    const int xa = int(u.xr & 0xffffu), xb = int(u.xr >> 16), ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
+    if (xa <= x0 && xb >= x0 + 31 && ya <= y0 && yb >= y0 + rows - 1) return 2;
+    return xa > x0 + 31 || xb < x0 || ya > y0 + rows - 1 || yb < y0 ? 0 : 1;
+}
+
+// An image's blocks: their largest |value| (one warp per block) and the image's own peak; copies the
+// image when copy_to is given.
+__global__ void __launch_bounds__(kHogThreads) hog_blocks_kernel(const float* __restrict__ img, float* __restrict__ copy_to,
+                                                                 int W, int lb, int nbx, float* top, int* applied,
+                                                                 unsigned long long* keys, float* vals, HogState* st,
+                                                                 int slot)
+{
+    const int lane = threadIdx.x & 31, nb = nbx * nbx;
+    const int warps = int(gridDim.x) * (kHogThreads / 32);
+    unsigned long long best = 0;
+    for (int b = int(blockIdx.x) * (kHogThreads / 32) + (threadIdx.x >> 5); b < nb; b += warps) {
+        const int x0 = (b % nbx) << lb, y0 = (b / nbx) << lb, side = 1 << lb;
+        const int ye = min(W, y0 + side);
+        unsigned long long k = 0;
+        for (int x = x0 + lane; x < min(W, x0 + side); x += 32) {
+            float t = -1.f, tv = 0.f;
+            int ty = 0;
+            for (int y = y0; y < ye; y += 8) {
+                float v[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[r] = y + r < ye ? __ldcs(img + (size_t(y + r) * W + x)) : 0.f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    if (y + r >= ye) break;
+                    if (copy_to) copy_to[size_t(y + r) * W + x] = v[r];
+                    if (fabsf(v[r]) > t) {  // rows in order: strict '>' keeps the first
+                        t = fabsf(v[r]);
+                        tv = v[r];
+                        ty = y + r;
+                    }
+                }
+            }
+            if (t >= 0.f) {
+                k = max(k, cand_key(tv, x, ty));
+            }
+        }
+        k = warp_max(k);
+        if (lane == 0) {
+            top[b] = cand_abs(k);
+            if (applied) applied[b] = 0;
+        }
+        best = max(best, k);
+    }
+    // the one-pass kernels' form of it: a flat index
+    const unsigned int at = cand_index(best), flat = (at >> 16) * unsigned(W) + (at & 0xffffu);
+    const unsigned long long old = best ? ((best >> 33) << 32) | unsigned(~flat) : 0ull;
+    finish_scan(old, cand_value(best), keys, vals, int(gridDim.x), st, slot);
+}
+
+constexpr int kLeadRows = 8;  // rows per warp: four warps per hot block, four blocks at a time
+constexpr int kLeadGroup = 32 / kLeadRows;
+
+struct LeadShared {
+    Update ring[kRing];
+    unsigned long long cand[2][kLeadCtas];  // the cluster's candidates, by iteration parity
+    unsigned long long arrived[2];          // mbarriers: all of cand[parity] is here
+    float bound[kOwned];
+    int applied[kOwned];
+    unsigned int at[kOwned];                // first row << 16 | first column
+    unsigned short hot[kOwned];
+    int nhot[2];
+};
+
+// The blocks are dealt to the cluster's CTAs in 4 x (CTAs / 4) tiles, so that neighbours, which
+// are hot together, are different CTAs'.  Block `own` of CTA `rank`:
+struct LeadDeal {
+    int nox, noy;  // blocks of a CTA per row and per column (some past the image)
+    __host__ __device__ LeadDeal(int nbx, int ctas) : nox((nbx + 3) / 4), noy((nbx + ctas / 4 - 1) / (ctas / 4)) {}
+    __device__ int x(int own, int rank) const { return own % nox * 4 + (rank & 3); }
+    __device__ int y(int own, int rank, int ctas) const { return own / nox * (ctas / 4) + (rank >> 2); }
+};
+
+// The pending updates up to iteration `to` of the CTA's nhot hot blocks, four warps per block, and the
+// blocks' candidates.  One short loop for every case (the code of an iteration has to stay in the
+// instruction cache: an iteration runs each line once).
+__device__ __forceinline__ void lead_apply(const DeferArgs& a, LeadShared& sh, unsigned long long* parts, int nhot, int base,
+                                           int to)
+{
+    constexpr int kRows = kLeadRows, kDeep = 4;  // kDeep updates' loads are in flight together
+    const int W = a.h.width, P = a.h.psf_width;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = warp / kLeadGroup; i < nhot; i += kLeadWarps / kLeadGroup) {
+        const int own = sh.hot[i], from = sh.applied[own];
+        unsigned long long c = 0;
+        for (int part = 0; part < 1 << (2 * (a.lb - 5)); ++part) {  // 32 x 32 pixels of the block
+            const int x = int(sh.at[own] & 0xffffu) + ((part & ((1 << (a.lb - 5)) - 1)) << 5) + lane;
+            const int y = int(sh.at[own] >> 16) + ((part >> (a.lb - 5)) << 5) + (warp % kLeadGroup) * kRows;
+            const int rows = x < W ? min(kRows, W - y) : 0;  // none past the image
+            float r[kRows];
+            float* rp = a.h.residual + (size_t(y) * W + x);
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) r[k] = k < rows ? rp[size_t(k) * W] : 0.f;
+            const float* __restrict__ pp = a.h.psf + (ptrdiff_t(y) * P + x);
+#pragma unroll 1
+            for (int q = from; q < to; q += kDeep) {
+                float pv[kDeep][kRows];
+#pragma unroll
+                for (int d = 0; d < kDeep; ++d) {
+                    if (q + d >= to) break;
+                    const Update u = sh.ring[q + d - base];
+                    const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
+                    const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
+#pragma unroll
+                    for (int k = 0; k < kRows; ++k)
+                        pv[d][k] = cx && y + k >= ya && y + k <= yb ? __ldg(pp + (u.off + ptrdiff_t(k) * P)) : 0.f;
+                }
+#pragma unroll
+                for (int d = 0; d < kDeep; ++d) {
+                    if (q + d >= to) break;
+                    const Update u = sh.ring[q + d - base];
+                    const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
+                    const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
+#pragma unroll
+                    for (int k = 0; k < kRows; ++k)
+                        if (cx && y + k >= ya && y + k <= yb) r[k] = __fsub_rn(r[k], __fmul_rn(u.t, pv[d][k]));
+                }
+            }
+            float top = -1.f, tv = 0.f;
+            int ty = 0;
+#pragma unroll
+            for (int k = 0; k < kRows; ++k)
+                if (k < rows) {
+                    rp[size_t(k) * W] = r[k];
+                    if (fabsf(r[k]) > top) {
+                        top = fabsf(r[k]);
+                        tv = r[k];
+                        ty = y + k;
+                    }
+                }
+            c = max(c, top < 0.f ? 0ull : cand_key(tv, x, ty));
+        }
+        c = warp_max(c);
+        if (lane == 0) parts[i * kLeadGroup + warp % kLeadGroup] = c;
+    }
+}
+
+
+// Iterations [it0, it1) by one cluster; the ring holds the updates from iteration base on.
+__global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, int it0, int it1, int base)
+{
+    extern __shared__ __align__(16) unsigned char lead_smem[];
+    LeadShared& sh = *reinterpret_cast<LeadShared*>(lead_smem);
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    HogState* st = a.h.state;
+    if (st->stopped) return;  // an earlier launch stopped the loop (the whole cluster returns)
+    const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int W = a.h.width, P = a.h.psf_width, ctas = int(gridDim.x), rank = int(blockIdx.x);
+    const int side = 1 << a.lb;
+    const LeadDeal deal(a.nbx, ctas);
+    const int owned = deal.nox * deal.noy;
+    // the hot blocks' candidates, a part per warp; the PSF blocks' largest |value|
+    unsigned long long* parts = reinterpret_cast<unsigned long long*>(lead_smem + sizeof(LeadShared));
+    float* pmax = reinterpret_cast<float*>(parts + owned * kLeadGroup);
+    for (int i = tid; i < owned; i += kLeadThreads) {
+        const int x = deal.x(i, rank), y = deal.y(i, rank, ctas);
+        const bool in = x < a.nbx && y < a.nbx;
+        sh.bound[i] = in ? a.bound[y * a.nbx + x] : 0.f;
+        sh.applied[i] = in ? a.applied[y * a.nbx + x] : 0;
+        sh.at[i] = in ? unsigned(y) << (16 + a.lb) | unsigned(x) << a.lb : 0xffffffffu;
+    }
+    for (int i = tid; i < it0 - base; i += kLeadThreads) sh.ring[i] = a.ring[i];
+    for (int i = tid; i < a.npx * a.npx; i += kLeadThreads) pmax[i] = a.pmax[i];
+    if (rank == 0 && tid == 0) st->nwarm = 0;
+    if (tid == 0) {
+        sh.nhot[0] = sh.nhot[1] = 0;
+        for (int p = 0; p < 2; ++p)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh.arrived[p])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const int px = int(st->psf_pos % unsigned(P)), py = int(st->psf_pos / unsigned(P));
+    const float at_peak = a.h.psf[size_t(px) * P + px];  // what an update takes t times of at its own peak
+    const unsigned int flat = key_index(st->win_key[0]);  // the scan's, or the last launch's last
+    int rx = int(flat % unsigned(W)), ry = int(flat / unsigned(W));
+    float peak = st->win_val[0];
+    // the model update of the last iteration, its load left in flight (one thread of the first CTA);
+    // the ring's entries are another thread's, both in warps that seldom have a block's bound
+    const bool models = rank == 0 && tid == kLeadThreads - 32, rings = tid == kLeadThreads - 64;
+    float m_old = 0.f, m_add = 0.f;
+    size_t m_pos = 0;
+    bool m_open = false;
+    unsigned long long skipped = 0;
+    int it = it0;
+    cluster.sync();  // every CTA runs (its shared memory is written to) and has read the state
+    for (; it < it1; ++it) {
+        const int par = it & 1;
+        if (fabsf(peak) < a.h.threshold) {  // every CTA holds the same winner: all stop here (HogbomGolden.cc:86-89)
+            if (rank == 0 && tid == 0) st->stopped = it + 1;
+            break;
+        }
+        const int diffx = rx - px, diffy = ry - px;  // diffy uses px, as the reference does
+        const float t = __fmul_rn(a.h.gain, peak), at = fabsf(t);
+        const float least = fabsf(__fsub_rn(peak, __fmul_rn(t, at_peak)));  // the peak's pixel after the update
+        if (tid == 0) {
+            sh.nhot[par ^ 1] = 0;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&sh.arrived[par])),
+                         "r"(ctas * 8) : "memory");
+        }
+        if (rings) {
+            const int startx = max(0, diffx), stopx = min(W - 1, rx + (P - px - 1));
+            const int starty = max(0, ry - py), stopy = min(W - 1, ry + (P - py - 1));
+            // rows whose PSF row lies inside the PSF (all of them unless its peak is off the diagonal)
+            const int ya = max(starty, diffy), yb = min(stopy, diffy + P - 1);
+            Update u;
+            u.t = t;
+            u.off = -(diffy * P + diffx);
+            u.xr = unsigned(startx) | (unsigned(stopx) << 16);
+            u.yr = yb >= ya ? unsigned(ya) | (unsigned(yb) << 16) : 1u;  // no row: first > last
+            sh.ring[it - base] = u;
+            if (rank == 0) a.ring[it - base] = u;
+            skipped += (unsigned long long)(stopy - starty + 1 - max(0, yb - ya + 1));
+        }
+        if (models) {  // model[absPeakPos] += absPeakVal * g_gain (HogbomGolden.cc:93)
+            if (m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
+            m_pos = size_t(ry) * W + rx;
+            m_add = __fmul_rn(peak, a.h.gain);
+            m_old = *reinterpret_cast<volatile float*>(a.h.model + m_pos);
+            m_open = true;
+            if (a.h.hist_val) a.h.hist_val[it] = peak;
+            if (a.h.hist_pos) a.h.hist_pos[it] = unsigned(m_pos);
+            st->done = it + 1;
+        }
+        for (int i = tid; i < owned; i += kLeadThreads) {
+            const unsigned int where = sh.at[i];
+            if (where == 0xffffffffu) continue;
+            const int bx = int(where & 0xffffu), by = int(where >> 16);
+            float bound = sh.bound[i];
+            // the PSF under the block (clipped to the PSF: where it ends nothing is subtracted)
+            const int u0 = max(0, bx - diffx), u1 = min(P - 1, bx + side - 1 - diffx);
+            const int v0 = max(0, by - diffy), v1 = min(P - 1, by + side - 1 - diffy);
+            if (u0 <= u1 && v0 <= v1) {
+                const int c0 = u0 >> a.lbp, c1 = u1 >> a.lbp;
+                const float *p0 = pmax + (v0 >> a.lbp) * a.npx, *p1 = pmax + (v1 >> a.lbp) * a.npx;
+                const float top = fmaxf(fmaxf(p0[c0], p0[c1]), fmaxf(p1[c0], p1[c1]));
+                bound = __fadd_ru(bound, __fmul_ru(at, top));
+                sh.bound[i] = bound;
+            }
+            if (!(bound < least)) {  // also when either is not a number
+                sh.hot[atomicAdd(&sh.nhot[par], 1)] = (unsigned short)(i);
+            }
+        }
+        __syncthreads();
+        const int nhot = sh.nhot[par];
+        lead_apply(a, sh, parts, nhot, base, it + 1);
+        __syncthreads();
+        if (warp == 0) {
+            unsigned long long c = 0;
+            for (int i = lane; i < nhot; i += 32) {
+                const int own = sh.hot[i];
+                unsigned long long k = parts[i * kLeadGroup];
+#pragma unroll
+                for (int j = 1; j < kLeadGroup; ++j) k = max(k, parts[i * kLeadGroup + j]);
+                sh.bound[own] = cand_abs(k);
+                sh.applied[own] = it + 1;
+                c = max(c, k);
+            }
+            c = warp_max(c);
+            // to every CTA of the cluster, each store counted by that CTA's barrier.  Two buffers
+            // suffice: a CTA sends iteration it + 2's after it has all of it + 1's, which the
+            // others sent having read it's.
+            if (lane < ctas) {
+                unsigned dst, bar;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_addr(&sh.cand[par][rank])), "r"(lane));
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_addr(&sh.arrived[par])), "r"(lane));
+                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(dst), "l"(c),
+                             "r"(bar) : "memory");
+            }
+        }
+        // this parity's barrier completes once per two iterations of this launch
+        const unsigned phase = unsigned((it - it0) >> 1) & 1u;
+        bool here = false;
+        for (unsigned spin = 0; spin < (1u << 22) && !here; ++spin) {
+            unsigned ok;
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                         " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(smem_addr(&sh.arrived[par])), "r"(phase) : "memory");
+            here = ok != 0;
+        }
+        if (!__syncthreads_and(here)) {  // not while the cluster's CTAs run: leave (tcv_hogbom_result says so)
+            st->error = 1;
+            break;
+        }
+        const unsigned long long c = warp_max(lane < ctas ? sh.cand[par][lane] : 0ull);
+        const bool zero = (c >> 33) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
+        const unsigned int idx = zero ? 0u : cand_index(c);
+        rx = int(idx & 0xffffu);
+        ry = int(idx >> 16);
+        peak = zero ? 0.f : cand_value(c);
+    }
+    cluster.sync();  // no CTA leaves while another's store to it may be under way
+    for (int i = tid; i < owned; i += kLeadThreads) {
+        if (sh.at[i] == 0xffffffffu) continue;
+        const int b = deal.y(i, rank, ctas) * a.nbx + deal.x(i, rank);
+        a.bound[b] = sh.bound[i];
+        a.applied[b] = sh.applied[i];
+        // near the peak: soon to be hot, and better without a long chain of updates to catch up on
+        if (sh.applied[i] < it && !(sh.bound[i] < 0.5f * fabsf(peak))) a.warm[atomicAdd(&st->nwarm, 1u)] = unsigned(b);
+    }
+    if (rank != 0) return;
+    if (models && m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
+    if (rings && skipped) st->skipped_rows += skipped;
+    if (tid == 0) {
+        st->win_key[0] = static_cast<unsigned int>(~(unsigned(ry) * unsigned(W) + unsigned(rx)));
+        st->win_val[0] = peak;
+    }
+    // this launch's updates: the last earlier one at the same place, a warp per update; then the
+    // batches and windows, on from the state of the last launch
+    __shared__ short prev[kLeadIters];
+    for (int j = warp; j < it - it0; j += kLeadWarps) {
+        const int q = it0 - base + j;
+        const Update u = sh.ring[q];
+        int last = -1;
+        for (int i = lane; i < q; i += 32) {
+            const Update o = sh.ring[i];
+            if (o.off == u.off && o.xr == u.xr && o.yr == u.yr) last = i;
+        }
+        last = __reduce_max_sync(0xffffffffu, last);
+        if (lane == 0) prev[j] = short(last);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int batch = it0 == base ? 0 : st->batch, used = it0 == base ? 0 : st->used;
+        for (int j = 0; j < it - it0; ++j) {
+            const int q = it0 - base + j, p = prev[j];
+            int slot;
+            if (p >= batch) {
+                slot = a.slots[p].slot;
+            } else {
+                if (used == kSlots) {
+                    batch = q;
+                    used = 0;
+                }
+                slot = used++;
+            }
+            a.slots[q] = UpdateSlot{short(p), short(slot), short(batch), 0};
+        }
+        st->batch = batch;
+        st->used = used;
+    }
+}
+
+// Apply what is pending to every block when `all`, else to those of the warm list.  A CTA works on
+// 32 x 16 pixels at a time; a lane keeps its four in registers and walks the updates in order.  The
+// PSF values it needs come from windows in shared memory, in which every lane copies
+// (asynchronously) and reads its own places only: updates at one peak share a window, so the
+// loads from L2 are one per distinct peak of a batch, not one per update, and an update of a pixel
+// costs 4 bytes from shared memory, a product and a difference.
+__global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, int base, int all)
+{
+    constexpr int kRows = kApplyRows;
+    static_assert(kRows == 4, "one float4 per lane and window");
+    extern __shared__ __align__(16) float apply_win[];  // [kSlots][kWindow]
+    __shared__ Update ring[kRing];
+    __shared__ UpdateSlot slots[kRing];
+    __shared__ float2 code[kRing];  // of the part's updates in order: -t and, as bits, the window
+    __shared__ unsigned short which[kRing], load[kSlots];  // ring entries: of the codes; to copy windows of
+    __shared__ unsigned short batch_end[kRing];
+    __shared__ int warps[2][kApplyThreads / 32];
+    __shared__ unsigned long long wk[kApplyThreads / 32];
+    const int to = a.h.state->done;
+    const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    const int W = a.h.width, P = a.h.psf_width, q1 = to - base, lsub = a.lb - 5;
+    const int count = all ? a.nbx * a.nbx : int(a.h.state->nwarm);
+    if (q1 <= 0 || count == 0) return;
+    for (int i = tid; i < q1; i += kApplyThreads) {
+        ring[i] = a.ring[i];
+        slots[i] = a.slots[i];
+        if (i + 1 == q1 || a.slots[i + 1].batch != a.slots[i].batch) batch_end[a.slots[i].batch] = (unsigned short)(i + 1);
+    }
+    float4* const mine = reinterpret_cast<float4*>(apply_win) + tid;  // this lane's place in the first window
+    for (int item = int(blockIdx.x); item < count; item += int(gridDim.x)) {
+        const int b = all ? item : int(a.warm[item]);
+        const int q0 = a.applied[b] - base;
+        if (q0 >= q1) continue;  // the same for the whole CTA, as all that follows but `rows`
+        unsigned long long best = 0;
+        for (int part = 0; part < kStrips << (2 * lsub); ++part) {
+            const int sub = part / kStrips;
+            const int x0 = ((b % a.nbx) << a.lb) + ((sub & ((1 << lsub) - 1)) << 5);
+            const int y0 = ((b / a.nbx) << a.lb) + ((sub >> lsub) << 5) + part % kStrips * (32 / kStrips);
+            if (x0 >= W || y0 >= W) continue;
+            const int x = x0 + lane, y = y0 + warp * kRows;
+            const int rows = x < W ? min(kRows, W - y) : 0;  // this lane's (none past the image)
+            float* rp = a.h.residual + (size_t(y) * W + x);
+            float r[kRows];
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) r[k] = k < rows ? __ldcs(rp + size_t(k) * W) : 0.f;
+            const float* __restrict__ pp = a.h.psf + (ptrdiff_t(y) * P + x);
+            for (int first = q0; first < q1;) {
+                __syncthreads();  // ring and slots are there; the last batch's codes are used
+                const int end = batch_end[slots[first].batch];
+                // the batch's updates that reach these pixels, in order, and those whose window is to
+                // be copied (no earlier one of the batch has it)
+                int n = 0, nc = 0;
+                bool partial = false;
+                for (int i0 = first; i0 < end; i0 += kApplyThreads) {
+                    const int i = i0 + tid;
+                    const int cover = i < end ? cover_of(ring[i], x0, y0, 32 / kStrips) : 0;
+                    const bool copy = cover && slots[i].prev < first;
+                    const unsigned bu = __ballot_sync(0xffffffffu, cover != 0), bc = __ballot_sync(0xffffffffu, copy);
+                    if (lane == 0) {
+                        warps[0][warp] = __popc(bu);
+                        warps[1][warp] = __popc(bc);
+                    }
+                    partial |= __syncthreads_or(cover == 1) != 0;
+                    int at = n, atc = nc;
+#pragma unroll
+                    for (int w = 0; w < kApplyThreads / 32; ++w) {
+                        if (w == warp) {
+                            at = n;
+                            atc = nc;
+                        }
+                        n += warps[0][w];
+                        nc += warps[1][w];
+                    }
+                    if (cover) {
+                        at += __popc(bu & ((1u << lane) - 1u));
+                        code[at] = make_float2(-ring[i].t, __int_as_float(int(slots[i].slot) * kApplyThreads));
+                        which[at] = (unsigned short)(i);
+                    }
+                    if (copy) load[atc + __popc(bc & ((1u << lane) - 1u))] = (unsigned short)(i);
+                    __syncthreads();
+                }
+                for (int i = 0; i < nc; ++i) {
+                    const int e = load[i];
+                    const Update u = ring[e];
+                    float* w = reinterpret_cast<float*>(mine + int(slots[e].slot) * kApplyThreads);
+                    const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
+                    const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
+#pragma unroll
+                    for (int k = 0; k < kRows; ++k)
+                        if (cx && y + k >= ya && y + k <= yb)
+                            __pipeline_memcpy_async(w + k, pp + (u.off + ptrdiff_t(k) * P), 4);
+                }
+                __pipeline_commit();
+                __pipeline_wait_prior(0);  // a lane reads only what it copied: no barrier
+                if (!partial) {
+                    // r + (-t) p is r - t p, bit for bit (the sums one by one: a paired product and a
+                    // paired sum would be contracted into one rounding)
+#pragma unroll 8
+                    for (int i = 0; i < n; ++i) {
+                        const float2 cd = code[i], nt = make_float2(cd.x, cd.x);
+                        const float4 w = mine[__float_as_int(cd.y)];
+                        const float2 s = __fmul2_rn(nt, make_float2(w.x, w.y)), v = __fmul2_rn(nt, make_float2(w.z, w.w));
+                        r[0] = __fadd_rn(r[0], s.x);
+                        r[1] = __fadd_rn(r[1], s.y);
+                        r[2] = __fadd_rn(r[2], v.x);
+                        r[3] = __fadd_rn(r[3], v.y);
+                    }
+                } else {
+                    for (int i = 0; i < n; ++i) {
+                        const float2 cd = code[i];
+                        const Update u = ring[which[i]];
+                        const float* w = reinterpret_cast<const float*>(mine + __float_as_int(cd.y));
+                        const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
+                        const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
+#pragma unroll
+                        for (int k = 0; k < kRows; ++k)
+                            if (cx && y + k >= ya && y + k <= yb) r[k] = __fadd_rn(r[k], __fmul_rn(cd.x, w[k]));
+                    }
+                }
+                first = end;
+            }
+            float top = -1.f, tv = 0.f;
+            int ty = 0;
+#pragma unroll
+            for (int k = 0; k < kRows; ++k)
+                if (k < rows) {
+                    __stcs(rp + size_t(k) * W, r[k]);
+                    if (fabsf(r[k]) > top) {
+                        top = fabsf(r[k]);
+                        tv = r[k];
+                        ty = y + k;
+                    }
+                }
+            best = max(best, top < 0.f ? 0ull : cand_key(tv, x, ty));
+        }
+        best = warp_max(best);
+        if (lane == 0) wk[warp] = best;
+        __syncthreads();
+        if (tid == 0) {
+            for (int i = 1; i < kApplyThreads / 32; ++i) best = max(best, wk[i]);
+            a.bound[b] = cand_abs(best);
+            a.applied[b] = to;
+        }
     }
 }
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// residual + PSF bytes up to which the persistent kernel is chosen (they stay in the 126 MB L2)
-constexpr size_t kPersistBytes = size_t(48) << 20;
 int g_hog_strategy = TCV_HOGBOM_AUTO;
 constexpr unsigned long long kDefaultWaitNs = 2000000000ull;  // 2 s
 unsigned long long g_wait_ns = kDefaultWaitNs;
@@ -407,6 +1170,208 @@ int hog_blocks(long long n)
     return int(std::max<long long>(1, std::min<long long>(kHogMaxBlocks, want)));
 }
 
+// log2 of the block side that covers `width` pixels with at most kBlkSide blocks (32 at least)
+int log2_side(int width)
+{
+    int lb = 5;
+    while ((width + (1 << lb) - 1) >> lb > kBlkSide) ++lb;
+    return lb;
+}
+
+// the workspace: state and the clusters' posted candidates (zeroed per call), candidates of the
+// scans, then what put-off updates need
+struct HogWork {
+    HogState* state;
+    unsigned long long *keys, *post;
+    float* vals;
+    float *bound, *pmax;
+    int* applied;
+    unsigned int* warm;
+    Update* ring;
+    UpdateSlot* slots;
+    size_t zeroed, total;
+    explicit HogWork(void* w)
+    {
+        char* q = static_cast<char*>(w);
+        auto take = [&](size_t bytes) {
+            char* r = q;
+            q += align256(bytes);
+            return static_cast<void*>(r);
+        };
+        state = static_cast<HogState*>(take(sizeof(HogState)));
+        post = static_cast<unsigned long long*>(take(size_t(2) * kResClusters * 2 * 8));
+        zeroed = size_t(q - static_cast<char*>(w));
+        keys = static_cast<unsigned long long*>(take(size_t(kHogMaxBlocks) * 8));
+        vals = static_cast<float*>(take(size_t(kHogMaxBlocks) * 4));
+        bound = static_cast<float*>(take(size_t(kBlkMax) * 4));
+        pmax = static_cast<float*>(take(size_t(kBlkMax) * 4));
+        applied = static_cast<int*>(take(size_t(kBlkMax) * 4));
+        warm = static_cast<unsigned int*>(take(size_t(kBlkMax) * 4));
+        ring = static_cast<Update*>(take(size_t(kRing) * sizeof(Update)));
+        slots = static_cast<UpdateSlot*>(take(size_t(kRing) * sizeof(UpdateSlot)));
+        total = size_t(q - static_cast<char*>(w));
+    }
+};
+
+// Scans of the PSF and of the dirty image that the one-pass kernels and the resident kernel start from:
+// the PSF's peak (HogbomGolden.cc:73-76), then residual = dirty with the first scan (:70).
+tcv_status first_scans(const HogArgs& a, const float* dirty, cudaStream_t st)
+{
+    const long long np = (long long)a.psf_width * a.psf_width;
+    const int pb = hog_blocks(np), nb = hog_blocks(a.n);
+    hog_scan_kernel<<<pb, kHogThreads, 0, st>>>(a.psf, nullptr, np, pb, a.keys, a.vals, a.state, 2);
+    TCV_CUDA(cudaGetLastError());
+    hog_scan_kernel<<<nb, kHogThreads, 0, st>>>(dirty, a.residual, a.n, nb, a.keys, a.vals, a.state, 0);
+    TCV_CUDA(cudaGetLastError());
+    return TCV_OK;
+}
+
+using ResKernel = void (*)(ResArgs, int, unsigned long long, unsigned int);
+
+template <int kRowsT>
+ResKernel resident_of(int chunks)
+{
+    switch (chunks) {
+        case 1: return hog_resident_kernel<kRowsT, 1>;
+        case 2: return hog_resident_kernel<kRowsT, 2>;
+        case 3: return hog_resident_kernel<kRowsT, 3>;
+        default: return hog_resident_kernel<kRowsT, 4>;
+    }
+}
+
+// All iterations with the residual in registers, in one cooperative launch of clusters.  ran = false:
+// the image does not fit (or the device cannot hold the clusters), nothing launched.
+tcv_status deconvolve_resident(const HogArgs& h, const HogWork& w, const float* dirty, int niters, cudaStream_t st, bool& ran)
+{
+    ran = false;
+    const int W = h.width;
+    if (W > kResChunks * kResThreads || h.psf_width > 65535) return TCV_OK;
+    int dev = 0, coop = 0;
+    TCV_CUDA(cudaGetDevice(&dev));
+    TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return TCV_OK;
+    const int chunks = (W + kResThreads - 1) / kResThreads;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kResThreads);
+    cfg.attrs = attr;
+    cfg.stream = st;
+    for (int rows_t : {4, 8, 16}) {
+        const ResKernel kernel = rows_t == 4 ? resident_of<4>(chunks) : rows_t == 8 ? resident_of<8>(chunks) : resident_of<16>(chunks);
+        // clusters of 16 where they fit: half as many meet as of 8 (300^2: 1.80 us an iteration, not 1.91)
+        int size = 16, most = 0;
+        cfg.dynamicSmemBytes = size_t(rows_t - res_direct(rows_t, chunks)) * chunks * kResThreads * sizeof(float);
+        if (cfg.dynamicSmemBytes)
+            TCV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cfg.dynamicSmemBytes)));
+        for (; size >= 8; size /= 2) {
+            attr[0].val.clusterDim.x = unsigned(size);
+            cfg.gridDim = dim3(unsigned(size));
+            cfg.numAttrs = 1;
+            if ((size == 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) == cudaSuccess && most > 0)
+                break;
+            cudaGetLastError();
+            most = 0;
+        }
+        most = std::min(most, kResClusters);
+        // rows per CTA: at least four, so that small images meet in few clusters
+        const int rows = std::max(4, (W + most * size - 1) / std::max(1, most * size));
+        if (most < 1 || rows > rows_t) continue;
+        TCV_CHECK(first_scans(h, dirty, st));
+        ran = true;
+        if (niters == 0) return TCV_OK;
+        ResArgs a{h, w.post, rows};
+        const int ctas = (W + rows - 1) / rows;
+        cfg.gridDim = dim3(unsigned((ctas + size - 1) / size * size));
+        cfg.numAttrs = 2;
+        TCV_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, niters, g_wait_ns, g_withheld));
+        return TCV_OK;
+    }
+    return TCV_OK;
+}
+
+// CTAs of the leading cluster: 16 where one such cluster can be resident, else 8, else 0
+int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArgs& a)
+{
+    constexpr size_t kMost =
+        sizeof(LeadShared) + size_t(kBlkMax) / 8 * kLeadGroup * sizeof(unsigned long long) + size_t(kBlkMax) * sizeof(float);
+    static_assert(kMost <= 227 * 1024, "shared memory of a CTA");
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg = cudaLaunchConfig_t{};
+    cfg.blockDim = dim3(kLeadThreads);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(hog_lead_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        cudaGetLastError();
+    if (cudaFuncSetAttribute(hog_lead_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMost)) != cudaSuccess)
+        return 0;
+    for (int n : {kLeadCtas, 8}) {
+        const LeadDeal deal(a.nbx, n);
+        cfg.dynamicSmemBytes = sizeof(LeadShared) + size_t(deal.nox) * deal.noy * kLeadGroup * sizeof(unsigned long long) +
+                               size_t(a.npx) * a.npx * sizeof(float);
+        attr.val.clusterDim.x = unsigned(n);
+        cfg.gridDim = dim3(unsigned(n));
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, hog_lead_kernel, &cfg) == cudaSuccess && clusters > 0) return n;
+        cudaGetLastError();
+    }
+    return 0;
+}
+
+// All iterations with put-off updates.  false: the device cannot hold the cluster, nothing launched.
+tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* dirty, int niters, cudaStream_t st, bool& ran)
+{
+    ran = false;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    DeferArgs a{};
+    a.h = h;
+    a.bound = w.bound;
+    a.applied = w.applied;
+    a.warm = w.warm;
+    a.pmax = w.pmax;
+    a.ring = w.ring;
+    a.slots = w.slots;
+    a.lb = log2_side(h.width);
+    a.nbx = (h.width + (1 << a.lb) - 1) >> a.lb;
+    a.lbp = std::max(a.lb, log2_side(h.psf_width));  // a block then lies on at most 2 x 2 of the PSF's
+    a.npx = (h.psf_width + (1 << a.lbp) - 1) >> a.lbp;
+    if (!lead_ctas(cfg, attr, a)) return TCV_OK;
+    cfg.stream = st;
+    const int nb = a.nbx * a.nbx;
+    auto scan_ctas = [](int blocks) { return std::min(kHogMaxBlocks, (blocks + kHogThreads / 32 - 1) / (kHogThreads / 32)); };
+    // the PSF's peak (HogbomGolden.cc:73-76), then residual = dirty with the first scan (:70)
+    hog_blocks_kernel<<<scan_ctas(a.npx * a.npx), kHogThreads, 0, st>>>(h.psf, nullptr, h.psf_width, a.lbp, a.npx, w.pmax,
+                                                                        nullptr, h.keys, h.vals, h.state, 2);
+    TCV_CUDA(cudaGetLastError());
+    hog_blocks_kernel<<<scan_ctas(nb), kHogThreads, 0, st>>>(dirty, h.residual, h.width, a.lb, a.nbx, w.bound, w.applied,
+                                                             h.keys, h.vals, h.state, 0);
+    TCV_CUDA(cudaGetLastError());
+    const size_t win = size_t(kSlots) * kWindow * sizeof(float);
+    TCV_CUDA(cudaFuncSetAttribute(hog_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(win)));
+    int dev = 0, sms = 0, per_sm = 0;
+    TCV_CUDA(cudaGetDevice(&dev));
+    TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_apply_kernel, kApplyThreads, win));
+    const int most = std::min(nb, sms * std::max(1, per_sm));
+    for (int it = 0, base = 0; it < niters; it += kLeadIters) {
+        const int to = std::min(niters, it + kLeadIters);
+        TCV_CUDA(cudaLaunchKernelEx(&cfg, hog_lead_kernel, a, it, to, base));
+        const int all = to == niters || to - base == kRing;
+        hog_apply_kernel<<<most, kApplyThreads, win, st>>>(a, base, all);
+        TCV_CUDA(cudaGetLastError());
+        if (all) base = to;
+    }
+    ran = true;
+    return TCV_OK;
+}
+
+
 }  // namespace
 }  // namespace tcv
 
@@ -417,7 +1382,7 @@ extern "C" {
 size_t tcv_hogbom_workspace_bytes(int width)
 {
     if (width < 1) return 0;
-    return align256(sizeof(HogState)) + 2 * align256(size_t(kHogMaxBlocks) * 8) + 2 * align256(size_t(kHogMaxBlocks) * 4);
+    return HogWork(nullptr).total;
 }
 
 tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d_psf, int psf_width, float* d_model,
@@ -430,17 +1395,11 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
         return TCV_ERR_UNSUPPORTED;
     if (work_bytes < tcv_hogbom_workspace_bytes(width)) return TCV_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    char* w = static_cast<char*>(d_work);
+    const HogWork w(d_work);
     HogArgs a{};
-    a.state = reinterpret_cast<HogState*>(w);
-    {
-        char* q = w + align256(sizeof(HogState));
-        a.keys = reinterpret_cast<unsigned long long*>(q);
-        a.keys2 = reinterpret_cast<unsigned long long*>(q + align256(size_t(kHogMaxBlocks) * 8));
-        q += 2 * align256(size_t(kHogMaxBlocks) * 8);
-        a.vals = reinterpret_cast<float*>(q);
-        a.vals2 = reinterpret_cast<float*>(q + align256(size_t(kHogMaxBlocks) * 4));
-    }
+    a.state = w.state;
+    a.keys = w.keys;
+    a.vals = w.vals;
     a.psf = d_psf;
     a.residual = d_residual;
     a.model = d_model;
@@ -452,44 +1411,15 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     a.nblocks = hog_blocks(a.n);
     a.gain = gain;
     a.threshold = threshold;
-    a.wait_ns = g_wait_ns;
-    a.withheld = g_withheld;
-    TCV_CUDA(cudaMemsetAsync(a.state, 0, sizeof(HogState), st));
-    // the PSF's peak (HogbomGolden.cc:73-76), then residual = dirty with the first scan (:70)
-    const long long np = (long long)psf_width * psf_width;
-    const int pb = hog_blocks(np);
-    hog_scan_kernel<<<pb, kHogThreads, 0, st>>>(d_psf, nullptr, np, pb, a.keys, a.vals, a.state, 2);
-    TCV_CUDA(cudaGetLastError());
-    hog_scan_kernel<<<a.nblocks, kHogThreads, 0, st>>>(d_dirty, d_residual, a.n, a.nblocks, a.keys, a.vals, a.state, 0);
-    TCV_CUDA(cudaGetLastError());
+    TCV_CUDA(cudaMemsetAsync(a.state, 0, w.zeroed, st));
+    bool ran = false;
+    tcv_status s = TCV_OK;
+    if (g_hog_strategy != TCV_HOGBOM_PER_LAUNCH) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
+    if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_AUTO && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
+        s = deconvolve_deferred(a, w, d_dirty, niters, st, ran);
+    if (s != TCV_OK || ran) return s;
+    TCV_CHECK(first_scans(a, d_dirty, st));
     const bool vec = width % 4 == 0 && reinterpret_cast<uintptr_t>(d_residual) % 16 == 0;
-    // images whose residual and PSF sit in L2 run every iteration in one cooperative launch
-    const size_t resident = size_t(a.n) * 4 + size_t(np) * 4;
-    bool persist = g_hog_strategy == TCV_HOGBOM_PERSISTENT ||
-                   (g_hog_strategy == TCV_HOGBOM_AUTO && resident <= kPersistBytes);
-    int dev = 0, coop = 0, sms = 0, per_sm = 0;
-    if (persist) {
-        TCV_CUDA(cudaGetDevice(&dev));
-        TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        if (vec)
-            TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_persist_kernel<true>, kHogThreads, 0));
-        else
-            TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_persist_kernel<false>, kHogThreads, 0));
-        persist = coop && per_sm > 0;
-    }
-    // the persistent loop's arrival count reaches niters x CTAs: keep it within 32 bits
-    if (persist && uint64_t(niters) * uint64_t(std::max(1, sms * 2)) >= (1ull << 32)) persist = false;
-    if (persist && niters > 0) {
-        // two CTAs per SM at most (fewer candidates per barrier), never more than resident
-        a.nblocks = std::max(1, std::min({sms * std::min(per_sm, 2), hog_blocks(a.n), width}));
-        int n_it = niters;
-        void* args[] = {&a, &n_it};
-        TCV_CUDA(cudaLaunchCooperativeKernel(vec ? reinterpret_cast<const void*>(hog_persist_kernel<true>)
-                                                 : reinterpret_cast<const void*>(hog_persist_kernel<false>),
-                                             dim3(unsigned(a.nblocks)), dim3(kHogThreads), args, 0, st));
-        return TCV_OK;
-    }
     for (int it = 0; it < niters; ++it) {
         if (vec)
             hog_iter_kernel<true><<<a.nblocks, kHogThreads, 0, st>>>(a, it);
@@ -534,10 +1464,10 @@ tcv_status tcv_find_peak(const float* d_image, int64_t n, float* val_out, int64_
     if (!d_image || n < 1 || !d_work || n >= int64_t(0xffffffffll)) return TCV_ERR_ARG;
     if (work_bytes < tcv_hogbom_workspace_bytes(1)) return TCV_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    char* w = static_cast<char*>(d_work);
-    HogState* state = reinterpret_cast<HogState*>(w);
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(w + align256(sizeof(HogState)));
-    float* vals = reinterpret_cast<float*>(w + align256(sizeof(HogState)) + 2 * align256(size_t(kHogMaxBlocks) * 8));
+    const HogWork w(d_work);
+    HogState* state = w.state;
+    unsigned long long* keys = w.keys;
+    float* vals = w.vals;
     TCV_CUDA(cudaMemsetAsync(state, 0, sizeof(HogState), st));
     const int nb = hog_blocks(n);
     hog_scan_kernel<<<nb, kHogThreads, 0, st>>>(d_image, nullptr, n, nb, keys, vals, state, 0);

@@ -580,23 +580,25 @@ tcv_status tcv_hogbom_deconvolve(const float *d_dirty, int width, const float *d
                                  float *d_model, float *d_residual, int niters, float gain,
                                  float threshold, float *d_hist_val, uint32_t *d_hist_pos,
                                  void *d_work, size_t work_bytes, void *stream);
-/* How tcv_hogbom_deconvolve issues the iterations (process-wide): AUTO (default) runs images
- * whose residual and PSF fit in 48 MiB as one cooperative launch of all iterations (CTAs meet at a
- * bounded grid barrier per iteration) and larger ones as one launch per iteration; the other two
- * force either form.  Results are identical. */
+/* How tcv_hogbom_deconvolve issues the iterations (process-wide): AUTO (default) runs images of up
+ * to 2048 x 2048 as one cooperative launch of all iterations with the residual in registers (the
+ * CTAs meet once per iteration, with bounded waits) and larger ones with updates put off until a
+ * block of pixels could hold the next peak (a launch of one cluster and a device-wide one per 16
+ * iterations; images or PSFs over 16384 wide take one launch per iteration).  PERSISTENT takes the
+ * cooperative form where the image fits it, PER_LAUNCH one launch per iteration; both otherwise
+ * the latter.  Results are identical. */
 enum { TCV_HOGBOM_AUTO = 0, TCV_HOGBOM_PER_LAUNCH = 1, TCV_HOGBOM_PERSISTENT = 2 };
 void tcv_hogbom_set_strategy(int strategy);
 /* The bounded waits of the cooperative form (process-wide, for launches made after the call):
- * limit_ns caps one grid-barrier wait (default and maximum 2e9 ns); withheld_arrivals (default 0)
- * raises every barrier's arrival target by that many CTAs that never arrive, so that every wait
- * runs out: a host-side hook that exercises the timeout path (the loop stops, every CTA returns,
+ * limit_ns caps one wait (default and maximum 2e9 ns); withheld_arrivals (default 0) makes the
+ * CTAs wait for that many more candidates than are ever posted, so that every wait runs out: a host-side hook that exercises the timeout path (the loop stops, every CTA returns,
  * tcv_hogbom_result reports TCV_ERR_TIMEOUT) without faulting or hanging the GPU.  Restore (2e9, 0)
  * afterwards.  The device-side counterpart of the reference's error accounting, which counts
  * disagreeing values instead of failing (attic/tConvolveBurnIn/tConvolveBurnIn.cc:94-107). */
 tcv_status tcv_hogbom_set_wait(uint64_t limit_ns, uint32_t withheld_arrivals);
 /* After tcv_hogbom_deconvolve (synchronises): iterations done, the iteration that met the
  * threshold (-1 if none), PSF rows skipped, the PSF peak index.  Any output may be NULL.
- * TCV_ERR_TIMEOUT if a grid-barrier wait of the persistent form gave up (the loop stopped). */
+ * TCV_ERR_TIMEOUT if a wait of the cooperative form gave up (the loop stopped). */
 tcv_status tcv_hogbom_result(const void *d_work, int *iters_done, int *stopped_at,
                              int64_t *skipped_rows, int64_t *psf_peak_pos, void *stream);
 /* findPeak (HogbomGolden.cc:127-139): the value of largest magnitude and its first index
