@@ -561,6 +561,10 @@ tcv_status launch_dense_grid(const tcv_plan* p, const float2* data, const void* 
     const typename Tab::elem* tab = static_cast<const typename Tab::elem*>(c);
     const unsigned int* order = p->vals[p->sel];
     const int4* grec = p->grec;
+    if (g.uniq) {  // the lists are of footprints: each one's data summed first
+        TCV_CHECK(uniq_sum(p, data, st));
+        data = p->usums;
+    }
     for (int grp = 0; grp < g.n_groups; ++grp) {
         GridArgs a = dense_args(p, grp, c_scale, grid);
         void* args[] = {const_cast<float2**>(&data), const_cast<unsigned int**>(&order), &tab, &grec,
@@ -592,13 +596,13 @@ tcv_status launch_dense_degrid(const tcv_plan* p, const float2* grid, const void
                         const_cast<uint32_t**>(&p->d_group_ustart), const_cast<float2**>(&p->slots), &max_tiles, &a};
         TCV_CUDA(cudaLaunchKernel(kernel, dim3(ctas), dim3(kDThreads), args, 0, st));
     }
-    return slot_reduce(p, c_scale, out, st);
+    return g.uniq ? uniq_slots(p, c_scale, out, st) : slot_reduce(p, c_scale, out, st);
 }
 
 tcv_status gather_pair_records(const tcv_plan* p, cudaStream_t st)
 {
     const PlanGeom& g = p->g;
-    if (!p->grec || g.n == 0) return TCV_OK;
+    if (!p->grec || g.n == 0 || g.uniq) return TCV_OK;  // (uniq_bin writes them)
     pair_records_kernel<<<unsigned(8 * sm_count()), 256, 0, st>>>(p->units, p->group_ustart, g.n_groups, p->vals[p->sel],
                                                                   p->iu, p->iv, p->coff, g.var ? p->ssz : nullptr, g.s,
                                                                   p->grec);

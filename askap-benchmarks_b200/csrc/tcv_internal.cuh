@@ -62,6 +62,10 @@ struct PlanGeom {
     // variable-width plans (one footprint width per w-plane; s and support are the widest)
     bool var;
     int n_planes;
+    // variable-width plans whose both passes are sample-parallel: binned by distinct footprint
+    // (tcv_unique.cu); bits of the sort key and of its table-offset and width-rank fields
+    bool uniq;
+    int u_bits, u_coff_bits, u_rank_bits;
 };
 
 }  // namespace tcv
@@ -122,6 +126,19 @@ struct tcv_plan {
     // first row, cOffset, width), gathered once per binning (nullptr unless a pass uses them)
     int4* grec;
     std::vector<int32_t> host_plane_s, host_plane_grp;
+    // plans binned by distinct footprint: order, slots, ntl and grec are of footprints, and
+    int32_t* plane_rank;           // per plane: its width among the distinct widths
+    std::vector<int32_t> host_plane_rank;
+    uint64_t* ukeys[2];            // sort keys, n
+    uint32_t* uvals[2];            // sample indices
+    int usel;                      // which of uvals is sorted: the samples of footprint after footprint
+    uint32_t* usum;                // per sorted sample: footprints up to it
+    int4* urec;                    // per footprint: first column, first row, cOffset, width
+    uint32_t* ufirst;              // per footprint: its first sorted sample
+    uint32_t* repu;                // per sample: its footprint (all ones: left out)
+    float2* usums;                 // per footprint: its samples' data, summed for a gridding pass
+    uint32_t* ucell;               // per cell: list length; first and end footprint that starts in it
+    uint32_t* n_uniq;              // [0] footprints; [1], [2] work-unit sizes in footprints
 };
 
 namespace tcv {
@@ -169,6 +186,12 @@ tcv_status launch_dense_grid(const tcv_plan* p, const float2* data, const void* 
 template <class Tab>
 tcv_status launch_dense_degrid(const tcv_plan* p, const float2* grid, const void* c, float c_scale, float2* out,
                                cudaStream_t st);
+// Plans binned by distinct footprint (tcv_unique.cu): the binning up to the cells' ranges, the sums of
+// the footprints' data before a gridding pass, the samples' values after a degridding pass.
+size_t uniq_temp_bytes(const PlanGeom& g);
+tcv_status uniq_bin(tcv_plan* p, cudaStream_t st);
+tcv_status uniq_sum(const tcv_plan* p, const float2* data, cudaStream_t st);
+tcv_status uniq_slots(const tcv_plan* p, float c_scale, float2* out, cudaStream_t st);
 // fill p->grec from the sorted pairs (after each binning of a plan that has it)
 tcv_status gather_pair_records(const tcv_plan* p, cudaStream_t st);
 // fold_kernel<8> over one plane group of a plan (the partial tiles of its split cells)

@@ -296,6 +296,7 @@ struct CellArgs {
     uint32_t cells, ntiles, split, dsplit;
     int n_groups;
     bool own_d;
+    const uint32_t* sizes;  // plans binned by footprint: split and dsplit, made on the device (else null)
     uint32_t* part;  // [kCellVals][blocks] block sums, scanned in place, then the kCellVals totals
     uint32_t *tile_start, *items, *n_items, *group_start;
     uint32_t *nunits, *ustart, *pstart, *group_ustart;
@@ -309,8 +310,9 @@ __device__ __forceinline__ uint32_t units_of(uint32_t cnt, uint32_t split)
     return cnt == 0 ? 0u : ((split && cnt >= 2u * split) ? cnt / split : 1u);
 }
 
-__device__ __forceinline__ void cell_vals(uint32_t cnt, uint32_t split, uint32_t dsplit, uint32_t* v)
+__device__ __forceinline__ void cell_vals(uint32_t cnt, const CellArgs& a, uint32_t* v)
 {
+    const uint32_t split = a.sizes ? a.sizes[0] : a.split, dsplit = a.sizes ? a.sizes[1] : a.dsplit;
     const uint32_t nu = units_of(cnt, split), dnu = units_of(cnt, dsplit);
     v[0] = cnt;
     v[1] = cnt ? 1u : 0u;
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(kCellThreads) cell_sums_kernel(CellArgs a)
 #pragma unroll
     for (int e = 0; e < kCellPer; ++e) {
         uint32_t v[kCellVals];
-        cell_vals(cnt[e], a.split, a.dsplit, v);
+        cell_vals(cnt[e], a, v);
 #pragma unroll
         for (int j = 0; j < kCellVals; ++j) s[j] += v[j];
     }
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(kCellThreads) cell_out_kernel(CellArgs a)
 #pragma unroll
     for (int e = 0; e < kCellPer; ++e) {
         uint32_t v[kCellVals];
-        cell_vals(cnt[e], a.split, a.dsplit, v);
+        cell_vals(cnt[e], a, v);
 #pragma unroll
         for (int j = 0; j < kCellVals; ++j) s[j] += v[j];
     }
@@ -464,7 +466,7 @@ __global__ void __launch_bounds__(kCellThreads) cell_out_kernel(CellArgs a)
         const uint32_t c = c0 + e;
         if (c >= a.cells) break;
         uint32_t v[kCellVals];
-        cell_vals(cnt[e], a.split, a.dsplit, v);
+        cell_vals(cnt[e], a, v);
         a.tile_start[c] = pre[0];
         a.tile_count[c] = cnt[e];
         if (c % a.ntiles == 0) {
@@ -518,6 +520,7 @@ inline size_t cell_scratch_bytes(const PlanGeom& g) { return (size_t(cell_blocks
 template <typename K>
 size_t cub_temp_bytes(const PlanGeom& g)
 {
+    if (g.uniq) return std::max(uniq_temp_bytes(g), cell_scratch_bytes(g));
     size_t a = 0, b = 0, c = 0, d = 0, f = 0;
     const int64_t np = g.n * g.max_tiles;
     const int acells = int(anchor_cells(g));
@@ -589,6 +592,39 @@ tcv_status plan_anchors_ready(const tcv_plan* cp, cudaStream_t st)
     return s;
 }
 
+// The cells' bookkeeping from their ranges (tile_start: starts, tile_count: ends).
+tcv_status cells_and_units(tcv_plan* p, cudaStream_t st)
+{
+    const PlanGeom& g = p->g;
+    const bool own_d = own_degrid_units(g);
+    const CellArgs ca{p->tile_count, uint32_t(grid_cells(g)), uint32_t(g.ntiles), uint32_t(g.split), uint32_t(g.dsplit),
+                      g.n_groups, own_d, g.uniq ? p->n_uniq + 1 : nullptr, static_cast<uint32_t*>(p->cub_temp),
+                      p->tile_start, p->items, p->n_items, p->group_start, p->nunits, p->ustart, p->pstart,
+                      p->group_ustart, p->units, own_d ? p->d_nunits : nullptr, own_d ? p->d_ustart : nullptr,
+                      own_d ? p->d_pstart : nullptr, own_d ? p->d_group_ustart : nullptr, own_d ? p->d_units : nullptr};
+    const uint32_t cb = cell_blocks(g);
+    cell_sums_kernel<<<cb, kCellThreads, 0, st>>>(ca);
+    TCV_CUDA(cudaGetLastError());
+    cell_scan_kernel<<<1, 1024, 0, st>>>(ca, cb);
+    TCV_CUDA(cudaGetLastError());
+    cell_out_kernel<<<cb, kCellThreads, 0, st>>>(ca);
+    TCV_CUDA(cudaGetLastError());
+    return TCV_OK;
+}
+
+tcv_status build_uniq(tcv_plan* p, cudaStream_t st)
+{
+    const size_t cells = grid_cells(p->g);
+    TCV_CUDA(cudaMemsetAsync(p->tile_count, 0, sizeof(uint32_t) * cells, st));
+    TCV_CUDA(cudaMemsetAsync(p->tile_start, 0, sizeof(uint32_t) * cells, st));
+    TCV_CUDA(cudaMemsetAsync(p->rejected, 0, sizeof(unsigned long long), st));
+    TCV_CUDA(cudaMemsetAsync(p->status, 0, kStatusWords * sizeof(unsigned int), st));
+    TCV_CUDA(cudaMemsetAsync(p->n_uniq, 0, 3 * sizeof(uint32_t), st));
+    if (p->g.n > 0) TCV_CHECK(uniq_bin(p, st));
+    p->anchors_ready = false;
+    return cells_and_units(p, st);
+}
+
 // The anchor binning is made with the plan's only when the plan degrids by anchor tiles at that
 // time; otherwise the first anchor degridding makes it (plan_anchors_ready).
 template <typename K>
@@ -636,19 +672,7 @@ tcv_status build(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_
     } else {
         p->sel = 0;
     }
-    const bool own_d = own_degrid_units(g);
-    const CellArgs ca{p->tile_count, uint32_t(cells), uint32_t(g.ntiles), uint32_t(g.split), uint32_t(g.dsplit),
-                      g.n_groups, own_d, static_cast<uint32_t*>(p->cub_temp), p->tile_start, p->items, p->n_items,
-                      p->group_start, p->nunits, p->ustart, p->pstart, p->group_ustart, p->units,
-                      own_d ? p->d_nunits : nullptr, own_d ? p->d_ustart : nullptr, own_d ? p->d_pstart : nullptr,
-                      own_d ? p->d_group_ustart : nullptr, own_d ? p->d_units : nullptr};
-    const uint32_t cb = cell_blocks(g);
-    cell_sums_kernel<<<cb, kCellThreads, 0, st>>>(ca);
-    TCV_CUDA(cudaGetLastError());
-    cell_scan_kernel<<<1, 1024, 0, st>>>(ca, cb);
-    TCV_CUDA(cudaGetLastError());
-    cell_out_kernel<<<cb, kCellThreads, 0, st>>>(ca);
-    TCV_CUDA(cudaGetLastError());
+    TCV_CHECK(cells_and_units(p, st));
     if (with_anchors) TCV_CHECK(sort_anchors<K>(p, st));
     p->anchors_ready = with_anchors;
     // a captured binning without anchors may be replayed on new samples behind the host's back:
@@ -692,10 +716,25 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
         p->plane_s = static_cast<int32_t*>(take(size_t(g.n_planes) * 4));
         p->plane_grp = static_cast<int32_t*>(take(size_t(g.n_planes) * 4));
     }
-    p->keys[0] = take(np * ks);
-    p->keys[1] = take(np * ks);
+    p->keys[0] = take(g.uniq ? 0 : np * ks);
+    p->keys[1] = take(g.uniq ? 0 : np * ks);
     p->vals[0] = static_cast<uint32_t*>(take(np * 4));
-    p->vals[1] = static_cast<uint32_t*>(take(np * 4));
+    p->vals[1] = static_cast<uint32_t*>(take(g.uniq ? 0 : np * 4));
+    if (g.uniq) {
+        const size_t n = size_t(g.n);
+        p->plane_rank = static_cast<int32_t*>(take(size_t(g.n_planes) * 4));
+        p->ukeys[0] = static_cast<uint64_t*>(take(n * 8));
+        p->ukeys[1] = static_cast<uint64_t*>(take(n * 8));
+        p->uvals[0] = static_cast<uint32_t*>(take(n * 4));
+        p->uvals[1] = static_cast<uint32_t*>(take(n * 4));
+        p->usum = static_cast<uint32_t*>(take(n * 4));
+        p->urec = static_cast<int4*>(take(n * sizeof(int4)));
+        p->ufirst = static_cast<uint32_t*>(take((n + 1) * 4));
+        p->repu = static_cast<uint32_t*>(take(n * 4));
+        p->usums = static_cast<float2*>(take(n * sizeof(float2)));
+        p->ucell = static_cast<uint32_t*>(take(grid_cells(g) * 3 * 4));
+        p->n_uniq = static_cast<uint32_t*>(take(3 * 4));
+    }
     p->akeys[0] = take(an * ks);
     p->akeys[1] = take(an * ks);
     p->avals[0] = static_cast<uint32_t*>(take(an * 4));
@@ -754,6 +793,9 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
         TCV_CUDA(cudaMemcpyAsync(p->plane_s, p->host_plane_s.data(), size_t(g.n_planes) * 4, cudaMemcpyHostToDevice, st));
         TCV_CUDA(cudaMemcpyAsync(p->plane_grp, p->host_plane_grp.data(), size_t(g.n_planes) * 4,
                                  cudaMemcpyHostToDevice, st));
+        if (g.uniq)
+            TCV_CUDA(cudaMemcpyAsync(p->plane_rank, p->host_plane_rank.data(), size_t(g.n_planes) * 4,
+                                     cudaMemcpyHostToDevice, st));
     }
     return TCV_OK;
 }
@@ -893,7 +935,14 @@ size_t plan_bytes(const PlanGeom& g, size_t* cub_bytes_out)
     b += align_up(size_t(g.n_jobs) * sizeof(JobDesc)) + align_up(size_t(g.n_jobs + 1) * 4);
     b += align_up(size_t(g.ntiles) * 4) + align_up(size_t(g.n) * 2);
     if (g.var) b += align_up(size_t(g.n) * 2) + 2 * align_up(size_t(g.n_planes) * 4);
-    b += 2 * align_up(np * ks) + 2 * align_up(np * 4);
+    if (g.uniq) {
+        const size_t n = size_t(g.n);
+        b += align_up(np * 4) + align_up(size_t(g.n_planes) * 4) + 2 * align_up(n * 8) + 4 * align_up(n * 4) +
+             align_up(n * sizeof(int4)) + align_up((n + 1) * 4) + align_up(n * sizeof(float2)) +
+             align_up(grid_cells(g) * 3 * 4) + align_up(3 * 4);
+    } else {
+        b += 2 * align_up(np * ks) + 2 * align_up(np * 4);
+    }
     b += 2 * align_up(an * ks) + 2 * align_up(an * 4);
     const size_t cells = grid_cells(g), acells = anchor_cells(g);
     b += 3 * align_up(cells * 4) + align_up(4) + align_up(size_t(g.n_groups + 1) * 4);
@@ -908,6 +957,20 @@ size_t plan_bytes(const PlanGeom& g, size_t* cub_bytes_out)
     if (g.dense || g.ddense) b += align_up(np * sizeof(int4));  // pair records (tcv_dense.cu)
     b += align_up(cb);
     return b;
+}
+
+// How many distinct widths the planes have; ranks (may be null): each plane's among them.
+int width_ranks(const int32_t* s_size, int n_planes, std::vector<int32_t>* ranks)
+{
+    std::vector<int32_t> w(s_size, s_size + n_planes);
+    std::sort(w.begin(), w.end());
+    w.erase(std::unique(w.begin(), w.end()), w.end());
+    if (ranks) {
+        ranks->resize(size_t(n_planes));
+        for (int k = 0; k < n_planes; ++k)
+            (*ranks)[size_t(k)] = int32_t(std::lower_bound(w.begin(), w.end(), s_size[k]) - w.begin());
+    }
+    return int(w.size());
 }
 
 // Geometry of a variable-width plan: the widest plane sets the tile reach; whole planes are
@@ -940,6 +1003,13 @@ PlanGeom make_geom_var(int64_t n, const int32_t* s_size, const int32_t* c_off0, 
     g.tile_bits = bits_for(uint64_t(g.n_groups) * uint64_t(g.ntiles) - 1);
     g.key_bits = g.tile_bits + 1;
     g.key64 = g.key_bits > 32;
+    if (g.dense && g.ddense) {
+        // distinct footprints, where (cell, table offset, place in the 64 x 32 tile, width) fits a key
+        g.u_coff_bits = bits_for(uint64_t(c_len - 1));
+        g.u_rank_bits = bits_for(uint64_t(width_ranks(s_size, n_planes, nullptr) - 1));
+        g.u_bits = g.tile_bits + g.u_coff_bits + 11 + g.u_rank_bits;
+        g.uniq = g.u_bits < 64;
+    }
     return g;
 }
 
@@ -950,7 +1020,9 @@ tcv_status plan_bin(tcv_plan* p, const int32_t* d_iu, const int32_t* d_iv, const
     p->iu = d_iu;
     p->iv = d_iv;
     p->coff = d_coff;
-    tcv_status s = p->g.key64 ? build<uint64_t>(p, d_iu, d_iv, d_coff, st) : build<uint32_t>(p, d_iu, d_iv, d_coff, st);
+    tcv_status s = p->g.uniq    ? build_uniq(p, st)
+                   : p->g.key64 ? build<uint64_t>(p, d_iu, d_iv, d_coff, st)
+                                : build<uint32_t>(p, d_iu, d_iv, d_coff, st);
     if (s == TCV_OK && p->grec) s = gather_pair_records(p, st);
     p->binned = s == TCV_OK;
     return s;
@@ -989,6 +1061,7 @@ tcv_status plan_init_var(tcv_plan* p, const int32_t* d_iu, const int32_t* d_iv, 
     p->g = make_geom_var(n, s_size, c_off0, n_planes, g_size, c_len, t, p->host_plane_grp);
     if (!geom_supported(p->g)) return TCV_ERR_UNSUPPORTED;
     p->host_plane_s.assign(s_size, s_size + n_planes);
+    if (p->g.uniq) width_ranks(s_size, n_planes, &p->host_plane_rank);
     p->wplane = d_wplane;
     const tcv_status s = plan_create(p, d_work, work_bytes, st);
     if (s != TCV_OK) return s;
