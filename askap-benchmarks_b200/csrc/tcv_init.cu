@@ -5,8 +5,10 @@
 // output (offsets bit for bit; the table up to the last-bit behaviour of the FP64 cos/exp).
 #include "tcv_internal.cuh"
 
-#include <cmath>
+#include <atomic>
 #include <climits>
+#include <cmath>
+#include <thread>
 #include <vector>
 
 namespace tcv {
@@ -43,7 +45,7 @@ struct CParams {
 
 // Benchmark.cc:236-258 in FP64, stored as float (imaginary part 0).  One thread per entry of the
 // planes w >= 0: plane -w has the same |w|, so the same values, and the thread stores them there
-// too (half the double-precision cosines, which bound this kernel: 378 -> 204 us at 33 planes of
+// too (half the double-precision cosines, which bound this kernel: 378 -> 243 us at 33 planes of
 // 64 x 129^2 entries).
 __global__ void init_c_kernel(CParams p, float2* c)
 {
@@ -95,7 +97,7 @@ __device__ __forceinline__ float cabs_ref(float2 z)
 //   sum_walk_kernel     one CTA walks the blocks, 1024 composed at a time; a block in which the
 //                       binade ends, or whose two binades do not hold s, is walked entry by entry
 // Both block kernels read the table once (281 MB at the default size: bandwidth); the walk is a
-// chain of ~25 binades of a few microseconds.  117.6 -> 0.25 ms at the default size.
+// chain of a dozen binades of a few microseconds.  117.6 -> 0.38 ms at the default size.
 // ------------------------------------------------------------------------------------------
 constexpr int kSumChunk = 4096;       // entries a CTA of the block kernels handles per round
 constexpr int kSumMaxBlocks = 4096;
@@ -294,8 +296,22 @@ __device__ void walk_entries(WalkShared& sh, const float2* __restrict__ c, int64
 __global__ void __launch_bounds__(kWalkThreads) sum_walk_kernel(const float2* __restrict__ c, SumBlocks b, float* out)
 {
     __shared__ WalkShared sh;
-    if (threadIdx.x == 0) sh.s = 0.f;
-    walk_entries(sh, c, 0, min(b.n, b.per));  // the first binades are short
+    // the first binades are short, and a round of all threads per binade (3.5 us each, a dozen in the
+    // first 4096 entries) costs more than one thread's 4096 additions (9 us)
+    __shared__ __align__(16) float head[kSumChunk];
+    const int64_t nh = min(b.n, int64_t(kSumChunk));
+    for (int i = threadIdx.x; i < kSumChunk; i += kWalkThreads) head[i] = i < nh ? cabs_ref(c[i]) : 0.f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < kSumChunk / 4; ++i) {  // (the places past the table add 0)
+            const float4 v = reinterpret_cast<const float4*>(head)[i];
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+        }
+        sh.s = s;
+    }
+    walk_entries(sh, c, nh, min(b.n, b.per));
     int k = 1;
     while (k < b.nb) {
         const float s = sh.s;
@@ -373,7 +389,36 @@ __global__ void offsets_kernel(OffParams p, const double* u, const double* v, co
 }
 
 // ---- table storage conversions ----
-__global__ void absmax_kernel(const float2* c, int64_t n, unsigned int* absmax_bits)
+// What a conversion reads back: a slot of a fixed device array per call in flight (taken and given
+// back on the host, so calls of several threads do not meet).  Allocating 16 bytes for it instead
+// took 0.6-1.4 ms a call, most of a small table's set-up.
+struct ConvCount {
+    unsigned long long imag_nonzero;
+    unsigned int absmax_bits, pad;
+};
+constexpr int kConvSlots = 64;
+__device__ ConvCount g_conv[kConvSlots];
+std::atomic<uint64_t> g_conv_taken{0};
+
+int take_conv_slot()  // waits while all are in use (each is given back when its call returns)
+{
+    for (;;) {
+        uint64_t m = g_conv_taken.load();
+        while (~m) {
+            const int i = __builtin_ctzll(~m);
+            if (g_conv_taken.compare_exchange_weak(m, m | uint64_t(1) << i)) return i;
+        }
+        std::this_thread::yield();
+    }
+}
+struct ConvSlot {
+    const int i = take_conv_slot();
+    ~ConvSlot() { g_conv_taken.fetch_and(~(uint64_t(1) << i)); }
+};
+
+__global__ void conv_clear_kernel(int slot) { g_conv[slot] = ConvCount{0ull, 0u, 0u}; }
+
+__global__ void absmax_kernel(const float2* c, int64_t n, int slot)
 {
     float m = 0.f;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -381,14 +426,13 @@ __global__ void absmax_kernel(const float2* c, int64_t n, unsigned int* absmax_b
         m = fmaxf(m, fmaxf(fabsf(z.x), fabsf(z.y)));
     }
     for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
+    if ((threadIdx.x & 31) == 0) atomicMax(&g_conv[slot].absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
 }
 
 // One entry per thread and step; counts the entries with an imaginary part as it goes (for the
 // forms without a scale this is the only pass over the table: 35 M entries to r32 in 175 us with a
-// counting pass before it, 85 us in one).
-__global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre_scale, void* out,
-                               unsigned long long* imag_nonzero)
+// counting pass before it, 107 us in one).
+__global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre_scale, void* out, int slot)
 {
     unsigned long long nz = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -411,7 +455,7 @@ __global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre
         }
     }
     for (int o = 16; o; o >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, o);
-    if ((threadIdx.x & 31) == 0 && nz) atomicAdd(imag_nonzero, nz);
+    if ((threadIdx.x & 31) == 0 && nz) atomicAdd(&g_conv[slot].imag_nonzero, nz);
 }
 
 inline int grid_blocks(int64_t n, int threads)
@@ -519,22 +563,24 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
     if (!d_out) return TCV_ERR_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const float2* c = reinterpret_cast<const float2*>(d_c64);
-    // set-up path: a 16-byte device scratch for the max-abs and imaginary-part counters
-    void* scratch = nullptr;
-    TCV_CUDA(cudaMalloc(&scratch, 16));
-    unsigned int* d_max = static_cast<unsigned int*>(scratch);
-    unsigned long long* d_nz = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 8);
-    cudaError_t e = cudaMemsetAsync(scratch, 0, 16, s);
+    const ConvSlot slot;
+    conv_clear_kernel<<<1, 1, 0, s>>>(slot.i);
+    cudaError_t e = cudaGetLastError();
+    auto read_back = [&](ConvCount& h) {
+        if (e == cudaSuccess)
+            e = cudaMemcpyFromSymbolAsync(&h, g_conv, sizeof(h), size_t(slot.i) * sizeof(h), cudaMemcpyDeviceToHost, s);
+        const cudaError_t w = cudaStreamSynchronize(s);  // also after an error: nothing uses the slot from here on
+        if (e == cudaSuccess) e = w;
+    };
+    ConvCount h{};
     float pre = 1.0f, post = 1.0f;
     if (e == cudaSuccess && (c_type == TCV_C_CF16 || c_type == TCV_C_RF16)) {
         // power-of-two scale putting max |C| in [2^14, 2^15): the table keeps FP16's full
         // precision without approaching its 65504 limit; kernels undo it exactly with c_scale.
-        unsigned int hmax = 0;
-        absmax_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, d_max);
+        absmax_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, slot.i);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&hmax, d_max, 4, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        const float amax = __builtin_bit_cast(float, hmax);
+        read_back(h);
+        const float amax = __builtin_bit_cast(float, h.absmax_bits);
         int ex = 0;
         if (amax > 0.f) {
             std::frexp(amax, &ex);  // amax = m * 2^ex, m in [0.5, 1)
@@ -543,17 +589,14 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
             post = std::ldexp(1.0f, -shift);
         }
     }
-    unsigned long long hnz = 0;
     if (e == cudaSuccess) {
-        convert_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, c_type, pre, d_out, d_nz);
+        convert_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, c_type, pre, d_out, slot.i);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hnz, d_nz, 8, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(scratch);
+    read_back(h);
     TCV_CUDA(e);
     if (c_scale_out) *c_scale_out = post;
-    if (imag_nonzero_out) *imag_nonzero_out = int64_t(hnz);
+    if (imag_nonzero_out) *imag_nonzero_out = int64_t(h.imag_nonzero);
     return TCV_OK;
 }
 
