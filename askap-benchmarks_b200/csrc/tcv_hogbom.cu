@@ -45,7 +45,7 @@
 //
 // Measured on one B200, us an iteration, and in brackets with one pass over the image per iteration
 // (in one cooperative launch up to 48 MiB of images, all CTAs waiting on one counter; a launch
-// each beyond): 223^2 1.8 (8.0), 1024^2 3.4 (4.64), 1884^2 6.8 (8.2), 4096^2 16.5 (27.0).
+// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1884^2 6.8 (8.2), 4096^2 16.5 (27.0).
 #include "tcv_internal.cuh"
 
 #include <cooperative_groups.h>
@@ -438,7 +438,7 @@ __device__ __forceinline__ bool wait_phase(const unsigned long long* bar, unsign
 // rows whose PSF values are loaded into registers: 32 values a thread at most, beside up to 64 pixels
 __host__ __device__ constexpr int res_direct(int rows, int chunks) { return rows * chunks <= 32 ? rows : 32 / chunks; }
 
-template <int kRowsT, int kChunks>
+template <int kRowsT, int kChunks, bool kOne>
 __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a, int niters, unsigned long long wait_ns,
                                                                       unsigned int withheld)
 {
@@ -495,8 +495,8 @@ __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a,
         const int ya = max(starty, diffy), yb = min(stopy, diffy + P - 1);
         const float t = __fmul_rn(a.h.gain, peak);
         if (tid == 0) {
-            if (rank == 0) expect_bytes(&bar_got[par], ctas * 8);
-            expect_bytes(&bar_win[par], 8);
+            if (kOne || rank == 0) expect_bytes(&bar_got[par], (ctas + (kOne ? int(withheld) : 0)) * 8);
+            if (!kOne) expect_bytes(&bar_win[par], 8);
         }
         if (models) {  // model[absPeakPos] += absPeakVal * g_gain (HogbomGolden.cc:93)
             if (m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
@@ -510,45 +510,64 @@ __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a,
             skipped += (unsigned long long)(stopy - starty + 1 - max(0, yb - ya + 1));
         }
         const float* __restrict__ p0 = a.h.psf + (ptrdiff_t(y0 - diffy) * P + (tid - diffx));
-        bool cols[kChunks];
+        // per chunk, what the update covers of the thread's column: all its rows (2; the common case,
+        // without a test per pixel), some (1) or none (0).  Rows past the image count as covered: they
+        // hold NaN.  A test per row and pixel cost 32 rows 1 us.
+        const int lasty = min(ry + (P - py - 1), diffy + P - 1);
+        const int rows = y0 >= ya && y0 + kRowsT - 1 <= lasty ? 2 : ya < ye && yb >= y0 ? 1 : 0;
+        int state[kChunks];
 #pragma unroll
-        for (int j = 0; j < kChunks; ++j) cols[j] = tid + j * kResThreads >= startx && tid + j * kResThreads <= stopx;
-        const int ia = ya - y0, ib = min(yb, ye - 1) - y0;  // this CTA's rows that are updated
+        for (int j = 0; j < kChunks; ++j) {
+            const int x = tid + j * kResThreads;
+            state[j] = x >= startx && x <= stopx ? rows : 0;
+        }
+        auto on = [&](int i) { return y0 + i >= ya && y0 + i <= yb; };
         // the whole iteration's PSF values in flight at once: the later rows' by asynchronous copies to
         // this thread's own places in shared memory, the first rows' in registers
         // (2048^2: 7.6 us an iteration with half of them loaded after the other half, 6.35 so)
-#pragma unroll
-        for (int i = kDirect; i < kRowsT; ++i)
-            if (i >= ia && i <= ib) {
-                const float* __restrict__ q = p0 + ptrdiff_t(i) * P;
-#pragma unroll
-                for (int j = 0; j < kChunks; ++j)
-                    if (cols[j])
-                        __pipeline_memcpy_async(later + ((i - kDirect) * kChunks + j) * kResThreads + tid, q + j * kResThreads, 4);
-            }
-        if (kDirect < kRowsT) __pipeline_commit();
         float pv[kDirect][kChunks], top = -1.f;  // only the largest |value| is kept here
 #pragma unroll
-        for (int i = 0; i < kDirect; ++i)
-            if (i >= ia && i <= ib) {
-                const float* __restrict__ q = p0 + ptrdiff_t(i) * P;
+        for (int j = 0; j < kChunks; ++j) {
+            const float* __restrict__ q = p0 + j * kResThreads;
+            if (state[j] == 2) {
 #pragma unroll
-                for (int j = 0; j < kChunks; ++j)
-                    if (cols[j]) pv[i][j] = __ldg(q + j * kResThreads);
+                for (int i = kDirect; i < kRowsT; ++i)
+                    __pipeline_memcpy_async(later + ((i - kDirect) * kChunks + j) * kResThreads + tid, q + ptrdiff_t(i) * P, 4);
+#pragma unroll
+                for (int i = 0; i < kDirect; ++i) pv[i][j] = __ldg(q + ptrdiff_t(i) * P);
+            } else if (state[j] == 1) {
+#pragma unroll
+                for (int i = kDirect; i < kRowsT; ++i)
+                    if (on(i))
+                        __pipeline_memcpy_async(later + ((i - kDirect) * kChunks + j) * kResThreads + tid, q + ptrdiff_t(i) * P, 4);
+#pragma unroll
+                for (int i = 0; i < kDirect; ++i)
+                    if (on(i)) pv[i][j] = __ldg(q + ptrdiff_t(i) * P);
             }
+        }
+        if (kDirect < kRowsT) __pipeline_commit();
+        auto value = [&](int i, int j) {
+            return i < kDirect ? pv[i < kDirect ? i : 0][j] : later[((i < kDirect ? 0 : i - kDirect) * kChunks + j) * kResThreads + tid];
+        };
 #pragma unroll
-        for (int i = 0; i < kRowsT; ++i) {
-            if (i == kDirect) __pipeline_wait_prior(0);
-            if (i >= ia && i <= ib) {
+        for (int i0 = 0; i0 < kRowsT; i0 += kDirect) {
+            if (i0) __pipeline_wait_prior(0);
 #pragma unroll
-                for (int j = 0; j < kChunks; ++j)
-                    if (cols[j])
-                        r[i][j] = __fsub_rn(r[i][j], __fmul_rn(t, i < kDirect ? pv[i < kDirect ? i : 0][j]
-                                                                              : later[((i - kDirect) * kChunks + j) * kResThreads + tid]));
+            for (int j = 0; j < kChunks; ++j) {
+                if (state[j] == 2) {
+#pragma unroll
+                    for (int i = i0; i < i0 + kDirect && i < kRowsT; ++i) r[i][j] = __fsub_rn(r[i][j], __fmul_rn(t, value(i, j)));
+                } else if (state[j] == 1) {
+#pragma unroll
+                    for (int i = i0; i < i0 + kDirect && i < kRowsT; ++i)
+                        if (on(i)) r[i][j] = __fsub_rn(r[i][j], __fmul_rn(t, value(i, j)));
+                }
             }
+        }
+#pragma unroll
+        for (int i = 0; i < kRowsT; ++i)
 #pragma unroll
             for (int j = 0; j < kChunks; ++j) top = fmaxf(top, fabsf(r[i][j]));  // (places past the image hold NaN)
-        }
         // the CTA's largest |value|, then its first place (only threads that hold that value look)
         const unsigned mine = top < 0.f ? 0u : __float_as_uint(top) + 1u;
         const unsigned most = __reduce_max_sync(0xffffffffu, mine);
@@ -557,20 +576,22 @@ __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a,
         __syncthreads();
         const unsigned all = __reduce_max_sync(0xffffffffu, lane < kResThreads / 32 ? wk[lane] : 0u);
         if (mine == all && all) {
-            bool found = false;
+            int at = 0;
+            float tv = 0.f;
 #pragma unroll
-            for (int i = 0; i < kRowsT; ++i)
-#pragma unroll
-                for (int j = 0; j < kChunks; ++j)
-                    if (!found && fabsf(r[i][j]) == top) {  // rows, then columns in order: the thread's first
-                        found = true;
-                        atomicMax(&key, cand_key(r[i][j], tid + j * kResThreads, y0 + i));
-                    }
+            for (int e = kRowsT * kChunks - 1; e >= 0; --e)  // rows, then columns in order: the thread's first
+                if (fabsf(r[e / kChunks][e % kChunks]) == top) {
+                    at = e;
+                    tv = r[e / kChunks][e % kChunks];
+                }
+            atomicMax(&key, cand_key(tv, tid + at % kChunks * kResThreads, y0 + at / kChunks));
         }
         __syncthreads();
         unsigned long long c;
         bool ok = true;
-        if (warp == 0) {
+        if (kOne) {  // one cluster: every CTA sends its candidate to every other
+            if (warp == 0 && lane < ctas) send_key(&got[par][rank], &bar_got[par], lane, key);
+        } else if (warp == 0) {
             c = key;
             if (lane == 0) send_key(&got[par][rank], &bar_got[par], 0, c);
             if (rank == 0) {
@@ -609,12 +630,12 @@ __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a,
                 if (ok && lane < ctas) send_key(&win[par], &bar_win[par], lane, c);
             }
         }
-        if (ok) ok = wait_phase(&bar_win[par], phase, wait_ns);
+        if (ok) ok = wait_phase(kOne ? &bar_got[par] : &bar_win[par], phase, wait_ns);
         if (!__syncthreads_and(ok)) {
             st->error = 1;
             break;
         }
-        c = win[par];
+        c = kOne ? warp_max(lane < ctas ? got[par][lane] : 0ull) : win[par];
         const bool zero = (c >> 33) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
         const unsigned int idx = zero ? 0u : cand_index(c);
         rx = int(idx & 0xffffu);
@@ -1232,10 +1253,10 @@ template <int kRowsT>
 ResKernel resident_of(int chunks)
 {
     switch (chunks) {
-        case 1: return hog_resident_kernel<kRowsT, 1>;
-        case 2: return hog_resident_kernel<kRowsT, 2>;
-        case 3: return hog_resident_kernel<kRowsT, 3>;
-        default: return hog_resident_kernel<kRowsT, 4>;
+        case 1: return hog_resident_kernel<kRowsT, 1, false>;
+        case 2: return hog_resident_kernel<kRowsT, 2, false>;
+        case 3: return hog_resident_kernel<kRowsT, 3, false>;
+        default: return hog_resident_kernel<kRowsT, 4, false>;
     }
 }
 
@@ -1260,8 +1281,18 @@ tcv_status deconvolve_resident(const HogArgs& h, const HogWork& w, const float* 
     cfg.blockDim = dim3(kResThreads);
     cfg.attrs = attr;
     cfg.stream = st;
-    for (int rows_t : {4, 8, 16}) {
-        const ResKernel kernel = rows_t == 4 ? resident_of<4>(chunks) : rows_t == 8 ? resident_of<8>(chunks) : resident_of<16>(chunks);
+    // up to 256 wide in one cluster, which meets in its shared memory alone (128^2: 1.23 us an
+    // iteration, 1.75 in clusters that meet through L2; 256^2 1.62 and 1.8; 300^2, with 32 rows a
+    // CTA, 2.5 and 1.75)
+    for (int rows_t : {-8, -16, 4, 8, 16}) {  // negative: one cluster
+        const bool one = rows_t < 0;
+        rows_t = std::abs(rows_t);
+        if (one && (W + 15) / 16 > rows_t) continue;
+        const ResKernel kernel = one ? (rows_t == 8 ? ResKernel(hog_resident_kernel<8, 1, true>)
+                                                    : ResKernel(hog_resident_kernel<16, 1, true>))
+                                 : rows_t == 4 ? resident_of<4>(chunks)
+                                 : rows_t == 8 ? resident_of<8>(chunks)
+                                               : resident_of<16>(chunks);
         // clusters of 16 where they fit: half as many meet as of 8 (300^2: 1.80 us an iteration, not 1.91)
         int size = 16, most = 0;
         cfg.dynamicSmemBytes = size_t(rows_t - res_direct(rows_t, chunks)) * chunks * kResThreads * sizeof(float);
@@ -1277,7 +1308,7 @@ tcv_status deconvolve_resident(const HogArgs& h, const HogWork& w, const float* 
             cudaGetLastError();
             most = 0;
         }
-        most = std::min(most, kResClusters);
+        most = std::min(most, one ? 1 : kResClusters);
         // rows per CTA: at least four, so that small images meet in few clusters
         const int rows = std::max(4, (W + most * size - 1) / std::max(1, most * size));
         if (most < 1 || rows > rows_t) continue;
