@@ -46,6 +46,154 @@ GridArgs make_args(const tcv_plan* p, int grp, float c_scale, float2* grid)
     return a;
 }
 
+// Gridding of a plan with few busy tiles.  A CTA of grid_tile_kernel walks its unit's samples one after
+// another, and with one CTA on an SM each sample costs a warp a full L2 latency (16 k samples of a
+// 45^2 footprint on 25 tiles, cells whole: 0.71 ms, 1.3 k cycles a sample and warp).  Here a tile is
+// shared out in slices of 8 rows to as many CTAs, a warp's block is 32 columns x 2 rows, and the
+// table rows of six samples are loaded before the first is added.  Every point still has one owner
+// that adds its samples in order, group after group, so the sums are the same, bit for bit; per
+// update it costs more instructions, which a device that is mostly idle has to spare.
+// Whole-cell plans take it when every plane group has at most 1.2 busy tiles per SM (plan_mode_kernel):
+// 169 tiles gain (0.72 -> 0.49 ms), 289 do not (0.38 and 0.51 ms).  The samples above take 0.162 ms,
+// 160 k samples of 29^2 on 9 tiles 4.3 ms (18.8 whole).  Six samples at four CTAs an SM: eight at three
+// take 0.165 and 4.1 ms but 0.55 ms on 169 tiles, four at four 0.19, 4.7 and 0.52.
+// A kernel of its own: inside grid_tile_kernel it cost the other path 1.4 % (registers).  It is launched
+// behind the tile kernels, whose ranges are then empty, without the usual gap (it waits for them
+// itself): where it is not taken that costs 0.3 us a pass, an ordinary launch before them 4 us.
+template <class Tab, int kR, bool kVar>
+__global__ void __launch_bounds__(kTileThreads, 4)
+grid_slice_kernel(const float2* __restrict__ data, const typename Tab::elem* __restrict__ ctab,
+                  const int* __restrict__ iu, const int* __restrict__ iv, const int* __restrict__ coff,
+                  const u32* __restrict__ order, const u32* __restrict__ tile_start, const u32* __restrict__ tile_count,
+                  const unsigned int* __restrict__ taken, int n_groups, GridArgs a)
+{
+    constexpr int kTH = tile_height(kR), kRows = 2, kDeep = 6;
+    constexpr u32 kSlices = kTH / (4 * kRows);  // a slice: four pairs of warps
+    constexpr u32 kLook = 4 * kTileThreads;     // tiles looked over at a time
+    cudaGridDependencySynchronize();  // launched ahead of the tile kernels' end
+    if (!*taken) return;
+    __shared__ float4 sm_rec[2][kTileChunk];  // (data.re, data.im, first column, first row)
+    __shared__ int sm_coff[2][kTileChunk];
+    __shared__ int sm_w[kVar ? 2 : 1][kVar ? kTileChunk : 1];
+    __shared__ unsigned char sm_mask[2][kTileChunk];  // per sample: the warps whose blocks it meets
+    __shared__ u32 busy[kLook], sm_n[4 * kTileWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s0 = a.s;
+    u32 before = 0;  // busy tiles of the looks before
+    for (u32 look = 0; look < u32(a.ntiles); look += kLook) {
+        // the busy tiles, in order (every CTA finds the same list)
+        bool on[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const u32 t = look + u32(e) * kTileThreads + threadIdx.x;
+            on[e] = false;
+            if (t < u32(a.ntiles))
+                for (int g = 0; g < n_groups; ++g) on[e] |= tile_count[u32(g) * u32(a.ntiles) + t] != 0u;
+        }
+        __syncthreads();  // the last look's list is used
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const u32 b = __ballot_sync(0xffffffffu, on[e]);
+            if (lane == 0) sm_n[e * kTileWarps + warp] = __popc(b);
+        }
+        __syncthreads();
+        const u32 mine = sm_n[lane];  // lane e * kTileWarps + w: 32 counts
+        static_assert(4 * kTileWarps == 32, "one count per lane");
+        const u32 n = __reduce_add_sync(0xffffffffu, mine);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const u32 b = __ballot_sync(0xffffffffu, on[e]);
+            const u32 at = __reduce_add_sync(0xffffffffu, lane < e * kTileWarps + warp ? mine : 0u) + __popc(b & ((1u << lane) - 1u));
+            if (on[e]) busy[at] = look + u32(e) * kTileThreads + threadIdx.x;
+        }
+        __syncthreads();
+        // items (busy tile, slice), numbered over all looks, dealt to the CTAs in turn
+        const u32 first = before * kSlices, rest = first % gridDim.x;
+        for (u32 item = rest <= blockIdx.x ? blockIdx.x - rest : gridDim.x - rest + blockIdx.x; item < n * kSlices;
+             item += gridDim.x) {
+            const u32 tile = busy[item / kSlices], ti = a.tinfo[tile];
+            const int x0 = rec_tx(ti) * kTileW, y0 = rec_ty(ti) * kTH + int(item % kSlices) * (4 * kRows);
+            const int gx = x0 + (warp & 1) * 32 + lane, gy0 = y0 + (warp >> 1) * kRows;
+            const JobDesc& jd = a.jobs[rec_job(ti)];
+            const int gs = jd.g_size;
+            float2* grid = a.grid ? a.grid : jd.grid;
+            for (int g = 0; g < n_groups; ++g) {
+                const u32 c = u32(g) * u32(a.ntiles) + tile, start = tile_start[c], cnt = tile_count[c];
+                if (cnt == 0) continue;  // the same for the whole CTA
+                float2 acc[kRows];
+#pragma unroll
+                for (int r = 0; r < kRows; ++r) acc[r] = make_float2(0.f, 0.f);
+                auto stage = [&](u32 base, int buf) {
+                    if (base + threadIdx.x >= cnt) return;
+                    const u32 k = order[start + base + threadIdx.x];
+                    const float2 d = data[k];
+                    const int sk = kVar ? int(a.ssz[k]) : s0;
+                    const int fx = iu[k] - (kVar ? sk / 2 : a.support), fy = iv[k];
+                    sm_rec[buf][threadIdx.x] =
+                        make_float4(d.x * a.c_scale, d.y * a.c_scale, __int_as_float(fx), __int_as_float(fy));
+                    sm_coff[buf][threadIdx.x] = coff[k];
+                    if (kVar) sm_w[kVar ? buf : 0][kVar ? threadIdx.x : 0] = sk;
+                    const int bx = x0 - fx, by = y0 - fy;
+                    u32 m = 0;
+#pragma unroll
+                    for (int w = 0; w < kTileWarps; ++w) {
+                        const int cx = bx + (w & 1) * 32, cy = by + (w >> 1) * kRows;
+                        m |= u32(cx < sk && cx + 32 > 0 && cy < sk && cy + kRows > 0) << w;
+                    }
+                    sm_mask[buf][threadIdx.x] = (unsigned char)m;
+                };
+                __syncthreads();  // the records before are used
+                stage(0, 0);
+                int buf = 0;
+                for (u32 base = 0; base < cnt; base += u32(kTileChunk), buf ^= 1) {
+                    __syncthreads();  // this chunk is staged, the one before is used
+                    stage(base + u32(kTileChunk), buf ^ 1);
+                    const int m = int(cnt - base < u32(kTileChunk) ? cnt - base : u32(kTileChunk));
+                    for (int e = 0; e < m; e += 32) {
+                        u32 bits = __ballot_sync(0xffffffffu, e + lane < m && ((sm_mask[buf][e + lane] >> warp) & 1u));
+                        while (bits) {
+                            float2 cv[kDeep][kRows], dv[kDeep];
+                            u32 has = 0;  // rows that this lane's column of the footprint has, kRows bits per sample
+#pragma unroll
+                            for (int b = 0; b < kDeep; ++b) {
+                                if (!bits) break;
+                                const int j = e + __ffs(bits) - 1;
+                                bits &= bits - 1;
+                                const float4 q = sm_rec[buf][j];
+                                const int s = kVar ? sm_w[kVar ? buf : 0][kVar ? j : 0] : s0;
+                                const int dx = gx - __float_as_int(q.z), dy = gy0 - __float_as_int(q.w);
+                                const int ci = sm_coff[buf][j] + dy * s + dx;
+                                dv[b] = make_float2(q.x, q.y);
+#pragma unroll
+                                for (int r = 0; r < kRows; ++r)
+                                    if (unsigned(dx) < unsigned(s) && unsigned(dy + r) < unsigned(s)) {
+                                        has |= 1u << (b * kRows + r);
+                                        cv[b][r] = Tab::load(ctab + (ci + r * s));
+                                    }
+                            }
+#pragma unroll
+                            for (int b = 0; b < kDeep; ++b)
+#pragma unroll
+                                for (int r = 0; r < kRows; ++r)
+                                    if ((has >> (b * kRows + r)) & 1u) cmac<Tab::kReal>(acc[r], dv[b], cv[b][r]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < kRows; ++r)
+                    if (gx < gs && gy0 + r < gs) {
+                        float2* gp = grid + ((unsigned long long)(gy0 + r) * gs + gx);
+                        float2 v = *gp;
+                        v.x += acc[r].x;
+                        v.y += acc[r].y;
+                        *gp = v;
+                    }
+            }
+        }
+        before += n;
+    }
+}
+
 // One persistent launch per plane group, in group order on the stream: launches of one stream
 // run one after another, so a tile's read-modify-write never races with another group's.
 template <class Tab, int kR, bool kVar = false>
@@ -64,9 +212,9 @@ tcv_status launch(const tcv_plan* p, const float2* data, const void* c, float c_
     const unsigned int* order = p->vals[p->sel];
     for (int grp = 0; grp < g.n_groups; ++grp) {
         GridArgs a = make_args(p, grp, c_scale, grid);
+        const uint32_t* range = p->grid_range ? p->grid_range + grp : p->group_ustart;  // [grp], [grp + 1]: first, end unit
         void* args[] = {&data, &tab, const_cast<const int32_t**>(&p->iu), const_cast<const int32_t**>(&p->iv),
-                        const_cast<const int32_t**>(&p->coff), &order, const_cast<uint4**>(&p->units),
-                        const_cast<uint32_t**>(&p->group_ustart), &a};
+                        const_cast<const int32_t**>(&p->coff), &order, const_cast<uint4**>(&p->units), &range, &a};
         TCV_CUDA(cudaLaunchKernel(kernel, dim3(ctas), dim3(kTileThreads), args, 0, st));
         if (g.split) {
             // the split cells' partial tiles into the grid, before the next group touches it
@@ -74,6 +222,23 @@ tcv_status launch(const tcv_plan* p, const float2* data, const void* c, float c_
                                                                   p->pstart, a);
             TCV_CUDA(cudaGetLastError());
         }
+    }
+    if (p->grid_range) {  // plans of few busy tiles: the launches above found no units
+        const void* slices = reinterpret_cast<const void*>(&grid_slice_kernel<Tab, kR, kVar>);
+        const GridArgs a = make_args(p, 0, c_scale, grid);
+        cudaLaunchAttribute early{};
+        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        early.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(unsigned(resident_of(slices)));
+        cfg.blockDim = dim3(kTileThreads);
+        cfg.stream = st;
+        cfg.attrs = &early;
+        cfg.numAttrs = 1;
+        TCV_CUDA(cudaLaunchKernelEx(&cfg, &grid_slice_kernel<Tab, kR, kVar>, data, tab, static_cast<const int*>(p->iu),
+                                    static_cast<const int*>(p->iv), static_cast<const int*>(p->coff), order,
+                                    static_cast<const u32*>(p->tile_start), static_cast<const u32*>(p->tile_count),
+                                    static_cast<const unsigned int*>(p->status + kSliceWord), int(g.n_groups), a));
     }
     return TCV_OK;
 }

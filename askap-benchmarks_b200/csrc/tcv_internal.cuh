@@ -88,6 +88,9 @@ struct tcv_plan {
     uint32_t* n_items;             // [0] = number of non-empty gridding cells
     uint32_t* group_start;         // n_groups + 1: items of group g are [group_start[g], group_start[g+1])
     uint32_t* group_ustart;        // n_groups + 1: work units of group g
+    uint32_t* grid_range;          // 2 n_groups: group g's first and end unit for the gridding tile
+                                   // kernels (empty when the plan is gridded in slices); NULL for
+                                   // plans of split cells or of more than kSliceGroups groups
     uint32_t* nunits;              // per item: work units of its cell
     uint32_t* ustart;              // per item: its first unit
     uint32_t* pstart;              // per item: its first partial tile (split cells)
@@ -145,6 +148,9 @@ namespace tcv {
 
 constexpr int kStatusWords = 8;  // the plan's status block, zeroed by every binning
 constexpr int kSchedWord = 4;    // first of the two work-item counters in it
+constexpr int kSliceWord = 6;    // 1: the plan is gridded in slices of its tiles (grid_slice_kernel)
+constexpr int kSliceGroups = 20;  // plans of more groups are not; their ranges would not fit the 256 bytes
+                                  // that group_ustart has in the workspace anyhow
 
 // Host helpers implemented in tcv_plan.cu
 // Geometry for jobs of the given grid sides (n samples in all); tuning may be nullptr.  anchors:

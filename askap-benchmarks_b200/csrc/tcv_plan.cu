@@ -592,6 +592,22 @@ tcv_status plan_anchors_ready(const tcv_plan* cp, cudaStream_t st)
     return s;
 }
 
+// Whether every plane group has at most `few` units: the plan is then gridded in slices of its tiles,
+// and the tile kernels' ranges are empty.
+__global__ void plan_mode_kernel(const uint32_t* __restrict__ group_ustart, int n_groups, uint32_t few, uint32_t* range,
+                                 unsigned int* sliced)
+{
+    static_assert(kSliceGroups <= 32, "a group per lane");
+    const int g = threadIdx.x;
+    const uint32_t from = g < n_groups ? group_ustart[g] : 0u, to = g < n_groups ? group_ustart[g + 1] : 0u;
+    const bool all_few = __all_sync(0xffffffffu, to - from <= few);
+    if (g < n_groups) {
+        range[2 * g] = all_few ? 0u : from;
+        range[2 * g + 1] = all_few ? 0u : to;
+    }
+    if (threadIdx.x == 0) *sliced = all_few;
+}
+
 // The cells' bookkeeping from their ranges (tile_start: starts, tile_count: ends).
 tcv_status cells_and_units(tcv_plan* p, cudaStream_t st)
 {
@@ -608,6 +624,12 @@ tcv_status cells_and_units(tcv_plan* p, cudaStream_t st)
     cell_scan_kernel<<<1, 1024, 0, st>>>(ca, cb);
     TCV_CUDA(cudaGetLastError());
     cell_out_kernel<<<cb, kCellThreads, 0, st>>>(ca);
+    TCV_CUDA(cudaGetLastError());
+    if (!p->grid_range) return TCV_OK;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    plan_mode_kernel<<<1, 32, 0, st>>>(p->group_ustart, g.n_groups, uint32_t(sms) * 6u / 5u, p->grid_range,
+                                       p->status + kSliceWord);
     TCV_CUDA(cudaGetLastError());
     return TCV_OK;
 }
@@ -746,6 +768,7 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
     p->n_items = static_cast<uint32_t*>(take(4));
     p->group_start = static_cast<uint32_t*>(take(size_t(g.n_groups + 1) * 4));
     p->group_ustart = static_cast<uint32_t*>(take(size_t(g.n_groups + 1) * 4));
+    p->grid_range = !g.split && g.n_groups <= kSliceGroups ? p->group_ustart + g.n_groups + 1 : nullptr;
     p->nunits = static_cast<uint32_t*>(take(cells * 4));
     p->ustart = static_cast<uint32_t*>(take(cells * 4));
     p->pstart = static_cast<uint32_t*>(take(cells * 4));
@@ -895,33 +918,24 @@ PlanGeom make_geom(int64_t n, int support, const int* g_sizes, int n_jobs, int64
     return g;
 }
 
-// Work units of a plan without a tuning.  Where the samples lie is not known on the host, and
-// samples that crowd into a few tiles leave most SMs idle with cells whole (16 k samples of a 45^2
-// footprint meet ~25 tiles of 64 x 64: gridding 0.71 ms whole, 0.074-0.080 ms in units of 32-64
-// samples; 60 k samples of 29^2 within 150^2 points: 7.2 and 0.12 ms), while samples spread over
-// many tiles are not split by a rule that aims at the device: about four units per SM slot of four
-// CTAs (2368), in whole powers of two.  Below 32 samples a unit's tile write costs more than its
-// work; above 512 no measured problem gained.  Degridding units need no partial tile, so they are
-// half as large (37 k samples of 65^2: 0.147 ms with 64, 0.140 ms with 32, 0.82 ms whole).
-// The partial tiles never push a plan past kUnitsBytes that would fit without them: that is the
-// scratch of the allocation-free entry, which takes every problem it took with cells whole.
+// Degridding units of a plan without a tuning.  Where the samples lie is not known on the host, and
+// samples that crowd into a few tiles leave most SMs idle with cells whole (37 k samples of a 65^2
+// footprint: 0.82 ms whole, 0.147 ms in units of 64 samples, 0.140 of 32), while samples spread over
+// many tiles are not split by a rule that aims at the device: about eight units per SM slot of four
+// CTAs (4736), in whole powers of two.  Below 32 samples a unit's tile read costs more than its work;
+// above 128 no measured problem gained.  A degridding unit writes its own samples' slots, so its
+// size changes no result.  Gridding keeps cells whole, each point's sum in sample order, and shares
+// crowded ones out in slices (tcv_grid.cu).
+// The unit list never pushes a plan past kUnitsBytes that would fit without it: that is the scratch
+// of the allocation-free entry, which takes every problem it took with cells whole.
 void default_units(PlanGeom& g)
 {
     constexpr size_t kUnitsBytes = size_t(64) << 20;
     const double reach = (double(g.s + g.tw - 1) / g.tw) * (double(g.s + g.th - 1) / g.th);
     const double pairs = double(g.n) * reach;  // mean tiles of a footprint
-    auto size = [&](double units, int most) {
-        int u = 32;
-        while (u < most && double(u) * units < pairs) u *= 2;
-        return u;
-    };
     const bool small = plan_bytes(g, nullptr) <= kUnitsBytes;
-    auto fits = [&] { return !small || plan_bytes(g, nullptr) <= kUnitsBytes; };
-    g.dsplit = size(2 * 2368.0, 128);
-    if (!fits()) g.dsplit = 0;
-    for (g.split = size(2368.0, 512); g.split <= 512; g.split *= 2)
-        if (fits()) return;
-    g.split = 0;
+    for (g.dsplit = 32; g.dsplit < 128 && g.dsplit * 4736.0 < pairs;) g.dsplit *= 2;
+    if (small && plan_bytes(g, nullptr) > kUnitsBytes) g.dsplit = 0;
 }
 
 size_t plan_bytes(const PlanGeom& g, size_t* cub_bytes_out)

@@ -1,7 +1,7 @@
 """The work units of a plan built without a tuning.
 
-A plan without a tuning cuts cells that many samples crowd into, so that a few busy tiles still fill
-the device.  Bars: the plan never outgrows the allocation-free entry's scratch where cells whole fit
+A plan without a tuning degrids cells that many samples crowd into in units of some samples, and grids
+a few busy tiles in slices of their rows, so that they still fill the device.  Bars: the plan never outgrows the allocation-free entry's scratch where cells whole fit
 it (host arithmetic); crowded samples grid and degrid within the parity bar of the FP32 path
 (relative L2 1e-5 of the oracle), the same bits on every run.
 """
@@ -69,3 +69,43 @@ def test_crowded_samples_match_oracle(tcv, orc, cuda_ok, n, support, g, spread):
     out64 = orc.degrid_f64(grid64, g, support, table64, coff, iu, iv)
     assert orc.rel_l2(runs[0][0], grid64) <= REL_L2_FP32
     assert orc.rel_l2(runs[0][1], out64) <= REL_L2_FP32
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [8, 16, 32])
+@pytest.mark.parametrize("form", ["c64", "r32", "rbf16"])
+@pytest.mark.parametrize("n,support", [(1, 10), (257, 10), (3000, 3), (1500, 40)])
+def test_whole_cells_in_slices_keep_their_bits(tcv, orc, cuda_ok, rows, form, n, support):
+    """A plan group with few busy tiles is gridded in slices of its tiles; samples of zero data all over
+    the grid make many tiles busy, which grids them whole.  The crowd's points get the same bits."""
+    import torch
+
+    from tconvolve import _lib, raw
+
+    rng = np.random.default_rng(n + support)
+    g, s = 2048, 2 * support + 1
+    c_len = 64 * s * s
+    c64 = torch.from_numpy(rng.standard_normal(c_len).astype(np.float32).astype(np.complex64)).cuda()
+    code = _lib.CTYPE_BY_NAME[form]
+    tab, scale = (c64, 1.0) if form == "c64" else raw.convert_c(c64, code)[:2]
+    iu = (700 + rng.integers(0, 60, n)).astype(np.int32)
+    iv = (900 + rng.integers(0, 60, n)).astype(np.int32)
+    far = np.arange(support, g - s, 32 if support < 30 else 60, dtype=np.int32)
+    fu, fv = (a.ravel().astype(np.int32) for a in np.meshgrid(far, far))
+    coff = (rng.integers(0, 64, n) * s * s).astype(np.int32)
+    vis = (rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    grids = []
+    for crowd in (True, False):
+        u, v, co, x = iu, iv, coff, vis
+        if not crowd:
+            u, v = np.concatenate([iu, fu]), np.concatenate([iv, fv])
+            co = np.concatenate([coff, np.zeros(fu.size, np.int32)])
+            x = np.concatenate([vis, np.zeros(fu.size, np.complex64)])
+        plan = raw.Plan(d(u), d(v), d(co), support, g, c_len, tuning=(rows, -1, 0, 0))
+        grid = torch.zeros(g * g, dtype=torch.complex64, device="cuda")
+        plan.grid(d(x), tab, code, grid, scale)
+        assert plan.rejected() == 0
+        grids.append(grid.cpu().numpy())
+    assert np.count_nonzero(grids[0]) > 0
+    assert np.array_equal(grids[0], grids[1])
