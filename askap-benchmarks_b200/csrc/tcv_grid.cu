@@ -226,19 +226,9 @@ tcv_status launch(const tcv_plan* p, const float2* data, const void* c, float c_
     if (p->grid_range) {  // plans of few busy tiles: the launches above found no units
         const void* slices = reinterpret_cast<const void*>(&grid_slice_kernel<Tab, kR, kVar>);
         const GridArgs a = make_args(p, 0, c_scale, grid);
-        cudaLaunchAttribute early{};
-        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        early.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(unsigned(resident_of(slices)));
-        cfg.blockDim = dim3(kTileThreads);
-        cfg.stream = st;
-        cfg.attrs = &early;
-        cfg.numAttrs = 1;
-        TCV_CUDA(cudaLaunchKernelEx(&cfg, &grid_slice_kernel<Tab, kR, kVar>, data, tab, static_cast<const int*>(p->iu),
-                                    static_cast<const int*>(p->iv), static_cast<const int*>(p->coff), order,
-                                    static_cast<const u32*>(p->tile_start), static_cast<const u32*>(p->tile_count),
-                                    static_cast<const unsigned int*>(p->status + kSliceWord), int(g.n_groups), a));
+        TCV_CHECK(launch_behind(&grid_slice_kernel<Tab, kR, kVar>, unsigned(resident_of(slices)), kTileThreads, st, data, tab,
+                                p->iu, p->iv, p->coff, order, p->tile_start, p->tile_count, p->status + kSliceWord,
+                                g.n_groups, a));
     }
     return TCV_OK;
 }

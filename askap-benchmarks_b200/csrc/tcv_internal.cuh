@@ -269,3 +269,25 @@ inline tcv_status cuda_status(cudaError_t e)
         cudaError_t _e = (call);                               \
         if (_e != cudaSuccess) return ::tcv::cuda_status(_e);  \
     } while (0)
+
+namespace tcv {
+
+// Launch of a kernel that waits for the stream's earlier work itself (cudaGridDependencySynchronize
+// before it reads or writes anything of theirs): its blocks start while the kernel before drains.
+template <typename... P, typename... A>
+inline tcv_status launch_behind(void (*kernel)(P...), unsigned blocks, int threads, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    TCV_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return TCV_OK;
+}
+
+}  // namespace tcv

@@ -11,7 +11,8 @@
 //               use).
 // Each cell's pair range comes from the run bounds of the sorted keys (no per-pair atomics), and
 // the per-cell bookkeeping (tile offsets, the non-empty cells, per-group ranges, the work-unit
-// lists) takes three launches over the cells.
+// lists) takes three launches over the cells.  Few samples are counted into their cells instead of
+// sorted (few_count_kernel), with the same arrays as the result.
 // Kernel indices kid = cOffset / sSize^2 (w-plane major, then the oversampling offsets) are
 // grouped into runs of whole w-planes whose slice of the table fits in L2 with room to spare.
 // The sort key is the work cell (group, tile), ordered group-major, so all SMs work through the
@@ -81,15 +82,20 @@ __device__ __forceinline__ uint32_t anchor_cell(const PlanGeom& g, uint32_t grp,
     return grp * uint32_t(g.natx * g.naty) + (fy / uint32_t(g.ta)) * uint32_t(g.natx) + fx / uint32_t(g.ta);
 }
 
-// The pairs of sample d (its footprint's tiles, then sentinels up to max_tiles) into kp/vp.
-template <typename K>
-__device__ __forceinline__ void sample_keys(const int32_t* __restrict__ iu, const int32_t* __restrict__ iv,
-                                            const int32_t* __restrict__ coff, const PlanGeom& g,
-                                            const JobDesc* __restrict__ jobs, const uint32_t* __restrict__ job_start,
-                                            int64_t d, K* kp, uint32_t* vp, K* akeys, uint32_t* avals,
-                                            uint32_t* atile_count, uint16_t* ntl, unsigned long long* rejected,
-                                            const VarPlanes& var, bool with_anchors)
+// The tiles that sample d's footprint meets: columns tx0 .. tx1, rows ty0 .. ty1 of the tiles of its
+// (plane group, job), whose first cell is cell0 (ntx tiles a row); ok false: the sample is left out.
+struct Reach {
+    bool ok;
+    uint32_t cell0, grp, fx, fy;
+    int ntx, tx0, tx1, ty0, ty1, s;
+};
+
+__device__ __forceinline__ Reach reach_of(const int32_t* __restrict__ iu, const int32_t* __restrict__ iv,
+                                          const int32_t* __restrict__ coff, const PlanGeom& g,
+                                          const JobDesc* __restrict__ jobs, const uint32_t* __restrict__ job_start,
+                                          int64_t d, const VarPlanes& var)
 {
+    Reach r{};
     const int job = g.n_jobs > 1 ? job_of(job_start, g.n_jobs, uint32_t(d)) : 0;
     const JobDesc jd = jobs[job];
     int64_t s = g.s, support = g.support;
@@ -100,15 +106,44 @@ __device__ __forceinline__ void sample_keys(const int32_t* __restrict__ iu, cons
         plane_ok = plane >= 0 && plane < g.n_planes;
         s = plane_ok ? var.plane_s[plane] : 1;
         support = s / 2;
-        var.ssz[d] = uint16_t(s);
     }
+    r.s = int(s);
     const int64_t fx = (int64_t)iu[d] - support;
     const int64_t fy = iv[d];
     const int64_t co = coff[d];
-    const bool ok = plane_ok && fx >= 0 && fx + s <= jd.g_size && fy >= 0 && fy + s <= jd.g_size && co >= 0 &&
-                    co + s * s <= g.c_len;
+    r.ok = plane_ok && fx >= 0 && fx + s <= jd.g_size && fy >= 0 && fy + s <= jd.g_size && co >= 0 &&
+           co + s * s <= g.c_len;
+    if (!r.ok) return r;
+    // in bounds, every operand below fits 32 bits (fx + s <= g_size, s*s <= c_len): 32-bit
+    // divisions (a 64-bit one is a long software sequence, several per sample)
+    const uint32_t us = uint32_t(s), utw = uint32_t(g.tw), uth = uint32_t(g.th);
+    r.fx = uint32_t(fx);
+    r.fy = uint32_t(fy);
+    r.grp = g.var ? uint32_t(var.plane_grp[plane])
+                  : (co <= int64_t(0xffffffffll) ? uint32_t(co) / (us * us) : uint32_t(co / (s * s))) /
+                        uint32_t(g.kid_group);
+    r.cell0 = r.grp * uint32_t(g.ntiles) + jd.tile_base;
+    r.ntx = jd.ntx;
+    r.tx0 = int(r.fx / utw);
+    r.tx1 = int((r.fx + us - 1) / utw);
+    r.ty0 = int(r.fy / uth);
+    r.ty1 = int((r.fy + us - 1) / uth);
+    return r;
+}
+
+// The pairs of sample d (its footprint's tiles, then sentinels up to max_tiles) into kp/vp.
+template <typename K>
+__device__ __forceinline__ void sample_keys(const int32_t* __restrict__ iu, const int32_t* __restrict__ iv,
+                                            const int32_t* __restrict__ coff, const PlanGeom& g,
+                                            const JobDesc* __restrict__ jobs, const uint32_t* __restrict__ job_start,
+                                            int64_t d, K* kp, uint32_t* vp, K* akeys, uint32_t* avals,
+                                            uint32_t* atile_count, uint16_t* ntl, unsigned long long* rejected,
+                                            const VarPlanes& var, bool with_anchors)
+{
+    const Reach f = reach_of(iu, iv, coff, g, jobs, job_start, d, var);
+    if (g.var) var.ssz[d] = uint16_t(f.s);
     const K sentinel = K(1) << (g.key_bits - 1);
-    if (!ok) {
+    if (!f.ok) {
         atomicAdd(rejected, 1ull);
         for (int t = 0; t < g.max_tiles; ++t) {
             kp[t] = sentinel;
@@ -121,20 +156,10 @@ __device__ __forceinline__ void sample_keys(const int32_t* __restrict__ iu, cons
         }
         return;
     }
-    // in bounds, every operand below fits 32 bits (fx + s <= g_size, s*s <= c_len): 32-bit
-    // divisions (a 64-bit one is a long software sequence, several per sample)
-    const uint32_t ufx = uint32_t(fx), ufy = uint32_t(fy), us = uint32_t(s);
-    const uint32_t grp = g.var ? uint32_t(var.plane_grp[plane])
-                               : (co <= int64_t(0xffffffffll) ? uint32_t(co) / (us * us) : uint32_t(co / (s * s))) /
-                                     uint32_t(g.kid_group);
-    const uint32_t cell0 = grp * uint32_t(g.ntiles) + jd.tile_base;
-    const uint32_t utw = uint32_t(g.tw), uth = uint32_t(g.th);
-    const int tx0 = int(ufx / utw), tx1 = int((ufx + us - 1) / utw);
-    const int ty0 = int(ufy / uth), ty1 = int((ufy + us - 1) / uth);
     int t = 0;
-    for (int ty = ty0; ty <= ty1; ++ty)
-        for (int tx = tx0; tx <= tx1; ++tx) {
-            kp[t] = K(cell0 + uint32_t(ty) * uint32_t(jd.ntx) + uint32_t(tx));
+    for (int ty = f.ty0; ty <= f.ty1; ++ty)
+        for (int tx = f.tx0; tx <= f.tx1; ++tx) {
+            kp[t] = K(f.cell0 + uint32_t(ty) * uint32_t(f.ntx) + uint32_t(tx));
             vp[t] = uint32_t(d);
             ++t;
         }
@@ -144,7 +169,7 @@ __device__ __forceinline__ void sample_keys(const int32_t* __restrict__ iu, cons
         vp[t] = uint32_t(d);
     }
     if (with_anchors) {
-        const uint32_t at = anchor_cell(g, grp, ufx, ufy);
+        const uint32_t at = anchor_cell(g, f.grp, f.fx, f.fy);
         akeys[d] = K(at);
         avals[d] = uint32_t(d);
         atomicAdd(&atile_count[at], 1u);
@@ -226,10 +251,14 @@ __global__ void anchor_keys_kernel(const int32_t* __restrict__ iu, const int32_t
     atomicAdd(&atile_count[at], 1u);
 }
 
-// the job table of a one-job plan (written on the device, so building such a plan is device
-// work only)
-__global__ void one_job_kernel(JobDesc* jobs, uint32_t* job_start, int g_size, int ntx, uint32_t ntiles, uint32_t n)
+// the job table and tile records of a one-job plan (written on the device, so building such a plan
+// is device work only)
+__global__ void one_job_kernel(JobDesc* jobs, uint32_t* job_start, int g_size, int ntx, uint32_t ntiles, uint32_t n,
+                               uint32_t* tinfo)
 {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < ntiles) tinfo[t] = tile_record(0u, t % uint32_t(ntx), t / uint32_t(ntx));
+    if (t != 0) return;
     jobs[0] = JobDesc{nullptr, g_size, ntx, 0u, ntiles};
     job_start[0] = 0;
     job_start[1] = n;
@@ -322,6 +351,53 @@ __device__ __forceinline__ void cell_vals(uint32_t cnt, const CellArgs& a, uint3
     v[5] = dnu > 1 ? dnu : 0u;
 }
 
+// cell c's own entries (all but its units), from its count, the exclusive sums and its values
+__device__ __forceinline__ void cell_entries(uint32_t c, uint32_t cnt, const uint32_t* pre, const uint32_t* v,
+                                             const CellArgs& a)
+{
+    a.tile_start[c] = pre[0];
+    a.tile_count[c] = cnt;
+    if (c % a.ntiles == 0) {
+        const uint32_t gi = c / a.ntiles;
+        a.group_start[gi] = pre[1];
+        a.group_ustart[gi] = pre[2];
+        if (a.own_d) a.d_group_ustart[gi] = pre[4];
+    }
+    if (cnt) {
+        const uint32_t k = pre[1];
+        a.items[k] = c;
+        a.nunits[k] = v[2];
+        a.ustart[k] = pre[2];
+        a.pstart[k] = pre[3];
+        if (a.own_d) {
+            a.d_nunits[k] = v[4];
+            a.d_ustart[k] = pre[4];
+            a.d_pstart[k] = pre[5];
+        }
+    }
+}
+
+// the item-indexed entries k past the last item
+__device__ __forceinline__ void cell_past(uint32_t k, const uint32_t* tot, const CellArgs& a)
+{
+    a.nunits[k] = 0;
+    a.ustart[k] = tot[2];
+    a.pstart[k] = tot[3];
+    if (a.own_d) {
+        a.d_nunits[k] = 0;
+        a.d_ustart[k] = tot[4];
+        a.d_pstart[k] = tot[5];
+    }
+}
+
+__device__ __forceinline__ void cell_totals(const uint32_t* tot, const CellArgs& a)
+{
+    *a.n_items = tot[1];
+    a.group_start[a.n_groups] = tot[1];
+    a.group_ustart[a.n_groups] = tot[2];
+    if (a.own_d) a.d_group_ustart[a.n_groups] = tot[4];
+}
+
 // pairs of each cell: run end - run start (tile_start holds the run starts until cell_out_kernel)
 __device__ __forceinline__ void load_counts(const CellArgs& a, uint32_t c0, uint32_t* cnt)
 {
@@ -397,13 +473,7 @@ __global__ void __launch_bounds__(1024) cell_scan_kernel(CellArgs a, uint32_t bl
         if (threadIdx.x == 0) a.part[size_t(kCellVals) * blocks + j] = carry_s;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const uint32_t* tot = a.part + size_t(kCellVals) * blocks;
-        *a.n_items = tot[1];
-        a.group_start[a.n_groups] = tot[1];
-        a.group_ustart[a.n_groups] = tot[2];
-        if (a.own_d) a.d_group_ustart[a.n_groups] = tot[4];
-    }
+    if (threadIdx.x == 0) cell_totals(a.part + size_t(kCellVals) * blocks, a);
 }
 
 // unit q takes the cell's pairs [floor(q*cnt/nu), floor((q+1)*cnt/nu)), stepped without a division
@@ -467,40 +537,231 @@ __global__ void __launch_bounds__(kCellThreads) cell_out_kernel(CellArgs a)
         if (c >= a.cells) break;
         uint32_t v[kCellVals];
         cell_vals(cnt[e], a, v);
-        a.tile_start[c] = pre[0];
-        a.tile_count[c] = cnt[e];
-        if (c % a.ntiles == 0) {
-            const uint32_t gi = c / a.ntiles;
-            a.group_start[gi] = pre[1];
-            a.group_ustart[gi] = pre[2];
-            if (a.own_d) a.d_group_ustart[gi] = pre[4];
-        }
+        cell_entries(c, cnt[e], pre, v, a);
         if (cnt[e]) {
-            const uint32_t k = pre[1];
-            a.items[k] = c;
-            a.nunits[k] = v[2];
-            a.ustart[k] = pre[2];
-            a.pstart[k] = pre[3];
             write_units(a.units, c, cnt[e], pre[0], v[2], pre[2], pre[3]);
-            if (a.own_d) {
-                a.d_nunits[k] = v[4];
-                a.d_ustart[k] = pre[4];
-                a.d_pstart[k] = pre[5];
-                write_units(a.d_units, c, cnt[e], pre[0], v[4], pre[4], pre[5]);
-            }
+            if (a.own_d) write_units(a.d_units, c, cnt[e], pre[0], v[4], pre[4], pre[5]);
         }
-        if (c >= tot[1]) {  // item-indexed entries past the last item
-            a.nunits[c] = 0;
-            a.ustart[c] = tot[2];
-            a.pstart[c] = tot[3];
-            if (a.own_d) {
-                a.d_nunits[c] = 0;
-                a.d_ustart[c] = tot[4];
-                a.d_pstart[c] = tot[5];
-            }
-        }
+        if (c >= tot[1]) cell_past(c, tot, a);
 #pragma unroll
         for (int j = 0; j < kCellVals; ++j) pre[j] += v[j];
+    }
+}
+
+// Whether every plane group has at most `few` units: the plan is then gridded in slices of its tiles,
+// and the tile kernels' ranges are empty.  One warp.
+__device__ __forceinline__ void plan_mode(const uint32_t* group_ustart, int n_groups, uint32_t few, uint32_t* range,
+                                          unsigned int* sliced)
+{
+    static_assert(kSliceGroups <= 32, "a group per lane");
+    const int g = threadIdx.x;
+    const uint32_t from = g < n_groups ? group_ustart[g] : 0u, to = g < n_groups ? group_ustart[g + 1] : 0u;
+    const bool all_few = __all_sync(0xffffffffu, to - from <= few);
+    if (g < n_groups) {
+        range[2 * g] = all_few ? 0u : from;
+        range[2 * g + 1] = all_few ? 0u : to;
+    }
+    if (threadIdx.x == 0) *sliced = all_few;
+}
+
+__global__ void plan_mode_kernel(const uint32_t* group_ustart, int n_groups, uint32_t few, uint32_t* range,
+                                 unsigned int* sliced)
+{
+    plan_mode(group_ustart, n_groups, few, range, sliced);
+}
+
+// ------------------------------------------------------------------------------------------
+// Binning of few samples: the same arrays as the sort and the cell kernels above make, in three
+// launches.  A sort of 16 k samples is twenty launches of 1 to 10 us with their gaps, 77 us of a call
+// whose gridding takes 162; counted instead of sorted, it is three, each launched while the one
+// before drains: 20 us.  Measured by whole calls (gridding, degridding; real table, us): 300 samples on
+// a 256^2 grid 52, 69 -> 33, 48; 16 k on 1024^2 241, 132 -> 184, 77; 65 k on 2048^2 510, 323 -> 452, 266;
+// on 4000^2, close to the most cells, 501, 429 -> 497, 424.
+//   few_count   a block of 256 samples: a word per warp and cell says which of the warp's samples meet
+//               the cell, so a sample's place among its block's samples of the cell is a population
+//               count, in sample order, and so is the block's count of the cell
+//   few_cells   per cell the exclusive sum of the blocks' counts, in block order; the block that
+//               finishes last makes the cells' offsets, items and work-unit ranges
+//   few_place   every sample index to its place, and the work units
+// For up to 65535 samples (16-bit counts) and 4096 cells (128 KB of words), while a row of counts per
+// block fits in the sort's key arrays and the degridding slots, which binning may use.
+// ------------------------------------------------------------------------------------------
+constexpr int kFewThreads = 256, kFewWarps = kFewThreads / 32;
+constexpr int kFewCellThreads = 512;
+constexpr uint32_t kFewCells = 4096;
+constexpr int64_t kFewSamples = 65535;
+constexpr int kFewRows = int((kFewSamples + kFewThreads - 1) / kFewThreads);  // blocks of samples at most
+constexpr int kTicketWord = 7;  // of the status block: blocks of few_cells_kernel that are done
+
+struct FewArgs {
+    const int32_t *iu, *iv, *coff;
+    const JobDesc* jobs;
+    const uint32_t* job_start;
+    VarPlanes var;
+    uint16_t *row0, *row1;  // counts of blocks [0, rows0) and from rows0 on, a row of `cells` each
+    uint32_t rows0, blocks, cells;
+    uint8_t* place;   // per pair: its sample's place among its block's samples of the cell
+    uint32_t* nrej;   // per block: samples left out
+    uint16_t* ntl;
+    uint32_t* vals;
+    unsigned long long* rejected;
+    unsigned int* status;
+    uint32_t few;      // gridding in slices up to this many units a group (plan_mode_kernel)
+    uint32_t* range;   // or null
+    __device__ uint16_t* row(uint32_t b) const
+    {
+        return b < rows0 ? row0 + size_t(b) * cells : row1 + size_t(b - rows0) * cells;
+    }
+};
+
+__global__ void __launch_bounds__(kFewThreads) few_count_kernel(FewArgs f, PlanGeom g)
+{
+    extern __shared__ __align__(16) uint32_t few_meet[];  // [warp][cell]: the lanes whose samples meet the cell
+    const uint32_t stride = (f.cells + 3u) & ~3u;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (uint32_t i = threadIdx.x; i < kFewWarps * stride / 4; i += kFewThreads)
+        reinterpret_cast<uint4*>(few_meet)[i] = make_uint4(0, 0, 0, 0);
+    if (blockIdx.x == 0 && threadIdx.x < kStatusWords) f.status[threadIdx.x] = 0;
+    const int64_t d = int64_t(blockIdx.x) * kFewThreads + threadIdx.x;
+    Reach r{};
+    if (d < g.n) {
+        r = reach_of(f.iu, f.iv, f.coff, g, f.jobs, f.job_start, d, f.var);
+        if (g.var) f.var.ssz[d] = uint16_t(r.s);
+        f.ntl[d] = uint16_t(r.ok ? (r.tx1 - r.tx0 + 1) * (r.ty1 - r.ty0 + 1) : 0);
+    }
+    const int left_out = __syncthreads_count(d < g.n && !r.ok);
+    if (threadIdx.x == 0) f.nrej[blockIdx.x] = uint32_t(left_out);
+    auto each_cell = [&](auto&& take) {
+        if (!r.ok) return;
+        for (int ty = r.ty0; ty <= r.ty1; ++ty)
+            for (int tx = r.tx0; tx <= r.tx1; ++tx) take(r.cell0 + uint32_t(ty) * uint32_t(r.ntx) + uint32_t(tx));
+    };
+    each_cell([&](uint32_t c) { atomicOr(&few_meet[warp * stride + c], 1u << lane); });
+    __syncthreads();
+    uint8_t* place = f.place + d * g.max_tiles;
+    each_cell([&](uint32_t c) {
+        uint32_t before = __popc(few_meet[warp * stride + c] & ((1u << lane) - 1u));
+        for (int k = 0; k < warp; ++k) before += __popc(few_meet[k * stride + c]);
+        *place++ = uint8_t(before);
+    });
+    uint16_t* row = f.row(blockIdx.x);
+    for (uint32_t c = threadIdx.x; c < f.cells; c += kFewThreads) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < kFewWarps; ++k) sum += __popc(few_meet[k * stride + c]);
+        row[c] = uint16_t(sum);
+    }
+}
+
+// 32 cells per block, a warp per sixteenth of the rows
+__global__ void __launch_bounds__(kFewCellThreads) few_cells_kernel(FewArgs f, CellArgs a)
+{
+    constexpr int kWarps = kFewCellThreads / 32, kPer = kFewRows / kWarps;
+    static_assert(kFewRows % kWarps == 0 && kCellVals * kWarps <= 128, "rows per warp");
+    __shared__ uint32_t part[kWarps][32], ws[kCellVals][kWarps];
+    __shared__ uint32_t last_s, rej_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cudaGridDependencySynchronize();
+    const uint32_t c = blockIdx.x * 32u + lane;
+    const uint32_t per = (f.blocks + kWarps - 1) / kWarps, r0 = warp * per;
+    uint32_t v[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        v[k] = 0;
+        if (k < int(per) && r0 + k < f.blocks && c < f.cells) v[k] = f.row(r0 + k)[c];
+        sum += v[k];
+    }
+    part[warp][lane] = sum;
+    __syncthreads();
+    uint32_t pre = 0;
+    for (int k = 0; k < warp; ++k) pre += part[k][lane];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+        if (k < int(per) && r0 + k < f.blocks && c < f.cells) {
+            f.row(r0 + k)[c] = uint16_t(pre);
+            pre += v[k];
+        }
+    if (warp == kWarps - 1 && c < f.cells) a.tile_count[c] = pre;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last_s = atomicAdd(f.status + kTicketWord, 1u) == gridDim.x - 1;
+        rej_s = 0;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    // the last block: all counts are there
+    uint32_t carry[kCellVals] = {};
+    for (uint32_t base = 0; base < a.cells; base += kFewCellThreads) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t cnt = i < a.cells ? __ldcg(a.tile_count + i) : 0u;
+        uint32_t s[kCellVals], x[kCellVals];
+        cell_vals(cnt, a, s);
+#pragma unroll
+        for (int j = 0; j < kCellVals; ++j) {
+            x[j] = s[j];
+#pragma unroll
+            for (int e = 1; e < 32; e <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x[j], e);
+                if (lane >= e) x[j] += y;
+            }
+            if (lane == 31) ws[j][warp] = x[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kCellVals; ++j) {
+            uint32_t lower = 0, all = 0;
+#pragma unroll
+            for (int k = 0; k < kWarps; ++k) {
+                const uint32_t y = ws[j][k];
+                lower += k < warp ? y : 0u;
+                all += y;
+            }
+            x[j] += carry[j] + lower - s[j];
+            carry[j] += all;
+        }
+        __syncthreads();  // ws is read
+        if (i < a.cells) cell_entries(i, cnt, x, s, a);
+    }
+    for (uint32_t i = threadIdx.x; i < f.blocks; i += kFewCellThreads) atomicAdd(&rej_s, f.nrej[i]);
+    for (uint32_t i = carry[1] + threadIdx.x; i < a.cells; i += kFewCellThreads) cell_past(i, carry, a);
+    if (threadIdx.x == 0) cell_totals(carry, a);
+    __syncthreads();
+    if (warp == 0 && f.range) plan_mode(a.group_ustart, a.n_groups, f.few, f.range, f.status + kSliceWord);
+    if (threadIdx.x == 0) {
+        *f.rejected = rej_s;
+        f.status[kTicketWord] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(kFewThreads) few_place_kernel(FewArgs f, PlanGeom g, CellArgs a)
+{
+    const int64_t d = int64_t(blockIdx.x) * kFewThreads + threadIdx.x;
+    Reach r{};
+    if (d < g.n) r = reach_of(f.iu, f.iv, f.coff, g, f.jobs, f.job_start, d, f.var);
+    cudaGridDependencySynchronize();
+    const uint16_t* row = f.row(blockIdx.x);
+    if (r.ok) {
+        const uint8_t* place = f.place + d * g.max_tiles;
+        for (int ty = r.ty0; ty <= r.ty1; ++ty)
+            for (int tx = r.tx0; tx <= r.tx1; ++tx) {
+                const uint32_t c = r.cell0 + uint32_t(ty) * uint32_t(r.ntx) + uint32_t(tx);
+                f.vals[a.tile_start[c] + row[c] + *place++] = uint32_t(d);
+            }
+    }
+    // the units, a warp per cell: unit q takes the cell's pairs [q*cnt/nu, (q+1)*cnt/nu)
+    const uint32_t n_items = *a.n_items, lane = threadIdx.x & 31;
+    for (uint32_t k = blockIdx.x * kFewWarps + (threadIdx.x >> 5); k < n_items; k += gridDim.x * kFewWarps) {
+        const uint32_t c = a.items[k], cnt = a.tile_count[c], first = a.tile_start[c];
+        auto units = [&](uint4* out, uint32_t nu, uint32_t u0, uint32_t p0) {
+            for (uint32_t q = lane; q < nu; q += 32) {
+                const uint32_t b0 = q * cnt / nu, b1 = (q + 1) * cnt / nu;  // cnt and nu fit 16 bits
+                out[u0 + q] = make_uint4(c, first + b0, b1 - b0, nu > 1 ? p0 + q : kDirect);
+            }
+        };
+        units(a.units, a.nunits[k], a.ustart[k], a.pstart[k]);
+        if (a.own_d) units(a.d_units, a.d_nunits[k], a.d_ustart[k], a.d_pstart[k]);
     }
 }
 
@@ -592,32 +853,30 @@ tcv_status plan_anchors_ready(const tcv_plan* cp, cudaStream_t st)
     return s;
 }
 
-// Whether every plane group has at most `few` units: the plan is then gridded in slices of its tiles,
-// and the tile kernels' ranges are empty.
-__global__ void plan_mode_kernel(const uint32_t* __restrict__ group_ustart, int n_groups, uint32_t few, uint32_t* range,
-                                 unsigned int* sliced)
+CellArgs cell_args(const tcv_plan* p)
 {
-    static_assert(kSliceGroups <= 32, "a group per lane");
-    const int g = threadIdx.x;
-    const uint32_t from = g < n_groups ? group_ustart[g] : 0u, to = g < n_groups ? group_ustart[g + 1] : 0u;
-    const bool all_few = __all_sync(0xffffffffu, to - from <= few);
-    if (g < n_groups) {
-        range[2 * g] = all_few ? 0u : from;
-        range[2 * g + 1] = all_few ? 0u : to;
-    }
-    if (threadIdx.x == 0) *sliced = all_few;
+    const PlanGeom& g = p->g;
+    const bool own_d = own_degrid_units(g);
+    return CellArgs{p->tile_count, uint32_t(grid_cells(g)), uint32_t(g.ntiles), uint32_t(g.split), uint32_t(g.dsplit),
+                    g.n_groups, own_d, g.uniq ? p->n_uniq + 1 : nullptr, static_cast<uint32_t*>(p->cub_temp),
+                    p->tile_start, p->items, p->n_items, p->group_start, p->nunits, p->ustart, p->pstart,
+                    p->group_ustart, p->units, own_d ? p->d_nunits : nullptr, own_d ? p->d_ustart : nullptr,
+                    own_d ? p->d_pstart : nullptr, own_d ? p->d_group_ustart : nullptr, own_d ? p->d_units : nullptr};
+}
+
+// busy tiles of a group up to which a plan is gridded in slices of them (tcv_grid.cu)
+uint32_t few_units()
+{
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return uint32_t(sms) * 6u / 5u;
 }
 
 // The cells' bookkeeping from their ranges (tile_start: starts, tile_count: ends).
 tcv_status cells_and_units(tcv_plan* p, cudaStream_t st)
 {
     const PlanGeom& g = p->g;
-    const bool own_d = own_degrid_units(g);
-    const CellArgs ca{p->tile_count, uint32_t(grid_cells(g)), uint32_t(g.ntiles), uint32_t(g.split), uint32_t(g.dsplit),
-                      g.n_groups, own_d, g.uniq ? p->n_uniq + 1 : nullptr, static_cast<uint32_t*>(p->cub_temp),
-                      p->tile_start, p->items, p->n_items, p->group_start, p->nunits, p->ustart, p->pstart,
-                      p->group_ustart, p->units, own_d ? p->d_nunits : nullptr, own_d ? p->d_ustart : nullptr,
-                      own_d ? p->d_pstart : nullptr, own_d ? p->d_group_ustart : nullptr, own_d ? p->d_units : nullptr};
+    const CellArgs ca = cell_args(p);
     const uint32_t cb = cell_blocks(g);
     cell_sums_kernel<<<cb, kCellThreads, 0, st>>>(ca);
     TCV_CUDA(cudaGetLastError());
@@ -626,11 +885,50 @@ tcv_status cells_and_units(tcv_plan* p, cudaStream_t st)
     cell_out_kernel<<<cb, kCellThreads, 0, st>>>(ca);
     TCV_CUDA(cudaGetLastError());
     if (!p->grid_range) return TCV_OK;
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    plan_mode_kernel<<<1, 32, 0, st>>>(p->group_ustart, g.n_groups, uint32_t(sms) * 6u / 5u, p->grid_range,
-                                       p->status + kSliceWord);
+    plan_mode_kernel<<<1, 32, 0, st>>>(p->group_ustart, g.n_groups, few_units(), p->grid_range, p->status + kSliceWord);
     TCV_CUDA(cudaGetLastError());
+    return TCV_OK;
+}
+
+// Binning by counting, where the plan allows it (*done false: nothing was launched).
+tcv_status build_few(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_t* coff, cudaStream_t st, bool* done)
+{
+    const PlanGeom& g = p->g;
+    *done = false;
+    const size_t cells = grid_cells(g), np = size_t(g.n) * g.max_tiles, ks = g.key64 ? 8 : 4;
+    if (g.n < 1 || g.n > kFewSamples || g.uniq || cells > kFewCells) return TCV_OK;
+    FewArgs f{};
+    f.blocks = uint32_t((g.n + kFewThreads - 1) / kFewThreads);
+    f.cells = uint32_t(cells);
+    f.rows0 = uint32_t(std::min<size_t>(2 * align_up(np * ks) / (2 * cells), f.blocks));  // keys[1] follows keys[0]
+    if (f.rows0 + align_up(np * sizeof(float2)) / (2 * cells) < f.blocks) return TCV_OK;
+    f.iu = iu;
+    f.iv = iv;
+    f.coff = coff;
+    f.jobs = p->jobs;
+    f.job_start = p->job_start;
+    f.var = VarPlanes{p->wplane, p->plane_s, p->plane_grp, p->ssz};
+    f.row0 = static_cast<uint16_t*>(p->keys[0]);
+    f.row1 = reinterpret_cast<uint16_t*>(p->slots);
+    f.nrej = p->vals[1];  // a word per block, then a byte per pair: fewer than 4 np bytes
+    f.place = reinterpret_cast<uint8_t*>(p->vals[1] + f.blocks);
+    f.ntl = p->ntl;
+    f.vals = p->vals[0];
+    f.rejected = p->rejected;
+    f.status = p->status;
+    f.few = few_units();
+    f.range = p->grid_range;
+    const CellArgs ca = cell_args(p);
+    const size_t smem = size_t(kFewWarps) * ((cells + 3) & ~size_t(3)) * 4;
+    if (smem > 48 * 1024)
+        TCV_CUDA(cudaFuncSetAttribute(few_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(kFewWarps * kFewCells * 4)));
+    few_count_kernel<<<f.blocks, kFewThreads, smem, st>>>(f, g);
+    TCV_CUDA(cudaGetLastError());
+    TCV_CHECK(launch_behind(&few_cells_kernel, unsigned((cells + 31) / 32), kFewCellThreads, st, f, ca));
+    TCV_CHECK(launch_behind(&few_place_kernel, f.blocks, kFewThreads, st, f, g, ca));
+    p->sel = 0;
+    *done = true;
     return TCV_OK;
 }
 
@@ -656,6 +954,15 @@ tcv_status build(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_
     const int64_t np = g.n * g.max_tiles;
     const int cells = int(grid_cells(g)), acells = int(anchor_cells(g));
     const bool with_anchors = g.anchors && p->degrid_variant == TCV_DEGRID_ANCHOR;
+    if (!with_anchors) {
+        bool done = false;
+        TCV_CHECK(build_few(p, iu, iv, coff, st, &done));
+        if (done) {
+            p->anchors_ready = false;
+            if (g.anchors && stream_capturing(st)) p->anchors_stale = true;  // as below
+            return TCV_OK;
+        }
+    }
     TCV_CUDA(cudaMemsetAsync(p->tile_count, 0, sizeof(uint32_t) * size_t(cells), st));  // run ends
     TCV_CUDA(cudaMemsetAsync(p->tile_start, 0, sizeof(uint32_t) * size_t(cells), st));  // run starts
     if (with_anchors) TCV_CUDA(cudaMemsetAsync(p->atile_count, 0, sizeof(uint32_t) * size_t(acells), st));
@@ -806,11 +1113,13 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
                                  cudaMemcpyHostToDevice, st));
         TCV_CUDA(cudaMemcpyAsync(p->job_start, p->host_job_start.data(), p->host_job_start.size() * 4,
                                  cudaMemcpyHostToDevice, st));
-    } else {
-        one_job_kernel<<<1, 1, 0, st>>>(p->jobs, p->job_start, g.g_size, g.ntx, uint32_t(g.ntiles), uint32_t(g.n));
-        TCV_CUDA(cudaGetLastError());
     }
-    tile_info_kernel<<<unsigned((g.ntiles + 255) / 256), 256, 0, st>>>(p->jobs, g.n_jobs, uint32_t(g.ntiles), p->tinfo);
+    const unsigned tile_blocks = unsigned((g.ntiles + 255) / 256);
+    if (p->batch)
+        tile_info_kernel<<<tile_blocks, 256, 0, st>>>(p->jobs, g.n_jobs, uint32_t(g.ntiles), p->tinfo);
+    else
+        one_job_kernel<<<tile_blocks, 256, 0, st>>>(p->jobs, p->job_start, g.g_size, g.ntx, uint32_t(g.ntiles),
+                                                    uint32_t(g.n), p->tinfo);
     TCV_CUDA(cudaGetLastError());
     if (g.var) {  // the plane widths and groups (host vectors owned by the plan)
         TCV_CUDA(cudaMemcpyAsync(p->plane_s, p->host_plane_s.data(), size_t(g.n_planes) * 4, cudaMemcpyHostToDevice, st));
