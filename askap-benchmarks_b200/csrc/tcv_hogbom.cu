@@ -30,7 +30,7 @@
 // exchange candidates through distributed shared memory: an iteration is a chain of latencies
 // (bounds, the hot blocks' loads, the exchange: 5 us at 4096^2), not a pass over the image.
 // hog_apply_kernel follows on the whole device: it brings blocks near the peak up to date, and
-// every kRing iterations and at the end all blocks (9 us an iteration at 4096^2, most of it the PSF
+// every kRing iterations and at the end all blocks (7.7 us an iteration at 4096^2, most of it the PSF
 // windows from L2).  A pixel's updates are applied in iteration order with the reference's
 // roundings whenever they are applied, so the bits do not depend on the schedule.
 //
@@ -45,7 +45,7 @@
 //
 // Measured on one B200, us an iteration, and in brackets with one pass over the image per iteration
 // (in one cooperative launch up to 48 MiB of images, all CTAs waiting on one counter; a launch
-// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1884^2 6.8 (8.2), 4096^2 16.5 (27.0).
+// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1884^2 6.8 (8.2), 4096^2 12.9 (27.0).
 #include "tcv_internal.cuh"
 
 #include <cooperative_groups.h>
@@ -358,7 +358,8 @@ constexpr int kLeadIters = 16;       // iterations per launch of the cluster (ev
 constexpr int kRing = 128;           // iterations whose updates may be pending (a multiple of kLeadIters)
 constexpr int kApplyThreads = 128;
 constexpr int kApplyRows = 4;        // rows per warp: a CTA works on 32 x 16 pixels at a time
-constexpr int kSlots = 48;           // PSF windows of that size an applying CTA holds
+constexpr int kApplyDeep = 4;        // windows whose copies are issued together
+constexpr int kSlots = 52;           // PSF windows of that size an applying CTA holds
 constexpr int kStrips = 32 / (kApplyThreads / 32 * kApplyRows);  // parts of 32 columns a 32 x 32 square is worked on in
 constexpr int kWindow = kApplyThreads * kApplyRows;  // pixels of a window
 
@@ -1037,16 +1038,23 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
 // PSF values it needs come from windows in shared memory, in which every lane copies
 // (asynchronously) and reads its own places only: updates at one peak share a window, so the
 // loads from L2 are one per distinct peak of a batch, not one per update, and an update of a pixel
-// costs 4 bytes from shared memory, a product and a difference.
+// costs 4 bytes from shared memory, a product and a difference.  Two CTAs of four warps fit on an SM,
+// so the copy loop is a chain of latencies: a window's place and cover come in one 16-byte read, the
+// reads of four windows go ahead of their copies, and a warp's places of a row are neighbours (one
+// float4 a lane made the copies conflict four ways): 15.9 -> 13.5 us an iteration at 4096^2; 52
+// windows, the most that two CTAs hold, 12.9 (48: 13.5; 32 at three CTAs: 15.3).  A pass of 128 updates
+// over all blocks takes 0.83 ms; loading each update's 4 bytes a pixel from L2 would take 0.67 alone.
+// Copying one batch while computing another (two halves of 25 windows) took 20 us an iteration.
 __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, int base, int all)
 {
     constexpr int kRows = kApplyRows;
-    static_assert(kRows == 4, "one float4 per lane and window");
+    static_assert(kRows % 2 == 0, "rows in pairs");
     extern __shared__ __align__(16) float apply_win[];  // [kSlots][kWindow]
     __shared__ Update ring[kRing];
     __shared__ UpdateSlot slots[kRing];
     __shared__ float2 code[kRing];  // of the part's updates in order: -t and, as bits, the window
-    __shared__ unsigned short which[kRing], load[kSlots];  // ring entries: of the codes; to copy windows of
+    __shared__ unsigned short which[kRing];               // the codes' ring entries
+    __shared__ int4 load[kSlots + kApplyDeep];            // windows to copy: PSF offset, place, columns, rows
     __shared__ unsigned short batch_end[kRing];
     __shared__ int warps[2][kApplyThreads / 32];
     __shared__ unsigned long long wk[kApplyThreads / 32];
@@ -1060,7 +1068,7 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
         slots[i] = a.slots[i];
         if (i + 1 == q1 || a.slots[i + 1].batch != a.slots[i].batch) batch_end[a.slots[i].batch] = (unsigned short)(i + 1);
     }
-    float4* const mine = reinterpret_cast<float4*>(apply_win) + tid;  // this lane's place in the first window
+    float* const mine = apply_win + tid;  // this lane's place in the first window
     for (int item = int(blockIdx.x); item < count; item += int(gridDim.x)) {
         const int b = all ? item : int(a.warm[item]);
         const int q0 = a.applied[b] - base;
@@ -1107,22 +1115,30 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
                     }
                     if (cover) {
                         at += __popc(bu & ((1u << lane) - 1u));
-                        code[at] = make_float2(-ring[i].t, __int_as_float(int(slots[i].slot) * kApplyThreads));
+                        code[at] = make_float2(-ring[i].t, __int_as_float(int(slots[i].slot) * kWindow));
                         which[at] = (unsigned short)(i);
                     }
-                    if (copy) load[atc + __popc(bc & ((1u << lane) - 1u))] = (unsigned short)(i);
+                    if (copy)
+                        load[atc + __popc(bc & ((1u << lane) - 1u))] =
+                            make_int4(ring[i].off, int(slots[i].slot) * kWindow, int(ring[i].xr), int(ring[i].yr));
                     __syncthreads();
                 }
-                for (int i = 0; i < nc; ++i) {
-                    const int e = load[i];
-                    const Update u = ring[e];
-                    float* w = reinterpret_cast<float*>(mine + int(slots[e].slot) * kApplyThreads);
-                    const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
-                    const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
+                for (int i0 = 0; i0 < nc; i0 += kApplyDeep) {
+                    int4 e[kApplyDeep];
 #pragma unroll
-                    for (int k = 0; k < kRows; ++k)
-                        if (cx && y + k >= ya && y + k <= yb)
-                            __pipeline_memcpy_async(w + k, pp + (u.off + ptrdiff_t(k) * P), 4);
+                    for (int d = 0; d < kApplyDeep; ++d) e[d] = load[i0 + d];
+#pragma unroll
+                    for (int d = 0; d < kApplyDeep; ++d) {
+                        if (i0 + d >= nc) break;
+                        const float* __restrict__ src = pp + e[d].x;
+                        float* w = mine + e[d].y;
+                        const int ya = e[d].w & 0xffff, yb = int(unsigned(e[d].w) >> 16);
+                        const bool cx = x >= (e[d].z & 0xffff) && x <= int(unsigned(e[d].z) >> 16);
+#pragma unroll
+                        for (int k = 0; k < kRows; ++k)
+                            if (!partial || (cx && y + k >= ya && y + k <= yb))
+                                __pipeline_memcpy_async(w + k * kApplyThreads, src + ptrdiff_t(k) * P, 4);
+                    }
                 }
                 __pipeline_commit();
                 __pipeline_wait_prior(0);  // a lane reads only what it copied: no barrier
@@ -1132,23 +1148,24 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
 #pragma unroll 8
                     for (int i = 0; i < n; ++i) {
                         const float2 cd = code[i], nt = make_float2(cd.x, cd.x);
-                        const float4 w = mine[__float_as_int(cd.y)];
-                        const float2 s = __fmul2_rn(nt, make_float2(w.x, w.y)), v = __fmul2_rn(nt, make_float2(w.z, w.w));
-                        r[0] = __fadd_rn(r[0], s.x);
-                        r[1] = __fadd_rn(r[1], s.y);
-                        r[2] = __fadd_rn(r[2], v.x);
-                        r[3] = __fadd_rn(r[3], v.y);
+                        const float* w = mine + __float_as_int(cd.y);
+#pragma unroll
+                        for (int k = 0; k < kRows; k += 2) {
+                            const float2 s = __fmul2_rn(nt, make_float2(w[k * kApplyThreads], w[(k + 1) * kApplyThreads]));
+                            r[k] = __fadd_rn(r[k], s.x);
+                            r[k + 1] = __fadd_rn(r[k + 1], s.y);
+                        }
                     }
                 } else {
                     for (int i = 0; i < n; ++i) {
                         const float2 cd = code[i];
                         const Update u = ring[which[i]];
-                        const float* w = reinterpret_cast<const float*>(mine + __float_as_int(cd.y));
+                        const float* w = mine + __float_as_int(cd.y);
                         const int ya = int(u.yr & 0xffffu), yb = int(u.yr >> 16);
                         const bool cx = x >= int(u.xr & 0xffffu) && x <= int(u.xr >> 16);
 #pragma unroll
                         for (int k = 0; k < kRows; ++k)
-                            if (cx && y + k >= ya && y + k <= yb) r[k] = __fadd_rn(r[k], __fmul_rn(cd.x, w[k]));
+                            if (cx && y + k >= ya && y + k <= yb) r[k] = __fadd_rn(r[k], __fmul_rn(cd.x, w[k * kApplyThreads]));
                     }
                 }
                 first = end;
