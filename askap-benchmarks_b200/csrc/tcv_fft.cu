@@ -36,6 +36,7 @@
 
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -177,6 +178,10 @@ __device__ __forceinline__ void dft(float2 (&v)[R])
     }
 }
 
+// Where the stage of ns = 2^log_ns (a multiple of 4, above 0) starts in the row pass's twiddles by
+// stage, in float4: the earlier stages have 2 ns each, 2 * (16 + 256 + ...).
+__host__ __device__ constexpr int packed_at(int log_ns) { return 2 * (((1 << log_ns) - 16) / 15); }
+
 // One radix-R Stockham stage over `lines` lines of length 2^log2n held in shared memory (line
 // l at l << log2n, padded), in place: every butterfly reads R values Nl/R apart, multiplies
 // value r by exp(-+2 pi i r (j mod Ns) / (Ns R)), takes the R-point DFT and writes the results
@@ -215,19 +220,30 @@ __device__ __forceinline__ void stage(float2* sm, int log2n, int log_ns, const f
             // twiddles w^r, w = exp(-+2 pi i kk / (Ns R)): r = 1, 2, 4, 8 from the table, the rest as products
             const int t = kk << (log2n - log_ns - kLogR + tscale);
             float2 w[R];
-            w[1] = conj_if<kInverse>(__ldg(tw + t));
-            if (R > 2) {
-                w[2] = conj_if<kInverse>(__ldg(tw + 2 * t));
-                w[3] = cmul(w[1], w[2]);
+            constexpr bool kPacked = kLines == 0 && R > 2;  // the rows' table by stage (fft_resources)
+            if constexpr (kPacked) {
+                const float4* by_stage = reinterpret_cast<const float4*>(tw + (1 << log2n)) + packed_at(log_ns) + kk;
+                const float4 a = __ldg(by_stage);
+                w[1] = conj_if<kInverse>(make_float2(a.x, a.y));
+                w[2] = conj_if<kInverse>(make_float2(a.z, a.w));
+                if constexpr (R > 4) {
+                    const float4 b = __ldg(by_stage + ns);
+                    w[4] = conj_if<kInverse>(make_float2(b.x, b.y));
+                    if constexpr (R > 8) w[8] = conj_if<kInverse>(make_float2(b.z, b.w));
+                }
+            } else {
+                w[1] = conj_if<kInverse>(__ldg(tw + t));
+                if constexpr (R > 2) w[2] = conj_if<kInverse>(__ldg(tw + 2 * t));
+                if constexpr (R > 4) w[4] = conj_if<kInverse>(__ldg(tw + 4 * t));
+                if constexpr (R > 8) w[8] = conj_if<kInverse>(__ldg(tw + 8 * t));
             }
-            if (R > 4) {
-                w[4] = conj_if<kInverse>(__ldg(tw + 4 * t));
+            if constexpr (R > 2) w[3] = cmul(w[1], w[2]);
+            if constexpr (R > 4) {
                 w[5] = cmul(w[1], w[4]);
                 w[6] = cmul(w[2], w[4]);
                 w[7] = cmul(w[3], w[4]);
             }
-            if (R > 8) {
-                w[8] = conj_if<kInverse>(__ldg(tw + 8 * t));
+            if constexpr (R > 8) {
 #pragma unroll
                 for (int r = 9; r < R; ++r) w[r] = cmul(w[r - 8], w[8]);
             }
@@ -362,7 +378,10 @@ fft_cols2_kernel(const float2* __restrict__ buf, float2* __restrict__ out, float
 
 struct FftRes {
     int device, n;
-    float2* tw;       // exp(-2 pi i k / n), k < n
+    float2* tw;       // exp(-2 pi i k / n), k < n; then the row pass's by stage: of its value j mod Ns = k,
+                      // (w, w^2) for k < Ns, (w^4, w^8) for k < Ns.  Read from the plain table, sixteen
+                      // neighbouring lanes' w^8 are sixteen cache lines, as much work for the load unit as the
+                      // stage's values: rows of 4096 took 55 (image in) and 58 us, now 44 and 48
     float2* scratch;  // n x n complex: the row pass's output, transformed in place by the first column pass
 };
 std::vector<FftRes> g_fft_res;  // guarded by g_fft_mu
@@ -395,10 +414,21 @@ tcv_status fft_resources(int n, FftRes* out)
         const double a = 2.0 * pi * double(k) / double(n);
         h[size_t(k)] = make_float2(float(std::cos(a)), float(-std::sin(a)));
     }
+    const int log2n = ilog2(n);
+    for (int log_ns = 4; log_ns < log2n; log_ns += 4) {
+        const int ns = 1 << log_ns, log_r = std::min(4, log2n - log_ns);
+        for (int part = 0; part < 2; ++part)
+            for (int k = 0; k < ns; ++k) {
+                const size_t t = size_t(k) << (log2n - log_ns - log_r);
+                const size_t mask = size_t(n) - 1;
+                h.push_back(h[(t << (2 * part)) & mask]);
+                h.push_back(h[(t << (2 * part + 1)) & mask]);
+            }
+    }
     FftRes r{dev, n, nullptr, nullptr};
-    TCV_CUDA(cudaMalloc(&r.tw, size_t(n) * sizeof(float2)));
+    TCV_CUDA(cudaMalloc(&r.tw, h.size() * sizeof(float2)));
     cudaError_t e = cudaMalloc(&r.scratch, size_t(n) * size_t(n) * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMemcpy(r.tw, h.data(), size_t(n) * sizeof(float2), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(r.tw, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(r.tw);
         if (r.scratch) cudaFree(r.scratch);
