@@ -12,21 +12,23 @@
 //     S F S X = F D S X:   transform of (-1)^(x+y) X[x + N/2]             (from a real model image)
 // Signs are exact, so only the transform rounds.
 //
-// Power-of-two sizes 128 .. 8192 use this file's own transform, in three passes over the grid:
+// Power-of-two sizes 128 .. 8192 use this file's own transform, in two passes over the grid (256 ..
+// 2048: rows, whole columns) or three:
 //   rows:    each CTA holds whole rows (4096 values, 256 threads; one row of 8192 with 512),
 //            transforms them in shared memory and writes them to a scratch grid;
 //   columns: the four-step split of a column of n = N1 N2 (y = N2 y1 + y2, k = k1 + N1 k2): a
 //            CTA holds 16 adjacent columns (128-byte row segments) of the N1 rows of one y2,
 //            takes their DFT_N1, multiplies by exp(-+2 pi i y2 k1 / n) and writes them back in
 //            place; then a CTA holds the N2 contiguous rows of one k1 and writes DFT_N2 to rows
-//            k1 + N1 k2 of the output.
+//            k1 + N1 k2 of the output;
+//   whole columns: a CTA holds 8 columns.
 // Each 1-D transform is the Stockham autosort form (Govindaraju et al., "High performance discrete
 // Fourier transforms on graphics processors", SC 2008) with radix-16 stages (a 16-point DFT in
 // registers as 4 x 4) and one radix-2, -4 or -8 stage for the rest of the exponent: a butterfly
 // reads R values, multiplies value r by exp(-+2 pi i r (j mod Ns) / (Ns R)), takes the R-point
 // DFT and writes the results Ns apart, so the output comes out in natural order.  The twiddles
 // come from a table of exp(-2 pi i k / n) computed in double precision and rounded once: w, w^2,
-// w^4, w^8 are read and the other powers formed as products.  The rotation and sign separate by
+// w^4, w^8 are read and the other powers formed as products (whole columns read them all).  The rotation and sign separate by
 // axis, so the row pass applies the row's half (value p = (-1)^p Z[p + n/2]) and the last column
 // pass the column's; the model step builds the complex rows from the float image in the row pass,
 // and image formation writes the float image from the last column pass.  Other even sizes use
@@ -87,6 +89,13 @@ __device__ __forceinline__ float chk(int x, int y) { return ((x + y) & 1) ? -1.f
 // Hand-written transform (power-of-two sizes)
 // ------------------------------------------------------------------------------------------
 constexpr int kFftMinN = 128, kFftMaxN = 8192;
+// Sizes 256 .. 2048 transform whole columns in one pass, 8 per CTA: two launches for three and 16 bytes
+// less traffic a value.  Image to grid and back, us, in brackets with the columns in two passes: 256^2
+// 21.8 (26.2), 512^2 21.7 (26.6), 1024^2 24.6 (36.4), 2048^2 64.6 (68.8).  4096^2 would hold 4 columns of 32 bytes a CTA, one
+// CTA an SM: 275 to 296 (270).  The pass reads all its twiddles from a table: powers formed as products made
+// its error larger than the two passes' (2048^2: 1.91e-7 of the values' norm against 1.89e-7; now 1.80e-7).
+// At 128^2 it stays larger all the same (1.344e-7 against 1.341e-7): two passes there.
+constexpr int kWholeMinLog = 8, kWholeLog = 11;
 constexpr int kColW = 16;  // columns per column-pass CTA: 128-byte row segments
 __host__ __device__ constexpr int fft_pad(int p) { return p + (p >> 4); }  // one slot in 16: fewer bank conflicts
 
@@ -182,6 +191,12 @@ __device__ __forceinline__ void dft(float2 (&v)[R])
 // stage, in float4: the earlier stages have 2 ns each, 2 * (16 + 256 + ...).
 __host__ __device__ constexpr int packed_at(int log_ns) { return 2 * (((1 << log_ns) - 16) / 15); }
 
+// and the whole columns' behind all of those, all of a value's together: 8 per value
+__host__ __device__ constexpr int full_at(int log2n, int log_ns)
+{
+    return packed_at((log2n + 3) / 4 * 4) + 8 * (((1 << log_ns) - 16) / 15);
+}
+
 // One radix-R Stockham stage over `lines` lines of length 2^log2n held in shared memory (line
 // l at l << log2n, padded), in place: every butterfly reads R values Nl/R apart, multiplies
 // value r by exp(-+2 pi i r (j mod Ns) / (Ns R)), takes the R-point DFT and writes the results
@@ -194,7 +209,7 @@ __host__ __device__ constexpr int packed_at(int log_ns) { return 2 * (((1 << log
 template <int kLines>
 __device__ __forceinline__ int fft_at(int l, int i, int log2n)
 {
-    return kLines ? i * kLines + l : fft_pad((l << log2n) + i);
+    return kLines == 0 ? fft_pad((l << log2n) + i) : kLines < kColW ? fft_pad(i) * kLines + l : i * kLines + l;
 }
 
 template <int R, bool kInverse, int kPer, int kLines, bool kSrcSm, bool kDstSm, class Load, class Store>
@@ -221,7 +236,16 @@ __device__ __forceinline__ void stage(float2* sm, int log2n, int log_ns, const f
             const int t = kk << (log2n - log_ns - kLogR + tscale);
             float2 w[R];
             constexpr bool kPacked = kLines == 0 && R > 2;  // the rows' table by stage (fft_resources)
-            if constexpr (kPacked) {
+            constexpr bool kFull = kLines > 0 && kLines < kColW;  // the whole columns': all R, no products
+            if constexpr (kFull) {
+                const float4* all = reinterpret_cast<const float4*>(tw + (1 << log2n)) + full_at(log2n, log_ns) + kk * 8;
+#pragma unroll
+                for (int r = 0; r < R; r += 2) {
+                    const float4 a = __ldg(all + r / 2);
+                    w[r] = conj_if<kInverse>(make_float2(a.x, a.y));  // w[0] = 1, not used
+                    w[r + 1] = conj_if<kInverse>(make_float2(a.z, a.w));
+                }
+            } else if constexpr (kPacked) {
                 const float4* by_stage = reinterpret_cast<const float4*>(tw + (1 << log2n)) + packed_at(log_ns) + kk;
                 const float4 a = __ldg(by_stage);
                 w[1] = conj_if<kInverse>(make_float2(a.x, a.y));
@@ -237,13 +261,13 @@ __device__ __forceinline__ void stage(float2* sm, int log2n, int log_ns, const f
                 if constexpr (R > 4) w[4] = conj_if<kInverse>(__ldg(tw + 4 * t));
                 if constexpr (R > 8) w[8] = conj_if<kInverse>(__ldg(tw + 8 * t));
             }
-            if constexpr (R > 2) w[3] = cmul(w[1], w[2]);
-            if constexpr (R > 4) {
+            if constexpr (R > 2 && !kFull) w[3] = cmul(w[1], w[2]);
+            if constexpr (R > 4 && !kFull) {
                 w[5] = cmul(w[1], w[4]);
                 w[6] = cmul(w[2], w[4]);
                 w[7] = cmul(w[3], w[4]);
             }
-            if constexpr (R > 8) {
+            if constexpr (R > 8 && !kFull) {
 #pragma unroll
                 for (int r = 9; r < R; ++r) w[r] = cmul(w[r - 8], w[8]);
             }
@@ -322,6 +346,28 @@ fft_rows_kernel(const float2* __restrict__ src, const float* __restrict__ image,
     fft_lines<kInverse, 0, kLog>(fsm, tw, log2n, load, store);
 }
 
+// Value X[k] of column x to its place: as is, with the column's half of the fftshift and sign (row
+// p = (-1)^p X[p + n/2]), or as the float image Re(.) * scale.
+template <int kOut>
+__device__ __forceinline__ void col_out(float2* __restrict__ out, float* __restrict__ image, float2* __restrict__ image_c,
+                                        float scale, int n, int h, int mask, int k, int x, float2 z)
+{
+    if (kOut == kFftOutGrid) {
+        out[(size_t)k * n + x] = z;
+        return;
+    }
+    const int p = (k - h) & mask;  // X[k] lands at row p, signed (-1)^p = (-1)^k
+    const float sg = (k & 1) ? -1.f : 1.f;
+    const size_t o = (size_t)p * n + x;
+    if (kOut == kFftOutRotated) {
+        out[o] = make_float2(sg * z.x, sg * z.y);
+    } else {
+        const float v = __fmul_rn(sg * z.x, scale);
+        if (image) image[o] = v;
+        if (image_c) image_c[o] = make_float2(v, 0.f);
+    }
+}
+
 // Column transforms of length n = N1 N2 in two passes (the four-step split, y = N2 y1 + y2,
 // k = k1 + N1 k2), each CTA holding kColW adjacent columns (128-byte row segments):
 //   first:  for one y2, the rows N2 y1 + y2: A[k1] = exp(-+2 pi i y2 k1 / n) * DFT_N1 over y1,
@@ -357,23 +403,23 @@ fft_cols2_kernel(const float2* __restrict__ buf, float2* __restrict__ out, float
     const int x0 = int(blockIdx.x) * kColW, k1 = int(blockIdx.y);
     auto load = [&](int l, int i) -> float2 { return buf[(size_t)(n2 * k1 + i) * n + x0 + l]; };
     auto store = [&](int l, int k2, float2 z) {
-        const int k = k1 + n1 * k2, x = x0 + l;
-        if (kOut == kFftOutGrid) {
-            out[(size_t)k * n + x] = z;
-        } else {
-            const int p = (k - h) & mask;  // X[k] lands at row p, signed (-1)^p = (-1)^k
-            const float sg = (k & 1) ? -1.f : 1.f;
-            const size_t o = (size_t)p * n + x;
-            if (kOut == kFftOutRotated) {
-                out[o] = make_float2(sg * z.x, sg * z.y);
-            } else {
-                const float v = __fmul_rn(sg * z.x, scale);
-                if (image) image[o] = v;
-                if (image_c) image_c[o] = make_float2(v, 0.f);
-            }
-        }
+        col_out<kOut>(out, image, image_c, scale, n, h, mask, k1 + n1 * k2, x0 + l, z);
     };
     fft_lines<kInverse, kColW, kLogL>(fsm, tw, log2n, load, store);
+}
+
+// Whole columns in one pass, kCols adjacent ones per CTA (kCols * n / 16 threads).
+template <bool kInverse, int kOut, int kCols, int kLog>
+__global__ void __launch_bounds__(kCols * (1 << kLog) / 16, 1)
+fft_cols_kernel(const float2* __restrict__ buf, float2* __restrict__ out, float* __restrict__ image,
+                float2* __restrict__ image_c, float scale, const float2* __restrict__ tw)
+{
+    extern __shared__ float2 fsm[];
+    constexpr int n = 1 << kLog, h = n >> 1, mask = n - 1;
+    const int x0 = int(blockIdx.x) * kCols;
+    auto load = [&](int l, int i) -> float2 { return buf[(size_t)i * n + x0 + l]; };
+    auto store = [&](int l, int k, float2 z) { col_out<kOut>(out, image, image_c, scale, n, h, mask, k, x0 + l, z); };
+    fft_lines<kInverse, kCols, kLog>(fsm, tw, kLog, load, store);
 }
 
 struct FftRes {
@@ -425,6 +471,13 @@ tcv_status fft_resources(int n, FftRes* out)
                 h.push_back(h[(t << (2 * part + 1)) & mask]);
             }
     }
+    if (log2n >= kWholeMinLog && log2n <= kWholeLog)
+        for (int log_ns = 4; log_ns < log2n; log_ns += 4) {
+            const int ns = 1 << log_ns, log_r = std::min(4, log2n - log_ns);
+            for (int k = 0; k < ns; ++k)
+                for (int q = 0; q < 16; ++q)
+                    h.push_back(h[(size_t(q * k) << (log2n - log_ns - log_r)) & (size_t(n) - 1)]);
+        }
     FftRes r{dev, n, nullptr, nullptr};
     TCV_CUDA(cudaMalloc(&r.tw, h.size() * sizeof(float2)));
     cudaError_t e = cudaMalloc(&r.scratch, size_t(n) * size_t(n) * sizeof(float2));
@@ -499,15 +552,37 @@ tcv_status launch_cols(bool forward, int out_kind, float2* sc, float2* grid, flo
                    : launch_fft(&fft_cols2_kernel<true, kFftOutGrid, kL2>, g, threads, smem, args, st);
 }
 
+// The column pass of a size whose columns are transformed whole.
+template <int kLog>
+tcv_status launch_whole_cols(bool forward, int out_kind, const float2* sc, float2* grid, float* image_out, float2* image_c,
+                             float scale, const float2* tw, cudaStream_t st)
+{
+    constexpr int n = 1 << kLog, kCols = 8, kThreads = kCols * n / 16;  // 64-byte row segments
+    const size_t smem = size_t(fft_pad(n)) * kCols * sizeof(float2);
+    void* args[] = {&sc, &grid, &image_out, &image_c, &scale, const_cast<const float2**>(&tw)};
+    const dim3 g(unsigned(n / kCols));
+    if (out_kind == kFftOutImage)
+        return forward ? launch_fft(&fft_cols_kernel<false, kFftOutImage, kCols, kLog>, g, kThreads, smem, args, st)
+                       : launch_fft(&fft_cols_kernel<true, kFftOutImage, kCols, kLog>, g, kThreads, smem, args, st);
+    if (out_kind == kFftOutRotated)
+        return forward ? launch_fft(&fft_cols_kernel<false, kFftOutRotated, kCols, kLog>, g, kThreads, smem, args, st)
+                       : launch_fft(&fft_cols_kernel<true, kFftOutRotated, kCols, kLog>, g, kThreads, smem, args, st);
+    return forward ? launch_fft(&fft_cols_kernel<false, kFftOutGrid, kCols, kLog>, g, kThreads, smem, args, st)
+                   : launch_fft(&fft_cols_kernel<true, kFftOutGrid, kCols, kLog>, g, kThreads, smem, args, st);
+}
+
 template <int kLog>
 tcv_status own_passes(float2* grid, const float* image_in, float* image_out, float2* image_c, float scale,
                       bool forward, int in_kind, int out_kind, const FftRes& res, cudaStream_t st)
 {
     TCV_CHECK(launch_rows<kLog>(forward, in_kind, out_kind != kFftOutGrid, grid, image_in, res.scratch, res.tw, st));
-    return launch_cols<kLog>(forward, out_kind, res.scratch, grid, image_out, image_c, scale, res.tw, st);
+    if constexpr (kLog >= kWholeMinLog && kLog <= kWholeLog)
+        return launch_whole_cols<kLog>(forward, out_kind, res.scratch, grid, image_out, image_c, scale, res.tw, st);
+    else
+        return launch_cols<kLog>(forward, out_kind, res.scratch, grid, image_out, image_c, scale, res.tw, st);
 }
 
-// The three passes of the own transform: rows (grid or rotated signed image -> scratch, with the
+// The passes of the own transform: rows (grid or rotated signed image -> scratch, with the
 // row half of the rotation when the output is rotated or an image), columns in place in the
 // scratch, columns from the scratch into the grid (as is, rotated and signed) or the float image.
 tcv_status own_transform(float2* grid, const float* image_in, float* image_out, float2* image_c, float scale, int n,
