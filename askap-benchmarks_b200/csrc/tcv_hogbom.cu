@@ -15,7 +15,8 @@
 //
 // Three forms, chosen by size (tcv_hogbom_deconvolve); all give the same bits.
 //
-// Up to 2048 x 2048 (hog_resident_kernel): the residual stays in registers, one cooperative launch.
+// Up to 2048 x 2048 where the device holds enough clusters (1792 here; hog_resident_kernel): the residual
+// stays in registers, one cooperative launch.
 //
 // Larger images: updates are put off.  The image is cut into blocks of at least 32 x 32 pixels, and
 // a block's updates wait until the block could hold the next peak:
@@ -31,7 +32,7 @@
 // (bounds, the hot blocks' loads, the exchange: 5 us at 4096^2), not a pass over the image.
 // hog_apply_kernel follows on the whole device: it brings blocks near the peak up to date, and
 // every kRing iterations and at the end all blocks (7.7 us an iteration at 4096^2, most of it the PSF
-// windows from L2).  A pixel's updates are applied in iteration order with the reference's
+// windows from L2).  Where many blocks stay hot, hog_pass_kernel takes over.  A pixel's updates are applied in iteration order with the reference's
 // roundings whenever they are applied, so the bits do not depend on the schedule.
 //
 // Beyond the block table's size (or with TCV_HOGBOM_PER_LAUNCH): a launch per iteration, which
@@ -45,7 +46,8 @@
 //
 // Measured on one B200, us an iteration, and in brackets with one pass over the image per iteration
 // (in one cooperative launch up to 48 MiB of images, all CTAs waiting on one counter; a launch
-// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1884^2 6.8 (8.2), 4096^2 12.9 (27.0).
+// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1700^2 7.2 (7.4), 1900^2 6.4 (8.2), 4096^2 12.9 (27.0);
+// put-off updates with 5 sources cleaned to noise 1900^2 8.1 (8.0), 4096^2 21.7 (26.5).
 #include "tcv_internal.cuh"
 
 #include <cooperative_groups.h>
@@ -72,6 +74,11 @@ struct HogState {
     int error;                        // a wait for other CTAs gave up
     int batch, used;                  // put-off updates: the ring's last batch and its PSF windows
     unsigned int nwarm;               // and the blocks of the list for hog_apply_kernel
+    unsigned int visits;              // most hot blocks that a leading CTA had in one launch
+    int pass;                         // 1: hog_pass_kernel has taken over
+    unsigned int meet;                // its CTAs' arrivals in the current launch
+    unsigned int win_next;            // and the winner that its last launch left
+    float val_next;
 };
 
 struct HogArgs {
@@ -683,6 +690,7 @@ struct DeferArgs {
     UpdateSlot* slots;      // [kRing]
     int lb, nbx;            // log2 of the block side; blocks per image side
     int lbp, npx;           // the same of the PSF
+    unsigned int visits_max;  // hog_pass_kernel takes over when a leading CTA had more
 };
 
 // An update's cover of the 32 columns from x0 and `rows` rows from y0: whole (2; they then lie
@@ -838,8 +846,13 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
     LeadShared& sh = *reinterpret_cast<LeadShared*>(lead_smem);
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     HogState* st = a.h.state;
+    cudaGridDependencySynchronize();  // launched ahead of the apply kernel's end
     if (st->stopped) return;  // an earlier launch stopped the loop (the whole cluster returns)
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+    if (st->pass) {
+        if (blockIdx.x == 0 && tid == 0) st->meet = 0;  // for its next launch
+        return;
+    }
     const int W = a.h.width, P = a.h.psf_width, ctas = int(gridDim.x), rank = int(blockIdx.x);
     const int side = 1 << a.lb;
     const LeadDeal deal(a.nbx, ctas);
@@ -875,6 +888,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
     size_t m_pos = 0;
     bool m_open = false;
     unsigned long long skipped = 0;
+    unsigned int visits = 0;
     int it = it0;
     cluster.sync();  // every CTA runs (its shared memory is written to) and has read the state
     for (; it < it1; ++it) {
@@ -936,6 +950,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
         }
         __syncthreads();
         const int nhot = sh.nhot[par];
+        visits += unsigned(nhot);
         lead_apply(a, sh, parts, nhot, base, it + 1);
         __syncthreads();
         if (warp == 0) {
@@ -990,6 +1005,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
         // near the peak: soon to be hot, and better without a long chain of updates to catch up on
         if (sh.applied[i] < it && !(sh.bound[i] < 0.5f * fabsf(peak))) a.warm[atomicAdd(&st->nwarm, 1u)] = unsigned(b);
     }
+    if (tid == 0) atomicMax(&st->visits, visits);
     if (rank != 0) return;
     if (models && m_open) a.h.model[m_pos] = __fadd_rn(m_old, m_add);
     if (rings && skipped) st->skipped_rows += skipped;
@@ -1058,6 +1074,8 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
     __shared__ unsigned short batch_end[kRing];
     __shared__ int warps[2][kApplyThreads / 32];
     __shared__ unsigned long long wk[kApplyThreads / 32];
+    cudaGridDependencySynchronize();  // launched ahead of the leading cluster's end
+    if (a.h.state->pass) return;
     const int to = a.h.state->done;
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int W = a.h.width, P = a.h.psf_width, q1 = to - base, lsub = a.lb - 5;
@@ -1192,6 +1210,87 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
             a.bound[b] = cand_abs(best);
             a.applied[b] = to;
         }
+    }
+}
+
+// Iterations [it0, it1) with a pass over the image each, all CTAs meeting in between, once put-off
+// updates do not pay any more: where the residual is down to noise, the next peak may be in thousands of
+// blocks, and the leading cluster takes most of the time (5 sources cleaned in 1000 iterations: 4096^2 32.8
+// us an iteration, with this kernel 21.7; 2048^2 12.0 and 8.2).  It takes over for good, at the start of a
+// ring (all blocks are up to date then) after a leading CTA had more than visits_max hot blocks in one
+// launch; until then a launch of it ends at once (11 us each, one per ring).  Two candidate buffers
+// suffice: a CTA cannot write iteration it + 1's before every CTA has arrived at barrier it, i.e. has
+// read iteration it - 1's.
+template <bool kVec>
+__global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, int it0, int it1, unsigned long long wait_ns)
+{
+    HogState* st = a.h.state;
+    if (st->stopped || st->error || st->visits <= a.visits_max) return;
+    const unsigned int psf_pos = st->psf_pos;
+    __shared__ int ok;
+    // from the leading cluster, or from this kernel's last launch (set behind a fence)
+    const bool own = *reinterpret_cast<volatile int*>(&st->pass) != 0;
+    unsigned int ppos = own ? __ldcg(&st->win_next) : key_index(__ldcg(&st->win_key[0]));
+    float peak = own ? __ldcg(&st->val_next) : __ldcg(&st->win_val[0]);
+    for (int it = it0; it < it1; ++it) {
+        if (fabsf(peak) < a.h.threshold) {  // every CTA holds the same winner: all stop here
+            if (blockIdx.x == 0 && threadIdx.x == 0) st->stopped = it + 1;
+            break;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            model_update(a.h, it, ppos, peak);
+            st->done = it + 1;
+        }
+        float bv;
+        unsigned long long skipped;
+        unsigned long long best = iter_body<kVec>(a.h, ppos, peak, psf_pos, bv, skipped);
+        if (skipped) atomicAdd(&st->skipped_rows, skipped);
+        best = block_max(best, bv);
+        unsigned long long* keys = a.h.keys + (it & 1) * a.h.nblocks;
+        float* vals = a.h.vals + (it & 1) * a.h.nblocks;
+        if (threadIdx.x == 0) {
+            keys[blockIdx.x] = best;
+            vals[blockIdx.x] = bv;
+            __threadfence();
+            atomicAdd(&st->meet, 1u);
+            const unsigned int target = unsigned(it - it0 + 1) * unsigned(a.h.nblocks);
+            ok = 0;
+            const unsigned long long t0 = global_ns();
+            for (unsigned int spin = 0; spin < (1u << 24); ++spin) {
+                if (*reinterpret_cast<volatile unsigned int*>(&st->meet) >= target) {
+                    ok = 1;
+                    break;
+                }
+                if (*reinterpret_cast<volatile int*>(&st->error)) break;
+                __nanosleep(32);
+                if ((spin & 63u) == 63u && global_ns() - t0 >= wait_ns) break;
+            }
+            if (!ok) st->error = 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!ok) return;
+        unsigned long long k = 0;
+        float v = 0.f;
+        for (int i = threadIdx.x; i < a.h.nblocks; i += kHogThreads) {
+            const unsigned long long ki = __ldcg(keys + i);
+            if (ki > k) {
+                k = ki;
+                v = __ldcg(vals + i);
+            }
+        }
+        k = block_max(k, v);
+        const bool zero = (k >> 32) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
+        ppos = zero ? 0u : key_index(k);
+        peak = zero ? 0.f : v;
+    }
+    // for the next launch.  A CTA that starts only now (all stopped at once) reads the winner it would
+    // have read before.
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->win_next = ppos;
+        st->val_next = peak;
+        __threadfence();
+        st->pass = 1;
     }
 }
 
@@ -1371,6 +1470,12 @@ int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArg
     return 0;
 }
 
+// Hot blocks of a leading CTA in one launch from which a pass over the image per iteration is faster.
+// With 5 and with 60 sources (us an iteration by the blocks per iteration at which the passes take over;
+// 10^6: never): 2048^2 12 8.3, 6 8.3, 0 9.0, 10^6 13.5 and 12 9.5, 6 8.95, 0 9.2, 10^6 9.5; 4096^2 12 21.7,
+// 6 21.7, 0 27.1, 10^6 36.4 and 12 19.9, 6 27.6, 0 29.5, 10^6 19.9.
+unsigned int visits_limit(long long n) { return unsigned(kLeadIters * (4 + (n >> 21))); }
+
 // All iterations with put-off updates.  false: the device cannot hold the cluster, nothing launched.
 tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* dirty, int niters, cudaStream_t st, bool& ran)
 {
@@ -1407,12 +1512,40 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_apply_kernel, kApplyThreads, win));
     const int most = std::min(nb, sms * std::max(1, per_sm));
+    // the one-pass kernel that may take over: two CTAs per SM at most, as many as are resident
+    const bool vec = h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0;
+    const void* pass = vec ? reinterpret_cast<const void*>(hog_pass_kernel<true>)
+                           : reinterpret_cast<const void*>(hog_pass_kernel<false>);
+    int coop = 0;
+    TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass, kHogThreads, 0));
+    const bool passes = coop && per_sm > 0;
+    a.visits_max = passes ? visits_limit(h.n) : 0xffffffffu;
+    DeferArgs ap = a;
+    ap.h.nblocks = std::max(1, std::min({sms * std::min(per_sm, 2), kHogMaxBlocks / 2, hog_blocks(h.n), h.width}));
+    unsigned long long wait_ns = kDefaultWaitNs;
+    cudaLaunchAttribute attrs[2] = {attr, {}};
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cudaLaunchConfig_t apply{};
+    apply.gridDim = dim3(unsigned(most));
+    apply.blockDim = dim3(kApplyThreads);
+    apply.dynamicSmemBytes = win;
+    apply.stream = st;
+    apply.attrs = attrs + 1;
+    apply.numAttrs = 1;
     for (int it = 0, base = 0; it < niters; it += kLeadIters) {
         const int to = std::min(niters, it + kLeadIters);
+        if (passes && it == base && it > 0) {  // all blocks are up to date
+            int from = it, end = std::min(niters, it + kRing);
+            void* args[] = {&ap, &from, &end, &wait_ns};
+            TCV_CUDA(cudaLaunchCooperativeKernel(pass, dim3(unsigned(ap.h.nblocks)), dim3(kHogThreads), args, 0, st));
+        }
+        cfg.numAttrs = it > base ? 2 : 1;  // behind the apply kernel
         TCV_CUDA(cudaLaunchKernelEx(&cfg, hog_lead_kernel, a, it, to, base));
         const int all = to == niters || to - base == kRing;
-        hog_apply_kernel<<<most, kApplyThreads, win, st>>>(a, base, all);
-        TCV_CUDA(cudaGetLastError());
+        TCV_CUDA(cudaLaunchKernelEx(&apply, hog_apply_kernel, a, base, all));
         if (all) base = to;
     }
     ran = true;

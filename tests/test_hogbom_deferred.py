@@ -77,3 +77,15 @@ def test_images(tcv, orc, cuda_ok, kind):
     elif kind == "tiny":  # subnormal values and products
         dirty, psf = (dirty * np.float32(1e-39)).astype(np.float32), psf
     _check(orc, dirty, psf, n)
+
+
+@pytest.mark.parametrize("width,psf,niters,threshold", [
+    (2100, 2100, 260, 0.0),   # noise: many blocks stay hot, passes take over at iteration 128, mid-ring end
+    (2099, 1050, 257, 0.0),   # a ragged width, one iteration in the last ring
+    (2100, 2101, 400, 4.16),  # the threshold stops a launch of passes
+])
+def test_passes_take_over(tcv, orc, cuda_ok, width, psf, niters, threshold):
+    from tconvolve.workload import synthetic_psf
+
+    dirty = np.random.default_rng(width + psf).standard_normal((width, width)).astype(np.float32)
+    _check(orc, dirty, synthetic_psf(psf), niters, threshold)
