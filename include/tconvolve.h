@@ -586,9 +586,9 @@ tcv_status tcv_hogbom_deconvolve(const float *d_dirty, int width, const float *d
  * iterations with the residual in registers (the CTAs meet once per iteration, with bounded waits)
  * and larger ones with updates put off until a block of pixels could hold the next peak (a launch
  * of one cluster and a device-wide one per 16 iterations, and cooperative launches of 128 once too
- * many blocks could; images or PSFs over 16384 wide take one launch per iteration).  PERSISTENT takes the
- * cooperative form where the image fits it, PER_LAUNCH one launch per iteration; both otherwise
- * the latter.  Results are identical. */
+ * many blocks could; images or PSFs over 16384 wide take one launch per iteration).  PERSISTENT
+ * takes the cooperative form where the image fits it, PER_LAUNCH one launch per iteration; both
+ * otherwise the latter.  Results are identical. */
 enum { TCV_HOGBOM_AUTO = 0, TCV_HOGBOM_PER_LAUNCH = 1, TCV_HOGBOM_PERSISTENT = 2 };
 void tcv_hogbom_set_strategy(int strategy);
 /* The bounded waits of the cooperative form (process-wide, for launches made after the call):
