@@ -74,7 +74,7 @@ struct HogState {
     int error;                        // a wait for other CTAs gave up
     int batch, used;                  // put-off updates: the ring's last batch and its PSF windows
     unsigned int nwarm;               // and the blocks of the list for hog_apply_kernel
-    unsigned int visits;              // most hot blocks that a leading CTA had in one launch
+    unsigned int visits;              // most hot blocks that a leading CTA had in the last launch
     int pass;                         // 1: hog_pass_kernel has taken over
     unsigned int meet;                // its CTAs' arrivals in the current launch
     unsigned int win_next;            // and the winner that its last launch left
@@ -690,7 +690,7 @@ struct DeferArgs {
     UpdateSlot* slots;      // [kRing]
     int lb, nbx;            // log2 of the block side; blocks per image side
     int lbp, npx;           // the same of the PSF
-    unsigned int visits_max;  // hog_pass_kernel takes over when a leading CTA had more
+    unsigned int visits_max;  // hog_pass_kernel takes over when a leading CTA had more in the ring's last launch
 };
 
 // An update's cover of the 32 columns from x0 and `rows` rows from y0: whole (2; they then lie
@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
     }
     for (int i = tid; i < it0 - base; i += kLeadThreads) sh.ring[i] = a.ring[i];
     for (int i = tid; i < a.npx * a.npx; i += kLeadThreads) pmax[i] = a.pmax[i];
-    if (rank == 0 && tid == 0) st->nwarm = 0;
+    if (rank == 0 && tid == 0) st->nwarm = st->visits = 0;
     if (tid == 0) {
         sh.nhot[0] = sh.nhot[1] = 0;
         for (int p = 0; p < 2; ++p)
@@ -1217,8 +1217,8 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
 // updates do not pay any more: where the residual is down to noise, the next peak may be in thousands of
 // blocks, and the leading cluster takes most of the time (5 sources cleaned in 1000 iterations: 4096^2 32.8
 // us an iteration, with this kernel 21.7; 2048^2 12.0 and 8.2).  It takes over for good, at the start of a
-// ring (all blocks are up to date then) after a leading CTA had more than visits_max hot blocks in one
-// launch; until then a launch of it ends at once (11 us each, one per ring).  Two candidate buffers
+// ring (all blocks are up to date then) when a leading CTA had more than visits_max hot blocks in the
+// last launch; until then a launch of it ends at once (11 us each, one per ring).  Two candidate buffers
 // suffice: a CTA cannot write iteration it + 1's before every CTA has arrived at barrier it, i.e. has
 // read iteration it - 1's.
 template <bool kVec>
@@ -1470,11 +1470,12 @@ int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArg
     return 0;
 }
 
-// Hot blocks of a leading CTA in one launch from which a pass over the image per iteration is faster.
-// With 5 and with 60 sources (us an iteration by the blocks per iteration at which the passes take over;
-// 10^6: never): 2048^2 12 8.3, 6 8.3, 0 9.0, 10^6 13.5 and 12 9.5, 6 8.95, 0 9.2, 10^6 9.5; 4096^2 12 21.7,
-// 6 21.7, 0 27.1, 10^6 36.4 and 12 19.9, 6 27.6, 0 29.5, 10^6 19.9.
-unsigned int visits_limit(long long n) { return unsigned(kLeadIters * (4 + (n >> 21))); }
+// Hot blocks of a leading CTA in one launch from which a pass over the image per iteration is faster: 6
+// an iteration at 2048^2, 18 at 4096^2.  us an iteration of 1000 by the blocks at which the passes take over
+// (0: never): 2048^2, 5 sources 0 13.0, 12 8.24, 6 8.22; 60 sources 0 9.07, 12 9.05, 6 8.30, 4 8.42; 40 sources,
+// 300 iterations 0 7.36, 6 7.40, 4 8.0.  2600^2, 20 sources 0 9.03, 8 9.02, 6 11.5.  4096^2, 5 sources 0 35.9,
+// 24 21.9, 12 21.9; 60 sources 0 19.5, 24 19.5, 12 21.4, 8 27.5.
+unsigned int visits_limit(long long n) { return unsigned(kLeadIters * (2 + (n >> 20))); }
 
 // All iterations with put-off updates.  false: the device cannot hold the cluster, nothing launched.
 tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* dirty, int niters, cudaStream_t st, bool& ran)
