@@ -248,13 +248,15 @@ __device__ unsigned walk_parts(WalkShared& sh, Inc2 inc, bool stop, unsigned m, 
     return first;
 }
 
-// The entries [lo, hi) added to sh.s.
+// The entries [lo, hi) added to sh.s.  A sum that is not a number (entries of a table set up with a
+// negative baseline are not) stays so, as it does added in order: it has no place in a binade.
 __device__ void walk_entries(WalkShared& sh, const float2* __restrict__ c, int64_t lo, int64_t hi)
 {
     constexpr int kPer = 4;
     while (lo < hi) {
         __syncthreads();
         const float s = sh.s;
+        if (s != s) break;  // the same for the whole CTA
         const int64_t at = lo + int64_t(threadIdx.x) * kPer;
         float x[kPer];
 #pragma unroll
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(kWalkThreads) sum_walk_kernel(const float2* __
     int k = 1;
     while (k < b.nb) {
         const float s = sh.s;
+        if (s != s) break;
         const int mine = k + int(threadIdx.x);
         unsigned first = 0, m0 = 0;
         if (s >= kSumTiny) {
