@@ -46,6 +46,7 @@ struct PlanGeom {
     int rows, tw, th;
     int split;          // samples per gridding work unit of a split cell (0: cells are never split)
     int dsplit;         // the same for degridding
+    bool own_units;     // dsplit is the plan's own choice (no tuning): it gives way to a small workspace
     bool dense;         // sample-parallel gridding kernel (tcv_dense.cu; 64 x 32 tiles)
     bool ddense;        // sample-parallel degridding kernel
     int ntx, nty;       // tiles per row / column of a one-job plan

@@ -1010,6 +1010,8 @@ tcv_status build(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_
     return TCV_OK;
 }
 
+constexpr int kMostUnit = 128;  // samples of a degridding unit that a plan chooses itself, at most
+
 bool valid_tuning(const tcv_tuning* t)
 {
     if (!t) return true;
@@ -1019,14 +1021,25 @@ bool valid_tuning(const tcv_tuning* t)
            t->degrid_split >= 0 && t->degrid_split <= (1 << 24);
 }
 
+// Larger degridding units, or cells whole, for a plan that chose its units itself and does not fit its
+// workspace: fewer samples take smaller units, so that a workspace made for the most samples, or for
+// whole cells (the tuned entry with the defaults), can be too small for fewer.  A unit's size changes no
+// result.  false: nothing is left to give up.
+bool larger_units(PlanGeom& g)
+{
+    if (!g.own_units || !g.dsplit) return false;
+    g.dsplit = g.dsplit < kMostUnit ? 2 * g.dsplit : 0;
+    return true;
+}
+
 // Lay the plan's arrays out in d_work and write the job table: from host memory for a batch,
 // by a one-thread kernel for a one-job plan (so that plan_init is device work only).
 tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_t st)
 {
     const PlanGeom& g = p->g;
     size_t cb = 0;
-    const size_t need = plan_bytes(g, &cb);
-    if (work_bytes < need) return TCV_ERR_WORKSPACE;
+    while (plan_bytes(g, &cb) > work_bytes)
+        if (!larger_units(p->g)) return TCV_ERR_WORKSPACE;
     const size_t ks = g.key64 ? 8 : 4;
     const size_t np = size_t(g.n) * g.max_tiles;
     const size_t an = g.anchors ? size_t(g.n) : 0;
@@ -1243,7 +1256,8 @@ void default_units(PlanGeom& g)
     const double reach = (double(g.s + g.tw - 1) / g.tw) * (double(g.s + g.th - 1) / g.th);
     const double pairs = double(g.n) * reach;  // mean tiles of a footprint
     const bool small = plan_bytes(g, nullptr) <= kUnitsBytes;
-    for (g.dsplit = 32; g.dsplit < 128 && g.dsplit * 4736.0 < pairs;) g.dsplit *= 2;
+    g.own_units = true;
+    for (g.dsplit = 32; g.dsplit < kMostUnit && g.dsplit * 4736.0 < pairs;) g.dsplit *= 2;
     if (small && plan_bytes(g, nullptr) > kUnitsBytes) g.dsplit = 0;
 }
 

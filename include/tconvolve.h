@@ -142,7 +142,8 @@ tcv_status tcv_plan_build(tcv_plan **plan_out, const int32_t *d_iu, const int32_
                           int64_t c_len, void *d_work, size_t work_bytes, void *stream);
 /* Such a plan (no tuning) has 16 tile rows and 32 MiB plane groups, grids cells whole, and cuts cells
  * of many samples into degridding work units as its sample count and footprint suggest
- * (tcv_plan_tuning reports them). */
+ * (tcv_plan_tuning reports them).  In a workspace too small for those it takes larger units, down to
+ * whole cells: one made for the most samples, or for the tuned entry's defaults, serves fewer too. */
 /* grid += gridding of d_data (n complex64) with table d_c of type c_type (Benchmark.cc:125-155).
  * d_grid is NULL for a batched plan (each job's own grid). */
 tcv_status tcv_plan_grid(const tcv_plan *plan, const float *d_data, const void *d_c, int c_type,
