@@ -421,26 +421,38 @@ struct ConvSlot {
 
 __global__ void conv_clear_kernel(int slot) { g_conv[slot] = ConvCount{0ull, 0u, 0u}; }
 
-__global__ void absmax_kernel(const float2* c, int64_t n, int slot)
+// The FP16 forms are scaled by the largest |value|, so they need a pass before the conversion: it counts
+// the imaginary parts as well, and the conversion is left running when the call returns (35 M entries to
+// rf16: 181 us; 231 with the count in the conversion, which the call then has to wait for).
+__global__ void absmax_imag_kernel(const float2* c, int64_t n, int slot)
 {
     float m = 0.f;
+    unsigned long long nz = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 z = c[i];
         m = fmaxf(m, fmaxf(fabsf(z.x), fabsf(z.y)));
+        nz += (z.y != 0.f);
     }
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&g_conv[slot].absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
+    for (int o = 16; o; o >>= 1) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        nz += __shfl_xor_sync(0xffffffffu, nz, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&g_conv[slot].absmax_bits, __float_as_uint(m));  // non-negative floats order like their bits
+        if (nz) atomicAdd(&g_conv[slot].imag_nonzero, nz);
+    }
 }
 
-// One entry per thread and step; counts the entries with an imaginary part as it goes (for the
-// forms without a scale this is the only pass over the table: 35 M entries to r32 in 175 us with a
+// One entry per thread and step; kCount: counts the entries with an imaginary part as it goes (for
+// the forms without a scale this is the only pass over the table: 35 M entries to r32 in 175 us with a
 // counting pass before it, 107 us in one).
+template <bool kCount>
 __global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre_scale, void* out, int slot)
 {
     unsigned long long nz = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 z = c[i];
-        nz += (z.y != 0.f);
+        if (kCount) nz += (z.y != 0.f);
         switch (c_type) {
             case TCV_C_R32: static_cast<float*>(out)[i] = z.x; break;
             case TCV_C_CBF16: {
@@ -457,8 +469,10 @@ __global__ void convert_kernel(const float2* c, int64_t n, int c_type, float pre
             default: break;
         }
     }
-    for (int o = 16; o; o >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, o);
-    if ((threadIdx.x & 31) == 0 && nz) atomicAdd(&g_conv[slot].imag_nonzero, nz);
+    if (kCount) {
+        for (int o = 16; o; o >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, o);
+        if ((threadIdx.x & 31) == 0 && nz) atomicAdd(&g_conv[slot].imag_nonzero, nz);
+    }
 }
 
 inline int grid_blocks(int64_t n, int threads)
@@ -577,10 +591,11 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
     };
     ConvCount h{};
     float pre = 1.0f, post = 1.0f;
-    if (e == cudaSuccess && (c_type == TCV_C_CF16 || c_type == TCV_C_RF16)) {
+    const bool scaled = c_type == TCV_C_CF16 || c_type == TCV_C_RF16;
+    if (e == cudaSuccess && scaled) {
         // power-of-two scale putting max |C| in [2^14, 2^15): the table keeps FP16's full
         // precision without approaching its 65504 limit; kernels undo it exactly with c_scale.
-        absmax_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, slot.i);
+        absmax_imag_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, slot.i);
         e = cudaGetLastError();
         read_back(h);
         const float amax = __builtin_bit_cast(float, h.absmax_bits);
@@ -593,10 +608,14 @@ tcv_status tcv_convert_c(const float* d_c64, int64_t c_len, int c_type, void* d_
         }
     }
     if (e == cudaSuccess) {
-        convert_kernel<<<grid_blocks(c_len, 256), 256, 0, s>>>(c, c_len, c_type, pre, d_out, slot.i);
+        const int blocks = grid_blocks(c_len, 256);
+        if (scaled)
+            convert_kernel<false><<<blocks, 256, 0, s>>>(c, c_len, c_type, pre, d_out, slot.i);
+        else
+            convert_kernel<true><<<blocks, 256, 0, s>>>(c, c_len, c_type, pre, d_out, slot.i);
         e = cudaGetLastError();
     }
-    read_back(h);
+    if (!scaled || e != cudaSuccess) read_back(h);
     TCV_CUDA(e);
     if (c_scale_out) *c_scale_out = post;
     if (imag_nonzero_out) *imag_nonzero_out = int64_t(h.imag_nonzero);

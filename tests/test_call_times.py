@@ -1,0 +1,44 @@
+"""Calls whose time is held against another form of the same work, measured side by side on the device.
+
+Each bar is the ratio that the two forms' passes over memory or launches give, with a margin for noise;
+medians of several runs of both in turn.
+"""
+from __future__ import annotations
+
+import statistics
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _us(f, g, reps=9):
+    """Median device times of f and g, run in turn."""
+    import torch
+
+    def once(h):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        torch.cuda.synchronize()
+        a.record()
+        h()
+        b.record()
+        b.synchronize()
+        return 1000 * a.elapsed_time(b)
+
+    for h in (f, g, f, g):
+        once(h)
+    t = [(once(f), once(g)) for _ in range(reps)]
+    return tuple(statistics.median(x) for x in zip(*t))
+
+
+def test_scaled_conversion_is_two_passes(tcv, cuda_ok):
+    """An FP16 table takes a pass for its scale and the conversion: 8 + 8 + 2 bytes an entry where a float
+    table takes 8 + 4, so 1.5 times the time, less what both have in common.  Bar: 1.5."""
+    import torch
+
+    from tconvolve import _lib, raw
+
+    c = torch.zeros(33 * 64 * 129 * 129, dtype=torch.complex64, device="cuda")
+    c.real.uniform_(-1.0, 1.0)
+    two, one = _us(lambda: raw.convert_c(c, _lib.CTYPE_BY_NAME["rf16"]), lambda: raw.convert_c(c, _lib.CTYPE_BY_NAME["r32"]))
+    assert two <= 1.5 * one, (two, one)
