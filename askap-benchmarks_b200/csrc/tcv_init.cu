@@ -40,7 +40,6 @@ __global__ void uvw_kernel(int64_t n, int baseline, uint64_t state0, double* u, 
 struct CParams {
     int s, os, w_size, c_center;
     double w_cell_size, freq0, cell_size;
-    int64_t n;
 };
 
 // Benchmark.cc:236-258 in FP64, stored as float (imaginary part 0).  One thread per entry of the
@@ -307,7 +306,7 @@ __global__ void __launch_bounds__(kWalkThreads) sum_walk_kernel(const float2* __
     if (threadIdx.x == 0) {
         float s = 0.f;
 #pragma unroll 8
-        for (int i = 0; i < kSumChunk / 4; ++i) {  // (the places past the table add 0)
+        for (int i = 0; i < (int(nh) + 3) / 4; ++i) {  // (the places past the table add 0)
             const float4 v = reinterpret_cast<const float4*>(head)[i];
             s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
         }
@@ -521,7 +520,7 @@ tcv_status tcv_init_c_raw(double freq0, double cell_size, int baseline, int w_si
     if (st != TCV_OK) return st;
     if (n > INT_MAX) return TCV_ERR_UNSUPPORTED;  // cOffset is a 32-bit int in the reference
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    CParams p{2 * support + 1, os, w_size, support, wcs, freq0, cell_size, n};
+    CParams p{2 * support + 1, os, w_size, support, wcs, freq0, cell_size};
     const int64_t half = n / w_size * (w_size / 2 + 1);  // entries of the planes w >= 0
     init_c_kernel<<<unsigned((half + 255) / 256), 256, 0, s>>>(p, reinterpret_cast<float2*>(d_c));
     TCV_CUDA(cudaGetLastError());
@@ -535,10 +534,12 @@ tcv_status tcv_init_c_raw(double freq0, double cell_size, int baseline, int w_si
     sb.incs = reinterpret_cast<Inc2*>(sb.sum + kSumMaxBlocks);
     sb.exps = reinterpret_cast<int*>(sb.incs + 2 * kSumMaxBlocks);
     const float2* table = reinterpret_cast<const float2*>(d_c);
-    sum_blocks_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
-    TCV_CUDA(cudaGetLastError());
-    sum_incs_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
-    TCV_CUDA(cudaGetLastError());
+    if (sb.nb > 1) {  // the walk takes the first block entry by entry
+        sum_blocks_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
+        TCV_CUDA(cudaGetLastError());
+        sum_incs_kernel<<<unsigned(sb.nb), 256, 0, s>>>(table, sb);
+        TCV_CUDA(cudaGetLastError());
+    }
     sum_walk_kernel<<<1, kWalkThreads, 0, s>>>(table, sb, d_sum);
     TCV_CUDA(cudaGetLastError());
     scale_c_kernel<<<grid_blocks(n, 256), 256, 0, s>>>(reinterpret_cast<float2*>(d_c), n,
