@@ -400,7 +400,7 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
 // ------------------------------------------------------------------------------------------
 constexpr int kResThreads = 512;
 constexpr int kResChunks = 4;       // columns per thread, at most: widths up to 2048
-constexpr int kResClusters = 32;    // clusters of a launch, at most
+constexpr int kResClusters = 31;    // clusters of a launch, at most: a lane each, and one for a withheld one
 
 struct ResArgs {
     HogArgs h;
@@ -691,6 +691,8 @@ struct DeferArgs {
     int lb, nbx;            // log2 of the block side; blocks per image side
     int lbp, npx;           // the same of the PSF
     unsigned int visits_max;  // hog_pass_kernel takes over when a leading CTA had more in the ring's last launch
+    unsigned long long wait_ns;  // limit of a wait
+    unsigned int withheld;       // candidates or arrivals more than are made (tcv_hogbom_set_wait)
 };
 
 // An update's cover of the 32 columns from x0 and `rows` rows from y0: whole (2; they then lie
@@ -847,7 +849,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     HogState* st = a.h.state;
     cudaGridDependencySynchronize();  // launched ahead of the apply kernel's end
-    if (st->stopped) return;  // an earlier launch stopped the loop (the whole cluster returns)
+    if (st->stopped || st->error) return;  // an earlier launch stopped the loop (the whole cluster returns)
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     if (st->pass) {
         if (blockIdx.x == 0 && tid == 0) st->meet = 0;  // for its next launch
@@ -902,8 +904,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
         const float least = fabsf(__fsub_rn(peak, __fmul_rn(t, at_peak)));  // the peak's pixel after the update
         if (tid == 0) {
             sh.nhot[par ^ 1] = 0;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&sh.arrived[par])),
-                         "r"(ctas * 8) : "memory");
+            expect_bytes(&sh.arrived[par], (ctas + int(a.withheld)) * 8);
         }
         if (rings) {
             const int startx = max(0, diffx), stopx = min(W - 1, rx + (P - px - 1));
@@ -968,24 +969,11 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
             // to every CTA of the cluster, each store counted by that CTA's barrier.  Two buffers
             // suffice: a CTA sends iteration it + 2's after it has all of it + 1's, which the
             // others sent having read it's.
-            if (lane < ctas) {
-                unsigned dst, bar;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_addr(&sh.cand[par][rank])), "r"(lane));
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_addr(&sh.arrived[par])), "r"(lane));
-                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(dst), "l"(c),
-                             "r"(bar) : "memory");
-            }
+            if (lane < ctas) send_key(&sh.cand[par][rank], &sh.arrived[par], lane, c);
         }
         // this parity's barrier completes once per two iterations of this launch
         const unsigned phase = unsigned((it - it0) >> 1) & 1u;
-        bool here = false;
-        for (unsigned spin = 0; spin < (1u << 22) && !here; ++spin) {
-            unsigned ok;
-            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                         " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(smem_addr(&sh.arrived[par])), "r"(phase) : "memory");
-            here = ok != 0;
-        }
-        if (!__syncthreads_and(here)) {  // not while the cluster's CTAs run: leave (tcv_hogbom_result says so)
+        if (!__syncthreads_and(wait_phase(&sh.arrived[par], phase, a.wait_ns))) {  // leave (tcv_hogbom_result says so)
             st->error = 1;
             break;
         }
@@ -1075,7 +1063,8 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
     __shared__ int warps[2][kApplyThreads / 32];
     __shared__ unsigned long long wk[kApplyThreads / 32];
     cudaGridDependencySynchronize();  // launched ahead of the leading cluster's end
-    if (a.h.state->pass) return;
+    // after a wait that ran out the iteration's windows are not laid out, nor is anything kept
+    if (a.h.state->pass || a.h.state->error) return;
     const int to = a.h.state->done;
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
     const int W = a.h.width, P = a.h.psf_width, q1 = to - base, lsub = a.lb - 5;
@@ -1222,7 +1211,7 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
 // suffice: a CTA cannot write iteration it + 1's before every CTA has arrived at barrier it, i.e. has
 // read iteration it - 1's.
 template <bool kVec>
-__global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, int it0, int it1, unsigned long long wait_ns)
+__global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, int it0, int it1)
 {
     HogState* st = a.h.state;
     if (st->stopped || st->error || st->visits <= a.visits_max) return;
@@ -1253,7 +1242,7 @@ __global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, i
             vals[blockIdx.x] = bv;
             __threadfence();
             atomicAdd(&st->meet, 1u);
-            const unsigned int target = unsigned(it - it0 + 1) * unsigned(a.h.nblocks);
+            const unsigned int target = unsigned(it - it0 + 1) * unsigned(a.h.nblocks) + a.withheld;
             ok = 0;
             const unsigned long long t0 = global_ns();
             for (unsigned int spin = 0; spin < (1u << 24); ++spin) {
@@ -1263,7 +1252,7 @@ __global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, i
                 }
                 if (*reinterpret_cast<volatile int*>(&st->error)) break;
                 __nanosleep(32);
-                if ((spin & 63u) == 63u && global_ns() - t0 >= wait_ns) break;
+                if ((spin & 63u) == 63u && global_ns() - t0 >= a.wait_ns) break;
             }
             if (!ok) st->error = 1;
             __threadfence();
@@ -1491,6 +1480,8 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     a.pmax = w.pmax;
     a.ring = w.ring;
     a.slots = w.slots;
+    a.wait_ns = g_wait_ns;
+    a.withheld = g_withheld;
     a.lb = log2_side(h.width);
     a.nbx = (h.width + (1 << a.lb) - 1) >> a.lb;
     a.lbp = std::max(a.lb, log2_side(h.psf_width));  // a block then lies on at most 2 x 2 of the PSF's
@@ -1524,7 +1515,6 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     a.visits_max = passes ? visits_limit(h.n) : 0xffffffffu;
     DeferArgs ap = a;
     ap.h.nblocks = std::max(1, std::min({sms * std::min(per_sm, 2), kHogMaxBlocks / 2, hog_blocks(h.n), h.width}));
-    unsigned long long wait_ns = kDefaultWaitNs;
     cudaLaunchAttribute attrs[2] = {attr, {}};
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1540,7 +1530,7 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
         const int to = std::min(niters, it + kLeadIters);
         if (passes && it == base && it > 0) {  // all blocks are up to date
             int from = it, end = std::min(niters, it + kRing);
-            void* args[] = {&ap, &from, &end, &wait_ns};
+            void* args[] = {&ap, &from, &end};
             TCV_CUDA(cudaLaunchCooperativeKernel(pass, dim3(unsigned(ap.h.nblocks)), dim3(kHogThreads), args, 0, st));
         }
         cfg.numAttrs = it > base ? 2 : 1;  // behind the apply kernel

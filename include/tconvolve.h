@@ -592,16 +592,17 @@ tcv_status tcv_hogbom_deconvolve(const float *d_dirty, int width, const float *d
  * otherwise the latter.  Results are identical. */
 enum { TCV_HOGBOM_AUTO = 0, TCV_HOGBOM_PER_LAUNCH = 1, TCV_HOGBOM_PERSISTENT = 2 };
 void tcv_hogbom_set_strategy(int strategy);
-/* The bounded waits of the cooperative form (process-wide, for launches made after the call):
- * limit_ns caps one wait (default and maximum 2e9 ns); withheld_arrivals (default 0) makes the
- * CTAs wait for that many more candidates than are ever posted, so that every wait runs out: a host-side hook that exercises the timeout path (the loop stops, every CTA returns,
- * tcv_hogbom_result reports TCV_ERR_TIMEOUT) without faulting or hanging the GPU.  Restore (2e9, 0)
- * afterwards.  The device-side counterpart of the reference's error accounting, which counts
+/* The bounded waits of the forms whose CTAs wait for one another (process-wide, for launches made after
+ * the call): limit_ns caps one wait (default and maximum 2e9 ns); withheld_arrivals (default 0) makes
+ * the CTAs wait for that many more candidates or arrivals than are ever made, so that every wait runs
+ * out: a host-side hook that exercises the timeout path (the loop stops, every CTA and every later launch
+ * returns, tcv_hogbom_result reports TCV_ERR_TIMEOUT) without faulting or hanging the GPU.  Restore
+ * (2e9, 0) afterwards.  The device-side counterpart of the reference's error accounting, which counts
  * disagreeing values instead of failing (attic/tConvolveBurnIn/tConvolveBurnIn.cc:94-107). */
 tcv_status tcv_hogbom_set_wait(uint64_t limit_ns, uint32_t withheld_arrivals);
 /* After tcv_hogbom_deconvolve (synchronises): iterations done, the iteration that met the
  * threshold (-1 if none), PSF rows skipped, the PSF peak index.  Any output may be NULL.
- * TCV_ERR_TIMEOUT if a wait of the cooperative form gave up (the loop stopped). */
+ * TCV_ERR_TIMEOUT if a wait for other CTAs gave up (the loop stopped; the images are then not valid). */
 tcv_status tcv_hogbom_result(const void *d_work, int *iters_done, int *stopped_at,
                              int64_t *skipped_rows, int64_t *psf_peak_pos, void *stream);
 /* findPeak (HogbomGolden.cc:127-139): the value of largest magnitude and its first index
