@@ -76,9 +76,11 @@ struct HogState {
     unsigned int nwarm;               // and the blocks of the list for hog_apply_kernel
     unsigned int visits;              // most hot blocks that a leading CTA had in the last launch
     int pass;                         // 1: hog_pass_kernel has taken over
+    int pass_end;                     // iterations that it has done
     unsigned int meet;                // its CTAs' arrivals in the current launch
     unsigned int win_next;            // and the winner that its last launch left
     float val_next;
+    unsigned int near, tops;          // blocks of the dirty image that reach half its peak; its second peak's limit
 };
 
 struct HogArgs {
@@ -680,6 +682,12 @@ struct UpdateSlot {
     short prev, slot, batch, pad;  // batch: ring index its batch starts at
 };
 
+// Where passes over the image take over from put-off updates (hog_pass_kernel): with more blocks than these
+struct PassLimits {
+    unsigned int near, tops;    // at the start: near half the peak; above the second peak's limit
+    unsigned int warm, visits;  // later: of the last launch's list for hog_apply_kernel; hot in a leading CTA
+};
+
 struct DeferArgs {
     HogArgs h;
     float* bound;           // per image block: limit of its |residual| as of the last update
@@ -690,7 +698,6 @@ struct DeferArgs {
     UpdateSlot* slots;      // [kRing]
     int lb, nbx;            // log2 of the block side; blocks per image side
     int lbp, npx;           // the same of the PSF
-    unsigned int visits_max;  // hog_pass_kernel takes over when a leading CTA had more in the ring's last launch
     unsigned long long wait_ns;  // limit of a wait
     unsigned int withheld;       // candidates or arrivals more than are made (tcv_hogbom_set_wait)
 };
@@ -704,53 +711,119 @@ __device__ __forceinline__ int cover_of(const Update& u, int x0, int y0, int row
     return xa > x0 + 31 || xb < x0 || ya > y0 + rows - 1 || yb < y0 ? 0 : 1;
 }
 
-// An image's blocks: their largest |value| (one warp per block) and the image's own peak; copies the
-// image when copy_to is given.
-__global__ void __launch_bounds__(kHogThreads) hog_blocks_kernel(const float* __restrict__ img, float* __restrict__ copy_to,
-                                                                 int W, int lb, int nbx, float* top, int* applied,
-                                                                 unsigned long long* keys, float* vals, HogState* st,
-                                                                 int slot)
+// Block b of an image by one warp: its largest |value| into top[b], the key returned; copies the
+// block when copy_to is given.
+__device__ __forceinline__ unsigned long long scan_block(const float* __restrict__ img, float* __restrict__ copy_to, int W,
+                                                         int lb, int nbx, int b, float* top)
 {
-    const int lane = threadIdx.x & 31, nb = nbx * nbx;
-    const int warps = int(gridDim.x) * (kHogThreads / 32);
-    unsigned long long best = 0;
-    for (int b = int(blockIdx.x) * (kHogThreads / 32) + (threadIdx.x >> 5); b < nb; b += warps) {
-        const int x0 = (b % nbx) << lb, y0 = (b / nbx) << lb, side = 1 << lb;
-        const int ye = min(W, y0 + side);
-        unsigned long long k = 0;
-        for (int x = x0 + lane; x < min(W, x0 + side); x += 32) {
-            float t = -1.f, tv = 0.f;
-            int ty = 0;
-            for (int y = y0; y < ye; y += 8) {
-                float v[8];
+    const int lane = threadIdx.x & 31;
+    const int x0 = (b % nbx) << lb, y0 = (b / nbx) << lb, side = 1 << lb;
+    const int ye = min(W, y0 + side);
+    unsigned long long k = 0;
+    for (int x = x0 + lane; x < min(W, x0 + side); x += 32) {
+        float t = -1.f, tv = 0.f;
+        int ty = 0;
+        for (int y = y0; y < ye; y += 8) {
+            float v[8];
 #pragma unroll
-                for (int r = 0; r < 8; ++r) v[r] = y + r < ye ? __ldcs(img + (size_t(y + r) * W + x)) : 0.f;
+            for (int r = 0; r < 8; ++r) v[r] = y + r < ye ? __ldcs(img + (size_t(y + r) * W + x)) : 0.f;
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    if (y + r >= ye) break;
-                    if (copy_to) copy_to[size_t(y + r) * W + x] = v[r];
-                    if (fabsf(v[r]) > t) {  // rows in order: strict '>' keeps the first
-                        t = fabsf(v[r]);
-                        tv = v[r];
-                        ty = y + r;
-                    }
+            for (int r = 0; r < 8; ++r) {
+                if (y + r >= ye) break;
+                if (copy_to) copy_to[size_t(y + r) * W + x] = v[r];
+                if (fabsf(v[r]) > t) {  // rows in order: strict '>' keeps the first
+                    t = fabsf(v[r]);
+                    tv = v[r];
+                    ty = y + r;
                 }
             }
-            if (t >= 0.f) {
-                k = max(k, cand_key(tv, x, ty));
-            }
         }
-        k = warp_max(k);
-        if (lane == 0) {
-            top[b] = cand_abs(k);
-            if (applied) applied[b] = 0;
-        }
-        best = max(best, k);
+        if (t >= 0.f) k = max(k, cand_key(tv, x, ty));
     }
-    // the one-pass kernels' form of it: a flat index
-    const unsigned int at = cand_index(best), flat = (at >> 16) * unsigned(W) + (at & 0xffffu);
-    const unsigned long long old = best ? ((best >> 33) << 32) | unsigned(~flat) : 0ull;
-    finish_scan(old, cand_value(best), keys, vals, int(gridDim.x), st, slot);
+    k = warp_max(k);
+    if (lane == 0) top[b] = cand_abs(k);
+    return k;
+}
+
+// The largest of the blocks' candidates, to every thread: its value v, and its flat index returned (an
+// all-zero image: 0 and 0, as findPeak has it).
+__device__ __forceinline__ unsigned int win_of(const unsigned long long* keys, const float* vals, int n, float& v)
+{
+    unsigned long long k = 0;
+    v = 0.f;
+    for (int i = threadIdx.x; i < n; i += kHogThreads) {
+        const unsigned long long ki = __ldcg(keys + i);
+        if (ki > k) {
+            k = ki;
+            v = __ldcg(vals + i);
+        }
+    }
+    k = block_max(k, v);
+    if ((k >> 32) != 0) return key_index(k);
+    v = 0.f;
+    return 0u;
+}
+
+// Both images' blocks (one warp per block) and peaks, residual = dirty, in one launch; the CTA that
+// finishes last finds the peaks and counts the blocks of the dirty image that say whether put-off updates
+// pay (a launch for each image and none for the count: as long).
+__global__ void __launch_bounds__(kHogThreads) hog_blocks_kernel(DeferArgs a, const float* __restrict__ dirty, float* pmax)
+{
+    HogState* st = a.h.state;
+    const int W = a.h.width, P = a.h.psf_width, nb = a.nbx * a.nbx, np = a.npx * a.npx, ctas = int(gridDim.x);
+    const int warp = int(blockIdx.x) * (kHogThreads / 32) + (threadIdx.x >> 5), warps = ctas * (kHogThreads / 32);
+    unsigned long long best[2] = {0, 0};  // the image's, the PSF's
+    for (int b = warp; b < np + nb; b += warps)
+        if (b < np) {
+            best[1] = max(best[1], scan_block(a.h.psf, nullptr, P, a.lbp, a.npx, b, pmax));
+        } else {
+            best[0] = max(best[0], scan_block(dirty, a.h.residual, W, a.lb, a.nbx, b - np, a.bound));
+            if ((threadIdx.x & 31) == 0) a.applied[b - np] = 0;
+        }
+    __shared__ bool last;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        // the one-pass kernels' form of a candidate: a flat index, and the value beside it
+        const unsigned int at = cand_index(best[i]), flat = (at >> 16) * unsigned(i ? P : W) + (at & 0xffffu);
+        float v = cand_value(best[i]);
+        const unsigned long long k = block_max(best[i] ? ((best[i] >> 33) << 32) | unsigned(~flat) : 0ull, v);
+        if (threadIdx.x == 0) {
+            a.h.keys[i * ctas + blockIdx.x] = k;
+            a.h.vals[i * ctas + blockIdx.x] = v;
+        }
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&st->arrived, 1u) == unsigned(ctas - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    float peak, psf_peak;
+    const unsigned int ppos = win_of(a.h.keys, a.h.vals, ctas, peak);
+    const unsigned int psf_pos = win_of(a.h.keys + ctas, a.h.vals + ctas, ctas, psf_peak);
+    unsigned int near = 0, tops = 0;
+    const int px = int(psf_pos % unsigned(P));
+    const float half = 0.5f * fabsf(peak);
+    // the peak's pixel after the first update, a lower limit of the second peak (see hog_lead_kernel)
+    const float least = fabsf(__fsub_rn(peak, __fmul_rn(__fmul_rn(a.h.gain, peak), a.h.psf[size_t(px) * P + px])));
+    for (int b = threadIdx.x; b < nb; b += kHogThreads) {
+        const float top = __ldcg(a.bound + b);
+        near += !(top < half);
+        tops += !(top < least);
+    }
+    near = __reduce_add_sync(0xffffffffu, near);
+    tops = __reduce_add_sync(0xffffffffu, tops);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&st->near, near);
+        atomicAdd(&st->tops, tops);
+    }
+    if (threadIdx.x == 0) {
+        st->win_key[0] = static_cast<unsigned int>(~ppos);
+        st->win_val[0] = peak;
+        st->psf_pos = psf_pos;
+        st->arrived = 0;
+    }
 }
 
 constexpr int kLeadRows = 8;  // rows per warp: four warps per hot block, four blocks at a time
@@ -848,13 +921,11 @@ __global__ void __launch_bounds__(kLeadThreads, 1) hog_lead_kernel(DeferArgs a, 
     LeadShared& sh = *reinterpret_cast<LeadShared*>(lead_smem);
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     HogState* st = a.h.state;
-    cudaGridDependencySynchronize();  // launched ahead of the apply kernel's end
+    cudaGridDependencySynchronize();  // launched ahead of the end of the kernel before
     if (st->stopped || st->error) return;  // an earlier launch stopped the loop (the whole cluster returns)
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
-    if (st->pass) {
-        if (blockIdx.x == 0 && tid == 0) st->meet = 0;  // for its next launch
-        return;
-    }
+    if (blockIdx.x == 0 && tid == 0) st->meet = 0;  // for the next launch of passes
+    if (st->pass) return;
     const int W = a.h.width, P = a.h.psf_width, ctas = int(gridDim.x), rank = int(blockIdx.x);
     const int side = 1 << a.lb;
     const LeadDeal deal(a.nbx, ctas);
@@ -1202,47 +1273,56 @@ __global__ void __launch_bounds__(kApplyThreads) hog_apply_kernel(DeferArgs a, i
     }
 }
 
-// Iterations [it0, it1) with a pass over the image each, all CTAs meeting in between, once put-off
-// updates do not pay any more: where the residual is down to noise, the next peak may be in thousands of
-// blocks, and the leading cluster takes most of the time (5 sources cleaned in 1000 iterations: 4096^2 32.8
-// us an iteration, with this kernel 21.7; 2048^2 12.0 and 8.2).  It takes over for good, at the start of a
-// ring (all blocks are up to date then) when a leading CTA had more than visits_max hot blocks in the
-// last launch; until then a launch of it ends at once (11 us each, one per ring).  Two candidate buffers
-// suffice: a CTA cannot write iteration it + 1's before every CTA has arrived at barrier it, i.e. has
-// read iteration it - 1's.
-template <bool kVec>
-__global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, int it0, int it1)
+// Iterations [it0, it1) with a pass over the image each, all CTAs meeting in between, where put-off
+// updates do not pay: where the residual is flat, as a cleaned one is, the next peak may be in thousands of
+// blocks, the leading cluster takes most of the time and the applying launches find most blocks near the
+// peak.  Takes over for good, at the start of a ring (all blocks are up to date then); until then a launch
+// ends at once (3 us each).  From the start for an image with more blocks near half its peak, or above the
+// limit of its second peak, than lim says; later by the last launch's list of blocks near the peak and its
+// hot blocks (PassLimits pass_limits()).  us for 100 iterations, and in brackets with put-off updates up to
+// the first ring's end: an image cleaned before 1900^2 881 (1270), 2600^2 1232 (1819), 4096^2 2342 (3862);
+// noise 883 (1655), 1233 (1930), 2504 (3420).
+// Two CTAs an SM where the images stay in L2, three beyond (4096^2 26.8 -> 24.5 us an iteration; 2048^2
+// 8.4 -> 9.2; they meet at 2800^2).  Two candidate buffers suffice: a CTA cannot write iteration it + 1's
+// before every CTA has arrived at barrier it, i.e. has read iteration it - 1's.
+template <bool kVec, int kCtas>
+__global__ void __launch_bounds__(kHogThreads, kCtas) hog_pass_kernel(HogArgs a, PassLimits lim, int it0, int it1,
+                                                                      unsigned long long wait_ns, unsigned int withheld)
 {
-    HogState* st = a.h.state;
-    if (st->stopped || st->error || st->visits <= a.visits_max) return;
+    HogState* st = a.state;
+    // set by an earlier launch, or behind a fence when this one is done
+    const bool own = *reinterpret_cast<volatile int*>(&st->pass) != 0;
+    if (st->stopped || st->error) return;
+    if (!own && (it0 == 0 ? st->near <= lim.near && st->tops <= lim.tops : st->nwarm <= lim.warm && st->visits <= lim.visits)) return;
+    if (own) it0 = max(it0, *reinterpret_cast<volatile int*>(&st->pass_end));
+    if (it0 >= it1) return;
     const unsigned int psf_pos = st->psf_pos;
     __shared__ int ok;
-    // from the leading cluster, or from this kernel's last launch (set behind a fence)
-    const bool own = *reinterpret_cast<volatile int*>(&st->pass) != 0;
     unsigned int ppos = own ? __ldcg(&st->win_next) : key_index(__ldcg(&st->win_key[0]));
     float peak = own ? __ldcg(&st->val_next) : __ldcg(&st->win_val[0]);
-    for (int it = it0; it < it1; ++it) {
-        if (fabsf(peak) < a.h.threshold) {  // every CTA holds the same winner: all stop here
+    int it = it0;
+    for (; it < it1; ++it) {
+        if (fabsf(peak) < a.threshold) {  // every CTA holds the same winner: all stop here
             if (blockIdx.x == 0 && threadIdx.x == 0) st->stopped = it + 1;
             break;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            model_update(a.h, it, ppos, peak);
+            model_update(a, it, ppos, peak);
             st->done = it + 1;
         }
         float bv;
         unsigned long long skipped;
-        unsigned long long best = iter_body<kVec>(a.h, ppos, peak, psf_pos, bv, skipped);
+        unsigned long long best = iter_body<kVec>(a, ppos, peak, psf_pos, bv, skipped);
         if (skipped) atomicAdd(&st->skipped_rows, skipped);
         best = block_max(best, bv);
-        unsigned long long* keys = a.h.keys + (it & 1) * a.h.nblocks;
-        float* vals = a.h.vals + (it & 1) * a.h.nblocks;
+        unsigned long long* keys = a.keys + (it & 1) * a.nblocks;
+        float* vals = a.vals + (it & 1) * a.nblocks;
         if (threadIdx.x == 0) {
             keys[blockIdx.x] = best;
             vals[blockIdx.x] = bv;
             __threadfence();
             atomicAdd(&st->meet, 1u);
-            const unsigned int target = unsigned(it - it0 + 1) * unsigned(a.h.nblocks) + a.withheld;
+            const unsigned int target = unsigned(it - it0 + 1) * unsigned(a.nblocks) + withheld;
             ok = 0;
             const unsigned long long t0 = global_ns();
             for (unsigned int spin = 0; spin < (1u << 24); ++spin) {
@@ -1252,32 +1332,21 @@ __global__ void __launch_bounds__(kHogThreads, 2) hog_pass_kernel(DeferArgs a, i
                 }
                 if (*reinterpret_cast<volatile int*>(&st->error)) break;
                 __nanosleep(32);
-                if ((spin & 63u) == 63u && global_ns() - t0 >= a.wait_ns) break;
+                if ((spin & 63u) == 63u && global_ns() - t0 >= wait_ns) break;
             }
             if (!ok) st->error = 1;
             __threadfence();
         }
         __syncthreads();
         if (!ok) return;
-        unsigned long long k = 0;
-        float v = 0.f;
-        for (int i = threadIdx.x; i < a.h.nblocks; i += kHogThreads) {
-            const unsigned long long ki = __ldcg(keys + i);
-            if (ki > k) {
-                k = ki;
-                v = __ldcg(vals + i);
-            }
-        }
-        k = block_max(k, v);
-        const bool zero = (k >> 32) == 0;  // an all-zero residual: the reference keeps maxPos = 0, maxVal = 0
-        ppos = zero ? 0u : key_index(k);
-        peak = zero ? 0.f : v;
+        ppos = win_of(keys, vals, a.nblocks, peak);
     }
-    // for the next launch.  A CTA that starts only now (all stopped at once) reads the winner it would
-    // have read before.
+    // for the next launch.  A CTA that starts only now (all stopped at once) finds what it would have
+    // found before.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->win_next = ppos;
         st->val_next = peak;
+        st->pass_end = it;
         __threadfence();
         st->pass = 1;
     }
@@ -1327,8 +1396,8 @@ struct HogWork {
         state = static_cast<HogState*>(take(sizeof(HogState)));
         post = static_cast<unsigned long long*>(take(size_t(2) * kResClusters * 2 * 8));
         zeroed = size_t(q - static_cast<char*>(w));
-        keys = static_cast<unsigned long long*>(take(size_t(kHogMaxBlocks) * 8));
-        vals = static_cast<float*>(take(size_t(kHogMaxBlocks) * 4));
+        keys = static_cast<unsigned long long*>(take(size_t(2) * kHogMaxBlocks * 8));  // two sets
+        vals = static_cast<float*>(take(size_t(2) * kHogMaxBlocks * 4));
         bound = static_cast<float*>(take(size_t(kBlkMax) * 4));
         pmax = static_cast<float*>(take(size_t(kBlkMax) * 4));
         applied = static_cast<int*>(take(size_t(kBlkMax) * 4));
@@ -1459,12 +1528,20 @@ int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArg
     return 0;
 }
 
-// Hot blocks of a leading CTA in one launch from which a pass over the image per iteration is faster: 6
-// an iteration at 2048^2, 18 at 4096^2.  us an iteration of 1000 by the blocks at which the passes take over
-// (0: never): 2048^2, 5 sources 0 13.0, 12 8.24, 6 8.22; 60 sources 0 9.07, 12 9.05, 6 8.30, 4 8.42; 40 sources,
-// 300 iterations 0 7.36, 6 7.40, 4 8.0.  2600^2, 20 sources 0 9.03, 8 9.02, 6 11.5.  4096^2, 5 sources 0 35.9,
-// 24 21.9, 12 21.9; 60 sources 0 19.5, 24 19.5, 12 21.4, 8 27.5.
-unsigned int visits_limit(long long n) { return unsigned(kLeadIters * (2 + (n >> 20))); }
+// At the start: more than 4 % of the blocks near half the peak (sources and their sidelobes: 0.2 to 2 %; an
+// extended source of a twelfth of the side 3.5, where both are as fast; 400 sources 5 to 8, cleaned images 25
+// to 60, noise 100), or more above the second peak's limit than an iteration may have hot (equal sources).
+// Later: two fifths near the peak (4096^2, 300 sources, 300 iterations 9.6 -> 7.4 ms; 20 sources cleaned by
+// 100, 1000 more 15.8 -> 14.5; a twelfth switched 3 sources too early, 200 iterations 2.72 -> 3.01), or hot
+// blocks of a leading CTA in one launch: 6 an iteration at 2048^2, 18 at 4096^2.  us an iteration of 1000 by
+// the hot blocks (0: never; nothing else): 2048^2, 5 sources 0 13.0, 12 8.24, 6 8.22; 60 sources 0 9.07, 12
+// 9.05, 6 8.30, 4 8.42; 40 sources, 300 iterations 0 7.36, 6 7.40, 4 8.0.  2600^2, 20 sources 0 9.03, 8 9.02,
+// 6 11.5.  4096^2, 5 sources 0 35.9, 24 21.9, 12 21.9; 60 sources 0 19.5, 24 19.5, 12 21.4, 8 27.5.
+PassLimits pass_limits(long long n, int blocks)
+{
+    const unsigned int hot = unsigned(2 + (n >> 20));
+    return PassLimits{unsigned(blocks) / 25u, hot * kLeadCtas, unsigned(blocks) * 2u / 5u, hot * kLeadIters};
+}
 
 // All iterations with put-off updates.  false: the device cannot hold the cluster, nothing launched.
 tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* dirty, int niters, cudaStream_t st, bool& ran)
@@ -1489,13 +1566,9 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     if (!lead_ctas(cfg, attr, a)) return TCV_OK;
     cfg.stream = st;
     const int nb = a.nbx * a.nbx;
-    auto scan_ctas = [](int blocks) { return std::min(kHogMaxBlocks, (blocks + kHogThreads / 32 - 1) / (kHogThreads / 32)); };
-    // the PSF's peak (HogbomGolden.cc:73-76), then residual = dirty with the first scan (:70)
-    hog_blocks_kernel<<<scan_ctas(a.npx * a.npx), kHogThreads, 0, st>>>(h.psf, nullptr, h.psf_width, a.lbp, a.npx, w.pmax,
-                                                                        nullptr, h.keys, h.vals, h.state, 2);
-    TCV_CUDA(cudaGetLastError());
-    hog_blocks_kernel<<<scan_ctas(nb), kHogThreads, 0, st>>>(dirty, h.residual, h.width, a.lb, a.nbx, w.bound, w.applied,
-                                                             h.keys, h.vals, h.state, 0);
+    // the PSF's peak (HogbomGolden.cc:73-76), residual = dirty with the first scan (:70)
+    const int scans = std::min(kHogMaxBlocks, (nb + a.npx * a.npx + kHogThreads / 32 - 1) / (kHogThreads / 32));
+    hog_blocks_kernel<<<scans, kHogThreads, 0, st>>>(a, dirty, w.pmax);
     TCV_CUDA(cudaGetLastError());
     const size_t win = size_t(kSlots) * kWindow * sizeof(float);
     TCV_CUDA(cudaFuncSetAttribute(hog_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(win)));
@@ -1504,21 +1577,30 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_apply_kernel, kApplyThreads, win));
     const int most = std::min(nb, sms * std::max(1, per_sm));
-    // the one-pass kernel that may take over: two CTAs per SM at most, as many as are resident
+    // the one-pass kernel that may take over, as many CTAs as are resident
     const bool vec = h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0;
-    const void* pass = vec ? reinterpret_cast<const void*>(hog_pass_kernel<true>)
-                           : reinterpret_cast<const void*>(hog_pass_kernel<false>);
+    const bool large = (h.n + (long long)h.psf_width * h.psf_width) * 4 > (64ll << 20);
+    const void* pass = large ? (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 3>)
+                                    : reinterpret_cast<const void*>(hog_pass_kernel<false, 3>))
+                             : (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 2>)
+                                    : reinterpret_cast<const void*>(hog_pass_kernel<false, 2>));
     int coop = 0;
     TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass, kHogThreads, 0));
     const bool passes = coop && per_sm > 0;
-    a.visits_max = passes ? visits_limit(h.n) : 0xffffffffu;
-    DeferArgs ap = a;
-    ap.h.nblocks = std::max(1, std::min({sms * std::min(per_sm, 2), kHogMaxBlocks / 2, hog_blocks(h.n), h.width}));
+    HogArgs hp = h;
+    hp.nblocks = std::max(1, std::min({sms * std::min(per_sm, large ? 3 : 2), kHogMaxBlocks, hog_blocks(h.n), h.width}));
+    PassLimits lim = pass_limits(h.n, nb);
+    auto pass_launch = [&](int from, int to) -> tcv_status {
+        void* args[] = {&hp, &lim, &from, &to, &a.wait_ns, &a.withheld};
+        TCV_CUDA(cudaLaunchCooperativeKernel(pass, dim3(unsigned(hp.nblocks)), dim3(kHogThreads), args, 0, st));
+        return TCV_OK;
+    };
     cudaLaunchAttribute attrs[2] = {attr, {}};
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
+    cfg.numAttrs = 2;
     cudaLaunchConfig_t apply{};
     apply.gridDim = dim3(unsigned(most));
     apply.blockDim = dim3(kApplyThreads);
@@ -1528,12 +1610,8 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     apply.numAttrs = 1;
     for (int it = 0, base = 0; it < niters; it += kLeadIters) {
         const int to = std::min(niters, it + kLeadIters);
-        if (passes && it == base && it > 0) {  // all blocks are up to date
-            int from = it, end = std::min(niters, it + kRing);
-            void* args[] = {&ap, &from, &end};
-            TCV_CUDA(cudaLaunchCooperativeKernel(pass, dim3(unsigned(ap.h.nblocks)), dim3(kHogThreads), args, 0, st));
-        }
-        cfg.numAttrs = it > base ? 2 : 1;  // behind the apply kernel
+        // all blocks are up to date; from the start to the end (the arrivals have to fit 32 bits)
+        if (passes && it == base) TCV_CHECK(pass_launch(it, std::min(niters, it == 0 ? 1 << 20 : it + kRing)));
         TCV_CUDA(cudaLaunchKernelEx(&cfg, hog_lead_kernel, a, it, to, base));
         const int all = to == niters || to - base == kRing;
         TCV_CUDA(cudaLaunchKernelEx(&apply, hog_apply_kernel, a, base, all));

@@ -42,3 +42,31 @@ def test_scaled_conversion_is_two_passes(tcv, cuda_ok):
     c.real.uniform_(-1.0, 1.0)
     two, one = _us(lambda: raw.convert_c(c, _lib.CTYPE_BY_NAME["rf16"]), lambda: raw.convert_c(c, _lib.CTYPE_BY_NAME["r32"]))
     assert two <= 1.5 * one, (two, one)
+
+
+@pytest.mark.parametrize("width,niters", [(1900, 100), (2600, 100), (4096, 40), (4096, 100)])
+def test_clean_of_a_flat_image(tcv, cuda_ok, width, niters):
+    """CLEAN of noise, which is what later cycles find: put-off updates would bring most blocks up to date again
+    and again, so it is a pass over the image an iteration.  Bar: a tenth over a launch per iteration."""
+    import torch
+
+    from tconvolve.hogbom import Workspace, deconvolve_device
+    from tconvolve.workload import synthetic_psf
+
+    L = tcv.lib()
+    d = torch.randn(width * width, generator=torch.Generator("cuda").manual_seed(width), device="cuda")
+    p = torch.from_numpy(synthetic_psf(width).ravel()).cuda()
+    m, r, ws = torch.zeros_like(d), torch.empty_like(d), Workspace(width)
+
+    def form(strategy):
+        def run():
+            L.tcv_hogbom_set_strategy(strategy)
+            deconvolve_device(d, width, p, width, m, r, niters, 0.1, 0.0, work=ws)
+
+        return run
+
+    try:
+        auto, each = _us(form(0), form(1))
+    finally:
+        L.tcv_hogbom_set_strategy(0)
+    assert auto <= 1.1 * each, (auto, each)
