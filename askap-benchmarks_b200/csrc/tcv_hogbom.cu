@@ -684,8 +684,8 @@ struct UpdateSlot {
 
 // Where passes over the image take over from put-off updates (hog_pass_kernel): with more blocks than these
 struct PassLimits {
-    unsigned int near, tops;    // at the start: near half the peak; above the second peak's limit
-    unsigned int warm, visits;  // later: of the last launch's list for hog_apply_kernel; hot in a leading CTA
+    int near, tops;    // at the start: near half the peak (-1: always); above the second peak's limit
+    int warm, visits;  // later: of the last launch's list for hog_apply_kernel; hot in a leading CTA
 };
 
 struct DeferArgs {
@@ -1293,7 +1293,9 @@ __global__ void __launch_bounds__(kHogThreads, kCtas) hog_pass_kernel(HogArgs a,
     // set by an earlier launch, or behind a fence when this one is done
     const bool own = *reinterpret_cast<volatile int*>(&st->pass) != 0;
     if (st->stopped || st->error) return;
-    if (!own && (it0 == 0 ? st->near <= lim.near && st->tops <= lim.tops : st->nwarm <= lim.warm && st->visits <= lim.visits)) return;
+    if (!own && (it0 == 0 ? int(st->near) <= lim.near && int(st->tops) <= lim.tops
+                          : int(st->nwarm) <= lim.warm && int(st->visits) <= lim.visits))
+        return;
     if (own) it0 = max(it0, *reinterpret_cast<volatile int*>(&st->pass_end));
     if (it0 >= it1) return;
     const unsigned int psf_pos = st->psf_pos;
@@ -1539,8 +1541,52 @@ int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArg
 // 6 11.5.  4096^2, 5 sources 0 35.9, 24 21.9, 12 21.9; 60 sources 0 19.5, 24 19.5, 12 21.4, 8 27.5.
 PassLimits pass_limits(long long n, int blocks)
 {
-    const unsigned int hot = unsigned(2 + (n >> 20));
-    return PassLimits{unsigned(blocks) / 25u, hot * kLeadCtas, unsigned(blocks) * 2u / 5u, hot * kLeadIters};
+    const int hot = int(2 + (n >> 20));
+    return PassLimits{blocks / 25, hot * kLeadCtas, blocks * 2 / 5, hot * kLeadIters};
+}
+
+// The kernel of passes for an image: as many CTAs as are resident; ctas 0 where it cannot run.
+struct Passes {
+    const void* kernel;
+    HogArgs h;
+    int ctas;
+};
+tcv_status passes_of(const HogArgs& h, Passes& p)
+{
+    const bool vec = h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0;
+    const bool large = (h.n + (long long)h.psf_width * h.psf_width) * 4 > (64ll << 20);
+    p.kernel = large ? (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 3>)
+                            : reinterpret_cast<const void*>(hog_pass_kernel<false, 3>))
+                     : (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 2>)
+                            : reinterpret_cast<const void*>(hog_pass_kernel<false, 2>));
+    int dev = 0, sms = 0, per_sm = 0, coop = 0;
+    TCV_CUDA(cudaGetDevice(&dev));
+    TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, kHogThreads, 0));
+    p.ctas = coop ? std::min({sms * std::min(per_sm, large ? 3 : 2), kHogMaxBlocks, hog_blocks(h.n), h.width}) : 0;
+    p.h = h;
+    p.h.nblocks = p.ctas;
+    return TCV_OK;
+}
+tcv_status launch_passes(Passes& p, PassLimits lim, int from, int to, cudaStream_t st)
+{
+    void* args[] = {&p.h, &lim, &from, &to, &g_wait_ns, &g_withheld};
+    TCV_CUDA(cudaLaunchCooperativeKernel(p.kernel, dim3(unsigned(p.ctas)), dim3(kHogThreads), args, 0, st));
+    return TCV_OK;
+}
+
+// All iterations as passes, in one cooperative launch.  ran = false: nothing launched.
+tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, cudaStream_t st, bool& ran)
+{
+    ran = false;
+    Passes p;
+    TCV_CHECK(passes_of(h, p));
+    // the arrivals reach niters x CTAs: within 32 bits
+    if (p.ctas < 1 || uint64_t(niters) * uint64_t(p.ctas) >= 1ull << 32) return TCV_OK;
+    TCV_CHECK(first_scans(h, dirty, st));
+    ran = true;
+    return niters > 0 ? launch_passes(p, PassLimits{-1, -1, -1, -1}, 0, niters, st) : TCV_OK;
 }
 
 // All iterations with put-off updates.  false: the device cannot hold the cluster, nothing launched.
@@ -1577,25 +1623,8 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hog_apply_kernel, kApplyThreads, win));
     const int most = std::min(nb, sms * std::max(1, per_sm));
-    // the one-pass kernel that may take over, as many CTAs as are resident
-    const bool vec = h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0;
-    const bool large = (h.n + (long long)h.psf_width * h.psf_width) * 4 > (64ll << 20);
-    const void* pass = large ? (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 3>)
-                                    : reinterpret_cast<const void*>(hog_pass_kernel<false, 3>))
-                             : (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 2>)
-                                    : reinterpret_cast<const void*>(hog_pass_kernel<false, 2>));
-    int coop = 0;
-    TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    TCV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass, kHogThreads, 0));
-    const bool passes = coop && per_sm > 0;
-    HogArgs hp = h;
-    hp.nblocks = std::max(1, std::min({sms * std::min(per_sm, large ? 3 : 2), kHogMaxBlocks, hog_blocks(h.n), h.width}));
-    PassLimits lim = pass_limits(h.n, nb);
-    auto pass_launch = [&](int from, int to) -> tcv_status {
-        void* args[] = {&hp, &lim, &from, &to, &a.wait_ns, &a.withheld};
-        TCV_CUDA(cudaLaunchCooperativeKernel(pass, dim3(unsigned(hp.nblocks)), dim3(kHogThreads), args, 0, st));
-        return TCV_OK;
-    };
+    Passes passes;  // may take over
+    TCV_CHECK(passes_of(h, passes));
     cudaLaunchAttribute attrs[2] = {attr, {}};
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1611,7 +1640,8 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     for (int it = 0, base = 0; it < niters; it += kLeadIters) {
         const int to = std::min(niters, it + kLeadIters);
         // all blocks are up to date; from the start to the end (the arrivals have to fit 32 bits)
-        if (passes && it == base) TCV_CHECK(pass_launch(it, std::min(niters, it == 0 ? 1 << 20 : it + kRing)));
+        if (passes.ctas && it == base)
+            TCV_CHECK(launch_passes(passes, pass_limits(h.n, nb), it, std::min(niters, it == 0 ? 1 << 20 : it + kRing), st));
         TCV_CUDA(cudaLaunchKernelEx(&cfg, hog_lead_kernel, a, it, to, base));
         const int all = to == niters || to - base == kRing;
         TCV_CUDA(cudaLaunchKernelEx(&apply, hog_apply_kernel, a, base, all));
@@ -1667,6 +1697,7 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     if (g_hog_strategy != TCV_HOGBOM_PER_LAUNCH) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
     if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_AUTO && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
         s = deconvolve_deferred(a, w, d_dirty, niters, st, ran);
+    if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_PERSISTENT) s = deconvolve_passes(a, d_dirty, niters, st, ran);
     if (s != TCV_OK || ran) return s;
     TCV_CHECK(first_scans(a, d_dirty, st));
     const bool vec = width % 4 == 0 && reinterpret_cast<uintptr_t>(d_residual) % 16 == 0;

@@ -582,14 +582,14 @@ tcv_status tcv_hogbom_deconvolve(const float *d_dirty, int width, const float *d
                                  float *d_model, float *d_residual, int niters, float gain,
                                  float threshold, float *d_hist_val, uint32_t *d_hist_pos,
                                  void *d_work, size_t work_bytes, void *stream);
-/* How tcv_hogbom_deconvolve issues the iterations (process-wide): AUTO (default) runs images of up
- * to 2048 x 2048 (fewer where the device holds fewer clusters) as one cooperative launch of all
- * iterations with the residual in registers (the CTAs meet once per iteration, with bounded waits)
- * and larger ones with updates put off until a block of pixels could hold the next peak (a launch
- * of one cluster and a device-wide one per 16 iterations, and cooperative launches of 128 once too
- * many blocks could; images or PSFs over 16384 wide take one launch per iteration).  PERSISTENT
- * takes the cooperative form where the image fits it, PER_LAUNCH one launch per iteration; both
- * otherwise the latter.  Results are identical. */
+/* How tcv_hogbom_deconvolve issues the iterations (process-wide): AUTO (default) runs images that fit the
+ * register files (up to 2048 x 2048 and as many clusters as the device holds: 1792 wide on a B200) as one
+ * cooperative launch of all iterations with the residual in registers, the CTAs meeting once per
+ * iteration; larger ones with updates put off until a block of pixels could hold the next peak (a launch
+ * of one cluster and a device-wide one per 16 iterations), or, where too many blocks are near the peak,
+ * as cooperative launches of a pass over the image per iteration; images or PSFs over 16384 wide with one
+ * launch per iteration.  PERSISTENT takes a cooperative launch of all iterations at any size, PER_LAUNCH
+ * one launch per iteration.  All waits are bounded (below).  Results are identical. */
 enum { TCV_HOGBOM_AUTO = 0, TCV_HOGBOM_PER_LAUNCH = 1, TCV_HOGBOM_PERSISTENT = 2 };
 void tcv_hogbom_set_strategy(int strategy);
 /* The bounded waits of the forms whose CTAs wait for one another (process-wide, for launches made after

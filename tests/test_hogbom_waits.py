@@ -55,3 +55,9 @@ def _check(strategy, w, limit_ns, niters=150):
 @pytest.mark.parametrize("limit_ns", [0, 1_000_000])
 def test_waits_run_out(tcv, cuda_ok, width, limit_ns):
     _check(AUTO, width, limit_ns)
+
+
+# the persistent form has waits at every size: widths that the registers do not hold, and odd ones
+@pytest.mark.parametrize("width", [1793, 2048, 2601, 4096])
+def test_persistent_form_is_cooperative(tcv, cuda_ok, width):
+    _check(PERSISTENT, width, 1_000_000, niters=20)
