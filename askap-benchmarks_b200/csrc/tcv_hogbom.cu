@@ -1576,6 +1576,11 @@ tcv_status launch_passes(Passes& p, PassLimits lim, int from, int to, cudaStream
     return TCV_OK;
 }
 
+// Iterations up to which a call is passes from the start: bringing all blocks up to date at its end costs as
+// much as several (us a call as passes, and in brackets with put-off updates: 1 iteration 1900^2 41 (71),
+// 4096^2 100 (217); 8 iterations 98 (103) and 280 (317), 10 116 (112) and 333 (333)).
+constexpr int kFewIters = 8;
+
 // All iterations as passes, in one cooperative launch.  ran = false: nothing launched.
 tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, cudaStream_t st, bool& ran)
 {
@@ -1695,9 +1700,10 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     bool ran = false;
     tcv_status s = TCV_OK;
     if (g_hog_strategy != TCV_HOGBOM_PER_LAUNCH) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
+    if (s == TCV_OK && !ran && (g_hog_strategy == TCV_HOGBOM_PERSISTENT || (g_hog_strategy == TCV_HOGBOM_AUTO && niters <= kFewIters)))
+        s = deconvolve_passes(a, d_dirty, niters, st, ran);
     if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_AUTO && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
         s = deconvolve_deferred(a, w, d_dirty, niters, st, ran);
-    if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_PERSISTENT) s = deconvolve_passes(a, d_dirty, niters, st, ran);
     if (s != TCV_OK || ran) return s;
     TCV_CHECK(first_scans(a, d_dirty, st));
     const bool vec = width % 4 == 0 && reinterpret_cast<uintptr_t>(d_residual) % 16 == 0;
