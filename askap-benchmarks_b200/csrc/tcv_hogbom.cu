@@ -1749,12 +1749,14 @@ tcv_status tcv_find_peak(const float* d_image, int64_t n, float* val_out, int64_
                          size_t work_bytes, void* stream)
 {
     if (!d_image || n < 1 || !d_work || n >= int64_t(0xffffffffll)) return TCV_ERR_ARG;
-    if (work_bytes < tcv_hogbom_workspace_bytes(1)) return TCV_ERR_WORKSPACE;
+    // the state and one set of candidates: less than a deconvolution's workspace
+    const size_t at_keys = align256(sizeof(HogState)), at_vals = at_keys + align256(size_t(kHogMaxBlocks) * 8);
+    if (work_bytes < at_vals + align256(size_t(kHogMaxBlocks) * 4)) return TCV_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const HogWork w(d_work);
-    HogState* state = w.state;
-    unsigned long long* keys = w.keys;
-    float* vals = w.vals;
+    char* w = static_cast<char*>(d_work);
+    HogState* state = reinterpret_cast<HogState*>(w);
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(w + at_keys);
+    float* vals = reinterpret_cast<float*>(w + at_vals);
     TCV_CUDA(cudaMemsetAsync(state, 0, sizeof(HogState), st));
     const int nb = hog_blocks(n);
     hog_scan_kernel<<<nb, kHogThreads, 0, st>>>(d_image, nullptr, n, nb, keys, vals, state, 0);

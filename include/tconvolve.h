@@ -606,7 +606,7 @@ tcv_status tcv_hogbom_set_wait(uint64_t limit_ns, uint32_t withheld_arrivals);
 tcv_status tcv_hogbom_result(const void *d_work, int *iters_done, int *stopped_at,
                              int64_t *skipped_rows, int64_t *psf_peak_pos, void *stream);
 /* findPeak (HogbomGolden.cc:127-139): the value of largest magnitude and its first index
- * (0 and 0 for an all-zero image).  Synchronises; d_work as for tcv_hogbom_deconvolve. */
+ * (0 and 0 for an all-zero image).  Synchronises; d_work as for tcv_hogbom_deconvolve (8 KiB do). */
 tcv_status tcv_find_peak(const float *d_image, int64_t n, float *val_out, int64_t *pos_out,
                          void *d_work, size_t work_bytes, void *stream);
 

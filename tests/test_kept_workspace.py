@@ -50,3 +50,17 @@ def test_kept_workspace(tcv, cuda_ok, n, made_for):
     small = torch.empty(256, dtype=torch.uint8, device="cuda")
     assert L.tcv_degrid_raw(vp(field), g, support, vp(tab), tcv.C64, 1.0, c_len, vp(co), vp(iu), vp(iv), vp(out), n,
                             vp(small), 256, st) == 7  # TCV_ERR_WORKSPACE
+
+
+@pytest.mark.gpu
+def test_find_peak_in_a_small_workspace(tcv, orc, cuda_ok):
+    """A peak's scan keeps a candidate per CTA: 8 KiB, not a deconvolution's workspace."""
+    import torch
+
+    L, a = tcv.lib(), np.random.default_rng(4).standard_normal(3_000_001).astype(np.float32)
+    d, work = torch.from_numpy(a).cuda(), torch.empty(8192, dtype=torch.uint8, device="cuda")
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    v, p = ctypes.c_float(), ctypes.c_int64()
+    assert L.tcv_find_peak(vp(d), a.size, ctypes.byref(v), ctypes.byref(p), vp(work), 8192, None) == 0
+    assert (v.value, p.value) == orc.find_peak(a)
+    assert L.tcv_find_peak(vp(d), a.size, ctypes.byref(v), ctypes.byref(p), vp(work), 4096, None) == 7  # TCV_ERR_WORKSPACE
