@@ -902,6 +902,7 @@ tcv_status build_few(tcv_plan* p, const int32_t* iu, const int32_t* iv, const in
     f.cells = uint32_t(cells);
     f.rows0 = uint32_t(std::min<size_t>(2 * align_up(np * ks) / (2 * cells), f.blocks));  // keys[1] follows keys[0]
     if (f.rows0 + align_up(np * sizeof(float2)) / (2 * cells) < f.blocks) return TCV_OK;
+    if (f.blocks * 4 + np > align_up(np * 4)) return TCV_OK;  // (one sample and tile: 5 bytes, in the padding)
     f.iu = iu;
     f.iv = iv;
     f.coff = coff;
@@ -910,7 +911,7 @@ tcv_status build_few(tcv_plan* p, const int32_t* iu, const int32_t* iv, const in
     f.var = VarPlanes{p->wplane, p->plane_s, p->plane_grp, p->ssz};
     f.row0 = static_cast<uint16_t*>(p->keys[0]);
     f.row1 = reinterpret_cast<uint16_t*>(p->slots);
-    f.nrej = p->vals[1];  // a word per block, then a byte per pair: fewer than 4 np bytes
+    f.nrej = p->vals[1];  // a word per block, then a byte per pair
     f.place = reinterpret_cast<uint8_t*>(p->vals[1] + f.blocks);
     f.ntl = p->ntl;
     f.vals = p->vals[0];
@@ -1088,6 +1089,7 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
     p->n_items = static_cast<uint32_t*>(take(4));
     p->group_start = static_cast<uint32_t*>(take(size_t(g.n_groups + 1) * 4));
     p->group_ustart = static_cast<uint32_t*>(take(size_t(g.n_groups + 1) * 4));
+    static_assert((3 * kSliceGroups + 1) * 4 <= 256, "the ranges lie in group_ustart's padding");
     p->grid_range = !g.split && g.n_groups <= kSliceGroups ? p->group_ustart + g.n_groups + 1 : nullptr;
     p->nunits = static_cast<uint32_t*>(take(cells * 4));
     p->ustart = static_cast<uint32_t*>(take(cells * 4));
