@@ -36,13 +36,19 @@ constexpr int kTX = 6, kTY = 5;  // log2 of the tile sides (64 x 32 tiles of 8-r
 static_assert((1 << kTX) == kTileW && (1 << kTY) == tile_height(8), "key fields");
 constexpr uint32_t kNone = 0xffffffffu;
 
-struct Head {  // 1 where a sorted key differs from the one before it (fillers of left-out samples: 0)
+// The samples of one footprint are summed in order by one thread, so a footprint of more than this is taken
+// as several: a sorted sample at a multiple of it starts another.  Gridding 2^18 samples of one footprint took
+// 9.8 ms and was 1.7e-5 off (relative L2), 2^20 39 ms; now 0.17 each and within 1e-5; the tracks' sums cost
+// the same.
+constexpr uint32_t kRun = 512;
+
+struct Head {  // 1 where a footprint starts (fillers of left-out samples: 0)
     const uint64_t* keys;
     uint64_t sentinel;
     __host__ __device__ __forceinline__ uint32_t operator()(uint32_t i) const
     {
         const uint64_t k = keys[i];
-        return k < sentinel && (i == 0 || keys[i - 1] != k) ? 1u : 0u;
+        return k < sentinel && (i % kRun == 0 || keys[i - 1] != k) ? 1u : 0u;
     }
 };
 
@@ -95,7 +101,7 @@ __global__ void uniq_records_kernel(PlanGeom g, const uint64_t* __restrict__ key
         repu[k] = u;
         cell = uint32_t(key >> shift);
         const uint64_t before = i ? keys[i - 1] : sentinel, after = i + 1 < g.n ? keys[i + 1] : sentinel;
-        if (before != key) {
+        if (before != key || i % kRun == 0) {  // as Head has it
             const int s = plane_s[wplane[k]], fx = iu[k] - s / 2, fy = iv[k];
             urec[u] = make_int4(fx, fy, coff[k], s);
             ustart[u] = uint32_t(i);
