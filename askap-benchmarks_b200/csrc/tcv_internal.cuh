@@ -63,9 +63,10 @@ struct PlanGeom {
     // variable-width plans (one footprint width per w-plane; s and support are the widest)
     bool var;
     int n_planes;
-    // variable-width plans whose both passes are sample-parallel: binned by distinct footprint
-    // (tcv_unique.cu); bits of the sort key and of its table-offset and width-rank fields
-    bool uniq;
+    // variable-width plans whose both passes are sample-parallel: work units sized by the pairs there are
+    // (unit_sizes), and binned by distinct footprint (tcv_unique.cu) where they have many samples; bits of
+    // that sort key and of its table-offset and width-rank fields
+    bool scaled, uniq;
     int u_bits, u_coff_bits, u_rank_bits;
 };
 
@@ -130,6 +131,7 @@ struct tcv_plan {
     // first row, cOffset, width), gathered once per binning (nullptr unless a pass uses them)
     int4* grec;
     std::vector<int32_t> host_plane_s, host_plane_grp;
+    uint32_t* sizes;               // plans of scaled units: the work-unit sizes, gridding and degridding
     // plans binned by distinct footprint: order, slots, ntl and grec are of footprints, and
     int32_t* plane_rank;           // per plane: its width among the distinct widths
     std::vector<int32_t> host_plane_rank;
@@ -142,10 +144,28 @@ struct tcv_plan {
     uint32_t* repu;                // per sample: its footprint (all ones: left out)
     float2* usums;                 // per footprint: its samples' data, summed for a gridding pass
     uint32_t* ucell;               // per cell: list length; first and end footprint that starts in it
-    uint32_t* n_uniq;              // [0] footprints; [1], [2] work-unit sizes in footprints
+    uint32_t* n_uniq;              // [0] footprints
 };
 
 namespace tcv {
+
+// Work-unit sizes (gridding, degridding) of a plan whose both passes are sample-parallel, from the pairs
+// (of samples or footprints, with tiles) in its cells: the tuning's, or smaller where it would give less
+// than some four units per warp group of a gridding launch (888 in three CTAs per SM) or ten per CTA of a
+// degridding one (740): 77 k samples of the spectral run 129 -> 65 us gridding, 62 -> 43 degridding, 383 k
+// 177 -> 139.  Smaller still costs a unit's tile again: continuum degridding 2.07 ms with 37 footprints a
+// unit, 1.56 ms with 128.  Not below what the unit lists and partial tiles, made for the most pairs
+// that the samples can have, have room for.
+__device__ __forceinline__ void unit_sizes(const PlanGeom& g, uint32_t pairs, uint32_t* sizes)
+{
+    const unsigned long long most = (unsigned long long)(g.n) * g.max_tiles;
+    const auto size = [&](uint32_t s, uint32_t units) {
+        const uint32_t room = uint32_t((pairs * (unsigned long long)(s) + most - 1) / most), want = pairs / units;
+        return s ? max(max(32u, room), min(s, want)) : 0u;
+    };
+    sizes[0] = size(uint32_t(g.split), 4096u);
+    sizes[1] = size(uint32_t(g.dsplit), 8192u);
+}
 
 constexpr int kStatusWords = 8;  // the plan's status block, zeroed by every binning
 constexpr int kSchedWord = 4;    // first of the two work-item counters in it

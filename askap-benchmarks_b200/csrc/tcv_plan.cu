@@ -214,7 +214,7 @@ __global__ void plan_keys_kernel(const int32_t* __restrict__ iu, const int32_t* 
 // no cell.
 template <typename K>
 __global__ void run_bounds_kernel(const K* __restrict__ keys, int64_t np, int key_bits, uint32_t* run_start,
-                                  uint32_t* run_end)
+                                  uint32_t* run_end, PlanGeom g, uint32_t* sizes)
 {
     const K sentinel = K(1) << (key_bits - 1);
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -223,6 +223,7 @@ __global__ void run_bounds_kernel(const K* __restrict__ keys, int64_t np, int ke
         if (k >= sentinel) continue;
         if (i == 0 || keys[i - 1] != k) run_start[k] = uint32_t(i);
         if (i + 1 == np || keys[i + 1] != k) run_end[k] = uint32_t(i + 1);
+        if (sizes && (i + 1 == np || keys[i + 1] >= sentinel)) unit_sizes(g, uint32_t(i + 1), sizes);
     }
 }
 
@@ -858,7 +859,7 @@ CellArgs cell_args(const tcv_plan* p)
     const PlanGeom& g = p->g;
     const bool own_d = own_degrid_units(g);
     return CellArgs{p->tile_count, uint32_t(grid_cells(g)), uint32_t(g.ntiles), uint32_t(g.split), uint32_t(g.dsplit),
-                    g.n_groups, own_d, g.uniq ? p->n_uniq + 1 : nullptr, static_cast<uint32_t*>(p->cub_temp),
+                    g.n_groups, own_d, g.scaled ? p->sizes : nullptr, static_cast<uint32_t*>(p->cub_temp),
                     p->tile_start, p->items, p->n_items, p->group_start, p->nunits, p->ustart, p->pstart,
                     p->group_ustart, p->units, own_d ? p->d_nunits : nullptr, own_d ? p->d_ustart : nullptr,
                     own_d ? p->d_pstart : nullptr, own_d ? p->d_group_ustart : nullptr, own_d ? p->d_units : nullptr};
@@ -896,7 +897,7 @@ tcv_status build_few(tcv_plan* p, const int32_t* iu, const int32_t* iv, const in
     const PlanGeom& g = p->g;
     *done = false;
     const size_t cells = grid_cells(g), np = size_t(g.n) * g.max_tiles, ks = g.key64 ? 8 : 4;
-    if (g.n < 1 || g.n > kFewSamples || g.uniq || cells > kFewCells) return TCV_OK;
+    if (g.n < 1 || g.n > kFewSamples || g.scaled || cells > kFewCells) return TCV_OK;
     FewArgs f{};
     f.blocks = uint32_t((g.n + kFewThreads - 1) / kFewThreads);
     f.cells = uint32_t(cells);
@@ -940,7 +941,7 @@ tcv_status build_uniq(tcv_plan* p, cudaStream_t st)
     TCV_CUDA(cudaMemsetAsync(p->tile_start, 0, sizeof(uint32_t) * cells, st));
     TCV_CUDA(cudaMemsetAsync(p->rejected, 0, sizeof(unsigned long long), st));
     TCV_CUDA(cudaMemsetAsync(p->status, 0, kStatusWords * sizeof(unsigned int), st));
-    TCV_CUDA(cudaMemsetAsync(p->n_uniq, 0, 3 * sizeof(uint32_t), st));
+    TCV_CUDA(cudaMemsetAsync(p->sizes, 0, 3 * sizeof(uint32_t), st));
     if (p->g.n > 0) TCV_CHECK(uniq_bin(p, st));
     p->anchors_ready = false;
     return cells_and_units(p, st);
@@ -969,6 +970,7 @@ tcv_status build(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_
     if (with_anchors) TCV_CUDA(cudaMemsetAsync(p->atile_count, 0, sizeof(uint32_t) * size_t(acells), st));
     TCV_CUDA(cudaMemsetAsync(p->rejected, 0, sizeof(unsigned long long), st));
     TCV_CUDA(cudaMemsetAsync(p->status, 0, kStatusWords * sizeof(unsigned int), st));
+    if (g.scaled) TCV_CUDA(cudaMemsetAsync(p->sizes, 0, 3 * sizeof(uint32_t), st));
     if (g.n > 0) {
         const VarPlanes var{p->wplane, p->plane_s, p->plane_grp, p->ssz};
         // staged key writes while a block's pairs fit the default 48 KB of shared memory
@@ -997,7 +999,8 @@ tcv_status build(tcv_plan* p, const int32_t* iu, const int32_t* iv, const int32_
         int sms = 148, dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int64_t rb = std::min<int64_t>((np + 255) / 256, int64_t(sms) * 8);
-        run_bounds_kernel<K><<<unsigned(rb), 256, 0, st>>>(kb.Current(), np, g.key_bits, p->tile_start, p->tile_count);
+        run_bounds_kernel<K><<<unsigned(rb), 256, 0, st>>>(kb.Current(), np, g.key_bits, p->tile_start, p->tile_count, g,
+                                                             g.scaled ? p->sizes : nullptr);
         TCV_CUDA(cudaGetLastError());
     } else {
         p->sel = 0;
@@ -1076,7 +1079,10 @@ tcv_status plan_create(tcv_plan* p, void* d_work, size_t work_bytes, cudaStream_
         p->repu = static_cast<uint32_t*>(take(n * 4));
         p->usums = static_cast<float2*>(take(n * sizeof(float2)));
         p->ucell = static_cast<uint32_t*>(take(grid_cells(g) * 3 * 4));
-        p->n_uniq = static_cast<uint32_t*>(take(3 * 4));
+    }
+    if (g.scaled) {
+        p->sizes = static_cast<uint32_t*>(take(3 * 4));
+        p->n_uniq = p->sizes + 2;
     }
     p->akeys[0] = take(an * ks);
     p->akeys[1] = take(an * ks);
@@ -1278,10 +1284,11 @@ size_t plan_bytes(const PlanGeom& g, size_t* cub_bytes_out)
         const size_t n = size_t(g.n);
         b += align_up(np * 4) + align_up(size_t(g.n_planes) * 4) + 2 * align_up(n * 8) + 4 * align_up(n * 4) +
              align_up(n * sizeof(int4)) + align_up((n + 1) * 4) + align_up(n * sizeof(float2)) +
-             align_up(grid_cells(g) * 3 * 4) + align_up(3 * 4);
+             align_up(grid_cells(g) * 3 * 4);
     } else {
         b += 2 * align_up(np * ks) + 2 * align_up(np * 4);
     }
+    if (g.scaled) b += align_up(3 * 4);
     b += 2 * align_up(an * ks) + 2 * align_up(an * 4);
     const size_t cells = grid_cells(g), acells = anchor_cells(g);
     b += 3 * align_up(cells * 4) + align_up(4) + align_up(size_t(g.n_groups + 1) * 4);
@@ -1311,6 +1318,9 @@ int width_ranks(const int32_t* s_size, int n_planes, std::vector<int32_t>* ranks
     }
     return int(w.size());
 }
+
+// Samples from which a plan is binned by distinct footprint: at least, and for each tile that one can touch
+constexpr int64_t kUniqSamples = 1 << 18, kUniqPerTile = 1 << 15;
 
 // Geometry of a variable-width plan: the widest plane sets the tile reach; whole planes are
 // grouped in order until a group's slice of the table passes group_mib (complex64).
@@ -1343,11 +1353,18 @@ PlanGeom make_geom_var(int64_t n, const int32_t* s_size, const int32_t* c_off0, 
     g.key_bits = g.tile_bits + 1;
     g.key64 = g.key_bits > 32;
     if (g.dense && g.ddense) {
-        // distinct footprints, where (cell, table offset, place in the 64 x 32 tile, width) fits a key
+        // Distinct footprints, where (cell, table offset, place in the 64 x 32 tile, width) fits a key and
+        // there are enough samples: fewer of a track share few footprints, and pay the longer sort and the
+        // lists, which look over as many cells as a footprint can touch tiles, for nothing.  us, by
+        // sample and by footprint, binning, gridding, degridding: spectral run (4 tiles) 77 k samples 85
+        // 65 43 and 176 69 45, 262 k 104 102 79 and 211 102 83, 765 k 157 241 185 and 280 187 148; continuum run
+        // (15) 109 k 116 232 210 and 314 270 220, 544 k 258 600 537 and 387 605 513, 2.2 M 716 1516 1529 and
+        // 620 1344 1031.  The line lies where a kept plan's passes take as long either way.
         g.u_coff_bits = bits_for(uint64_t(c_len - 1));
         g.u_rank_bits = bits_for(uint64_t(width_ranks(s_size, n_planes, nullptr) - 1));
         g.u_bits = g.tile_bits + g.u_coff_bits + 11 + g.u_rank_bits;
-        g.uniq = g.u_bits < 64;
+        g.uniq = g.u_bits < 64 && n >= std::max(kUniqSamples, kUniqPerTile * g.max_tiles);
+        g.scaled = true;
     }
     return g;
 }

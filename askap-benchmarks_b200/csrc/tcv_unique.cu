@@ -5,8 +5,8 @@
 // width (the 12 h track of current/tConvolveMPI/Benchmark.cc:61-165: 3.83 M samples have 0.93 M
 // distinct footprints in the spectral run, 5.44 M have 1.57 M in the continuum run).  Gridding is
 // linear in the data, so a footprint is gridded once with the sum of its samples' data, and
-// degridding gives all its samples one value.  Plans whose both passes are sample-parallel are
-// binned so; the passes then work on footprints ("uniques", numbered 0 .. n_uniq - 1) where they
+// degridding gives all its samples one value.  Plans of many samples whose both passes are
+// sample-parallel are binned so (kUniqSamples); the passes then work on footprints ("uniques", numbered 0 .. n_uniq - 1) where they
 // worked on samples.
 //
 // One radix sort orders the samples by (work cell of the footprint's first point, table offset, row
@@ -170,21 +170,11 @@ uniq_lists_kernel(PlanGeom g, uint32_t cells, int reach_x, int reach_y, const in
     }
 }
 
-// The work-unit sizes in footprints: the tuning's, or smaller where the lists, shorter than samples make
-// them, would give less than some four units per warp group of a gridding launch (888 in three CTAs
-// per SM) or ten per CTA of a degridding one (740).  Smaller still costs a unit's tile again:
-// continuum degridding 2.07 ms with 37 footprints a unit, 1.56 ms with 128.  Not below what the
-// unit lists and partial tiles, made for the samples' pairs, have room for.
+// the work-unit sizes in footprints
 __global__ void uniq_split_kernel(PlanGeom g, uint32_t cells, const uint32_t* __restrict__ count,
-                                  const uint32_t* __restrict__ start, uint32_t* n_uniq)
+                                  const uint32_t* __restrict__ start, uint32_t* sizes)
 {
-    const unsigned long long pairs = start[cells - 1u] + count[cells - 1u], most = (unsigned long long)(g.n) * g.max_tiles;
-    const auto size = [&](uint32_t s, uint32_t units) {
-        const uint32_t room = uint32_t((pairs * s + most - 1) / most), want = uint32_t(pairs / units);
-        return s ? max(max(32u, room), min(s, want)) : 0u;
-    };
-    n_uniq[1] = size(uint32_t(g.split), 4096u);
-    n_uniq[2] = size(uint32_t(g.dsplit), 8192u);
+    unit_sizes(g, start[cells - 1u] + count[cells - 1u], sizes);
 }
 
 // the sums of the footprints' data, in sample order
@@ -271,7 +261,6 @@ tcv_status uniq_bin(tcv_plan* p, cudaStream_t st)
     const uint32_t cells = uint32_t(g.n_groups) * uint32_t(g.ntiles);
     const unsigned blocks = unsigned((g.n + 255) / 256);
     TCV_CUDA(cudaMemsetAsync(p->ucell, 0, size_t(cells) * 3 * sizeof(uint32_t), st));
-    TCV_CUDA(cudaMemsetAsync(p->n_uniq, 0, sizeof(uint32_t), st));
     uniq_keys_kernel<<<blocks, 256, 0, st>>>(g, p->iu, p->iv, p->coff, p->wplane, p->plane_s, p->plane_grp, p->plane_rank,
                                              p->ukeys[0], p->uvals[0], p->rejected);
     TCV_CUDA(cudaGetLastError());
@@ -291,7 +280,7 @@ tcv_status uniq_bin(tcv_plan* p, cudaStream_t st)
     const int ctas = list_ctas(cells);
     tb = p->cub_bytes;
     TCV_CUDA(cub::DeviceScan::ExclusiveSum(p->cub_temp, tb, count, p->tile_start, int64_t(cells), st));
-    uniq_split_kernel<<<1, 1, 0, st>>>(g, cells, count, p->tile_start, p->n_uniq);
+    uniq_split_kernel<<<1, 1, 0, st>>>(g, cells, count, p->tile_start, p->sizes);
     TCV_CUDA(cudaGetLastError());
     // few cells have long lists (spectral run: 561 cells, up to 37 k footprints): large CTAs there
     if (cells < 4096)

@@ -89,3 +89,35 @@ def test_clean_of_few_iterations(tcv, cuda_ok, width, niters):
 
     auto, each = _clean(tcv, width, torch.from_numpy(synthetic_dirty(width, 20, 1e-3, seed=5).ravel()).cuda(), niters)
     assert auto <= 1.1 * each, (auto, each)
+
+
+@pytest.mark.parametrize("run,part", [(1, 0.02), (1, 0.06), (0, 0.02)])
+def test_new_plan_of_a_short_track(tcv, cuda_ok, run, part):
+    """A plan of a short stretch of the 12 h track, made for one gridding pass, both passes sample-parallel:
+    binning costs about what it costs a plan that degrids by tiles (binned by sample, gridded alike with units
+    of 512 samples).  Bar: a tenth over that."""
+    import torch
+
+    from tconvolve import current, raw
+
+    b = current.Benchmark()
+    b.setRunType(run)
+    b.init()
+    geo, n = b.geometry(), int(part * b.nVisibilitiesGridded())
+    iu, iv, wp, co = (torch.from_numpy(a[:n].copy()).cuda() for a in b.offsets())
+    (s_size, off0), c = b.planes(), torch.from_numpy(b.C()).cuda()
+    b.close()
+    data = torch.ones(n, dtype=torch.complex64, device="cuda")
+    grid = torch.zeros(int(geo.g_size) ** 2, dtype=torch.complex64, device="cuda")
+    plans = [raw.VarPlan(iu, iv, co, wp, s_size, off0, int(geo.g_size), int(geo.c_len), tuning=(8, -1, 512, 128, k)) for k in (3, 1)]
+    vp = lambda t: raw._ptr(t)  # noqa: E731
+
+    def once(plan):
+        def run_():
+            assert tcv.lib().tcv_plan_bin(plan.handle, vp(iu), vp(iv), vp(co), raw._stream()) == 0
+            plan.grid(data, c, tcv.C64, grid)
+
+        return run_
+
+    both, one = _us(once(plans[0]), once(plans[1]))
+    assert both <= 1.1 * one, (both, one)
