@@ -1443,9 +1443,10 @@ tcv_status deconvolve_resident(const HogArgs& h, const HogWork& w, const float* 
     ran = false;
     const int W = h.width;
     if (W > kResChunks * kResThreads || h.psf_width > 65535) return TCV_OK;
-    int dev = 0, coop = 0;
+    int dev = 0, coop = 0, sms = 0;
     TCV_CUDA(cudaGetDevice(&dev));
     TCV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    TCV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (!coop) return TCV_OK;
     const int chunks = (W + kResThreads - 1) / kResThreads;
     cudaLaunchAttribute attr[2];
@@ -1463,7 +1464,7 @@ tcv_status deconvolve_resident(const HogArgs& h, const HogWork& w, const float* 
     for (int rows_t : {-8, -16, 4, 8, 16}) {  // negative: one cluster
         const bool one = rows_t < 0;
         rows_t = std::abs(rows_t);
-        if (one && (W + 15) / 16 > rows_t) continue;
+        if (W > (one ? 16 : sms) * rows_t) continue;  // too few CTAs (asking the device takes 5 us)
         const ResKernel kernel = one ? (rows_t == 8 ? ResKernel(hog_resident_kernel<8, 1, true>)
                                                     : ResKernel(hog_resident_kernel<16, 1, true>))
                                  : rows_t == 4 ? resident_of<4>(chunks)
@@ -1579,7 +1580,8 @@ tcv_status launch_passes(Passes& p, PassLimits lim, int from, int to, cudaStream
 // Iterations up to which a call is passes from the start: bringing all blocks up to date at its end costs as
 // much as several (us a call as passes, and in brackets with put-off updates: 1 iteration 1900^2 41 (71),
 // 4096^2 100 (217); 8 iterations 98 (103) and 280 (317), 10 116 (112) and 333 (333)).
-constexpr int kFewIters = 8;
+// One or two are a launch each: the cooperative launch alone takes 3 us more.
+constexpr int kFewIters = 8, kLeastPasses = 3;
 
 // All iterations as passes, in one cooperative launch.  ran = false: nothing launched.
 tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, cudaStream_t st, bool& ran)
@@ -1699,10 +1701,11 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     TCV_CUDA(cudaMemsetAsync(a.state, 0, w.zeroed, st));
     bool ran = false;
     tcv_status s = TCV_OK;
-    if (g_hog_strategy != TCV_HOGBOM_PER_LAUNCH) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
-    if (s == TCV_OK && !ran && (g_hog_strategy == TCV_HOGBOM_PERSISTENT || (g_hog_strategy == TCV_HOGBOM_AUTO && niters <= kFewIters)))
+    const bool any = g_hog_strategy == TCV_HOGBOM_AUTO, passes = g_hog_strategy == TCV_HOGBOM_PERSISTENT;
+    if (any || passes) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
+    if (s == TCV_OK && !ran && (passes || (any && niters >= kLeastPasses && niters <= kFewIters)))
         s = deconvolve_passes(a, d_dirty, niters, st, ran);
-    if (s == TCV_OK && !ran && g_hog_strategy == TCV_HOGBOM_AUTO && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
+    if (s == TCV_OK && !ran && any && niters > kFewIters && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
         s = deconvolve_deferred(a, w, d_dirty, niters, st, ran);
     if (s != TCV_OK || ran) return s;
     TCV_CHECK(first_scans(a, d_dirty, st));
