@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kHogThreads) hog_scan_kernel(const float* __re
 
 // subtractPSF (HogbomGolden.cc:99-124) over this CTA's share of the image, and the scan of the
 // updated values: returns the CTA-thread's candidate key (0 if it saw no pixel) and value.
-// kVec: width a multiple of 4 and the residual 16-byte aligned (float4 residual I/O).
+// kVec: width a multiple of 4 and the residual 16-byte aligned (float4 residual I/O).  Whole rows per CTA.
 template <bool kVec>
 __device__ __forceinline__ unsigned long long iter_body(const HogArgs& a, unsigned int ppos, float peak,
                                                         unsigned int psf_pos, float& bv_out,
@@ -275,22 +275,40 @@ __device__ __forceinline__ unsigned long long iter_body(const HogArgs& a, unsign
             }
         }
     } else {
-        const long long per = (a.n + a.nblocks - 1) / a.nblocks;
-        const long long lo = per * blockIdx.x, hi = min(a.n, lo + per);
-        for (long long i = lo + threadIdx.x; i < hi; i += kHogThreads) {
-            const unsigned ui = unsigned(i);  // n < 2^32
-            const int y = int(ui / unsigned(W)), x = int(ui - unsigned(y) * unsigned(W));
-            float r = a.residual[i];
-            const int prow = y - diffy;
-            if (y >= starty && y <= stopy && x >= startx && x <= stopx) {
-                if (prow >= 0 && prow < P) {
-                    r = __fsub_rn(r, __fmul_rn(t, a.psf[(long long)prow * P + (x - diffx)]));
-                    a.residual[i] = r;
-                } else if (x == startx) {
-                    ++skipped;
+        // the same by single pixels
+        constexpr int U = 8;
+        const int rows_per = (W + a.nblocks - 1) / a.nblocks;
+        const int r0 = int(blockIdx.x) * rows_per, r1 = min(W, r0 + rows_per);
+        const int nch = (W + kHogThreads - 1) / kHogThreads;
+        if (threadIdx.x == 0)
+            for (int y = r0; y < r1; ++y)
+                if (y >= starty && y <= stopy && !(y - diffy >= 0 && y - diffy < P)) ++skipped;
+        int y = r0, c = 0;
+        while (y < r1) {
+            float r[U], pv[U];
+            bool sub[U], val[U];
+            unsigned int at[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int x = int(threadIdx.x) + kHogThreads * c, prow = y - diffy;
+                val[u] = y < r1 && x < W;
+                sub[u] = val[u] && y >= starty && y <= stopy && prow >= 0 && prow < P && x >= startx && x <= stopx;
+                at[u] = unsigned(y) * unsigned(W) + unsigned(x);  // n < 2^32
+                r[u] = val[u] ? __ldcg(a.residual + at[u]) : 0.f;
+                pv[u] = sub[u] ? __ldg(a.psf + ((long long)prow * P + (x - diffx))) : 0.f;
+                if (++c == nch) {
+                    c = 0;
+                    ++y;
                 }
             }
-            track(r, ui);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (sub[u]) {
+                    r[u] = __fsub_rn(r[u], __fmul_rn(t, pv[u]));
+                    __stcg(a.residual + at[u], r[u]);
+                }
+                if (val[u]) track(r[u], at[u]);
+            }
         }
     }
     const unsigned long long best =
@@ -326,7 +344,7 @@ __global__ void __launch_bounds__(kHogThreads, 4) hog_iter_kernel(HogArgs a, int
         model_update(a, it, ppos, peak);
         st->done = it + 1;
     }
-    if (kVec && it > 0) {
+    if (it > 0) {
         // rows wholly outside this iteration's PSF overlap do not change: the CTA's candidate from
         // an earlier iteration (same row partition; iteration 0 always scans, after the image
         // scan's pixel partition) still holds, so it is left as it is without reading the rows
@@ -1302,6 +1320,13 @@ __global__ void __launch_bounds__(kHogThreads, kCtas) hog_pass_kernel(HogArgs a,
     __shared__ int ok;
     unsigned int ppos = own ? __ldcg(&st->win_next) : key_index(__ldcg(&st->win_key[0]));
     float peak = own ? __ldcg(&st->val_next) : __ldcg(&st->win_val[0]);
+    // the CTA's rows (iter_body's): beyond L2, where an update does not reach them its candidate stays as it is
+    // and they are not read (4096^2 with a PSF of half the width 21.0 -> 18.8 us an iteration; the test alone
+    // costs 2048^2 0.15)
+    const int W = a.width, P = a.psf_width, py = int(psf_pos / unsigned(P));
+    const int rows = (W + a.nblocks - 1) / a.nblocks, r0 = int(blockIdx.x) * rows, r1 = min(W, r0 + rows);
+    unsigned long long best = 0;
+    float bv = 0.f;
     int it = it0;
     for (; it < it1; ++it) {
         if (fabsf(peak) < a.threshold) {  // every CTA holds the same winner: all stop here
@@ -1312,11 +1337,13 @@ __global__ void __launch_bounds__(kHogThreads, kCtas) hog_pass_kernel(HogArgs a,
             model_update(a, it, ppos, peak);
             st->done = it + 1;
         }
-        float bv;
-        unsigned long long skipped;
-        unsigned long long best = iter_body<kVec>(a, ppos, peak, psf_pos, bv, skipped);
-        if (skipped) atomicAdd(&st->skipped_rows, skipped);
-        best = block_max(best, bv);
+        const int ry = kCtas > 2 ? int(ppos / unsigned(W)) : 0;
+        if (kCtas == 2 || it == it0 || (r1 > ry - py && r0 <= ry + (P - py - 1))) {
+            unsigned long long skipped;
+            best = iter_body<kVec>(a, ppos, peak, psf_pos, bv, skipped);
+            if (skipped) atomicAdd(&st->skipped_rows, skipped);
+            best = block_max(best, bv);
+        }
         unsigned long long* keys = a.keys + (it & 1) * a.nblocks;
         float* vals = a.vals + (it & 1) * a.nblocks;
         if (threadIdx.x == 0) {
@@ -1540,9 +1567,13 @@ int lead_ctas(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, const DeferArg
 // the hot blocks (0: never; nothing else): 2048^2, 5 sources 0 13.0, 12 8.24, 6 8.22; 60 sources 0 9.07, 12
 // 9.05, 6 8.30, 4 8.42; 40 sources, 300 iterations 0 7.36, 6 7.40, 4 8.0.  2600^2, 20 sources 0 9.03, 8 9.02,
 // 6 11.5.  4096^2, 5 sources 0 35.9, 24 21.9, 12 21.9; 60 sources 0 19.5, 24 19.5, 12 21.4, 8 27.5.
-PassLimits pass_limits(long long n, int blocks)
+// By single pixels (an odd width) a pass takes nearly twice as long: where blocks are small only twice as many
+// hot blocks count (ms of 1000 iterations by that number times 1, 2, 3, never: 60 sources 2049^2 12.9, 9.4,
+// 9.4, 9.4, 2601^2 19.8, 12.4, 12.4, 12.4; noise 2049^2 15.1, 15.1, 15.0, 33.0, 4095^2 44.1, 44.0, 44.0, 59.1).
+PassLimits pass_limits(long long n, int blocks, bool singles)
 {
-    const int hot = int(2 + (n >> 20));
+    const int hot = int(2 + (n >> 20)), most = 0x7fffffff;
+    if (singles) return PassLimits{most, most, most, 2 * hot * kLeadIters};
     return PassLimits{blocks / 25, hot * kLeadCtas, blocks * 2 / 5, hot * kLeadIters};
 }
 
@@ -1552,9 +1583,11 @@ struct Passes {
     HogArgs h;
     int ctas;
 };
+bool whole_float4s(const HogArgs& h) { return h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0; }
+
 tcv_status passes_of(const HogArgs& h, Passes& p)
 {
-    const bool vec = h.width % 4 == 0 && reinterpret_cast<uintptr_t>(h.residual) % 16 == 0;
+    const bool vec = whole_float4s(h);
     const bool large = (h.n + (long long)h.psf_width * h.psf_width) * 4 > (64ll << 20);
     p.kernel = large ? (vec ? reinterpret_cast<const void*>(hog_pass_kernel<true, 3>)
                             : reinterpret_cast<const void*>(hog_pass_kernel<false, 3>))
@@ -1580,8 +1613,9 @@ tcv_status launch_passes(Passes& p, PassLimits lim, int from, int to, cudaStream
 // Iterations up to which a call is passes from the start: bringing all blocks up to date at its end costs as
 // much as several (us a call as passes, and in brackets with put-off updates: 1 iteration 1900^2 41 (71),
 // 4096^2 100 (217); 8 iterations 98 (103) and 280 (317), 10 116 (112) and 333 (333)).
-// One or two are a launch each: the cooperative launch alone takes 3 us more.
-constexpr int kFewIters = 8, kLeastPasses = 3;
+// By single pixels up to three (2049^2 76 and 91, 2601^2 123 and 127; four 143 and 130).  One or two are a
+// launch each: the cooperative launch alone takes 3 us more.
+constexpr int kFewIters = 8, kFewSingle = 3, kLeastPasses = 3;
 
 // All iterations as passes, in one cooperative launch.  ran = false: nothing launched.
 tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, cudaStream_t st, bool& ran)
@@ -1632,6 +1666,7 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
     const int most = std::min(nb, sms * std::max(1, per_sm));
     Passes passes;  // may take over
     TCV_CHECK(passes_of(h, passes));
+    const PassLimits lim = pass_limits(h.n, nb, !whole_float4s(h) && a.lb == 5);
     cudaLaunchAttribute attrs[2] = {attr, {}};
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1648,7 +1683,7 @@ tcv_status deconvolve_deferred(const HogArgs& h, const HogWork& w, const float* 
         const int to = std::min(niters, it + kLeadIters);
         // all blocks are up to date; from the start to the end (the arrivals have to fit 32 bits)
         if (passes.ctas && it == base)
-            TCV_CHECK(launch_passes(passes, pass_limits(h.n, nb), it, std::min(niters, it == 0 ? 1 << 20 : it + kRing), st));
+            TCV_CHECK(launch_passes(passes, lim, it, std::min(niters, it == 0 ? 1 << 20 : it + kRing), st));
         TCV_CUDA(cudaLaunchKernelEx(&cfg, hog_lead_kernel, a, it, to, base));
         const int all = to == niters || to - base == kRing;
         TCV_CUDA(cudaLaunchKernelEx(&apply, hog_apply_kernel, a, base, all));
@@ -1701,15 +1736,16 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     TCV_CUDA(cudaMemsetAsync(a.state, 0, w.zeroed, st));
     bool ran = false;
     tcv_status s = TCV_OK;
+    const int few = whole_float4s(a) ? kFewIters : kFewSingle;
     const bool any = g_hog_strategy == TCV_HOGBOM_AUTO, passes = g_hog_strategy == TCV_HOGBOM_PERSISTENT;
     if (any || passes) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
-    if (s == TCV_OK && !ran && (passes || (any && niters >= kLeastPasses && niters <= kFewIters)))
+    if (s == TCV_OK && !ran && (passes || (any && niters >= kLeastPasses && niters <= few)))
         s = deconvolve_passes(a, d_dirty, niters, st, ran);
-    if (s == TCV_OK && !ran && any && niters > kFewIters && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
+    if (s == TCV_OK && !ran && any && niters > few && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
         s = deconvolve_deferred(a, w, d_dirty, niters, st, ran);
     if (s != TCV_OK || ran) return s;
     TCV_CHECK(first_scans(a, d_dirty, st));
-    const bool vec = width % 4 == 0 && reinterpret_cast<uintptr_t>(d_residual) % 16 == 0;
+    const bool vec = whole_float4s(a);
     for (int it = 0; it < niters; ++it) {
         if (vec)
             hog_iter_kernel<true><<<a.nblocks, kHogThreads, 0, st>>>(a, it);
