@@ -81,12 +81,14 @@ struct TabC64 {
     static constexpr bool kReal = false;
     using elem = float2;
     __device__ __forceinline__ static float2 load(const elem* p) { return __ldg(p); }
+    __device__ __forceinline__ static float2 value(elem u) { return u; }  // of an entry loaded as it is stored
 };
 struct TabR32 {
     static constexpr int kMinBlocks = 4;
     static constexpr bool kReal = true;
     using elem = float;
     __device__ __forceinline__ static float2 load(const elem* p) { return make_float2(__ldg(p), 0.f); }
+    __device__ __forceinline__ static float2 value(elem u) { return make_float2(u, 0.f); }
 };
 struct TabCBF16 {
     static constexpr int kMinBlocks = 3;
@@ -95,6 +97,10 @@ struct TabCBF16 {
     __device__ __forceinline__ static float2 load(const elem* p)
     {
         const u32 u = __ldg(p);
+        return value(u);
+    }
+    __device__ __forceinline__ static float2 value(elem u)
+    {
         return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
     }
 };
@@ -107,6 +113,7 @@ struct TabRBF16 {
         const u32 u = __ldg(p);
         return make_float2(__uint_as_float(u << 16), 0.f);
     }
+    __device__ __forceinline__ static float2 value(elem u) { return make_float2(__uint_as_float(u32(u) << 16), 0.f); }
 };
 
 // acc += a * b (complex), FP32 fused multiply-adds issued as paired FMAs (one instruction for the

@@ -152,7 +152,9 @@ grid_slice_kernel(const float2* __restrict__ data, const typename Tab::elem* __r
                     for (int e = 0; e < m; e += 32) {
                         u32 bits = __ballot_sync(0xffffffffu, e + lane < m && ((sm_mask[buf][e + lane] >> warp) & 1u));
                         while (bits) {
-                            float2 cv[kDeep][kRows], dv[kDeep];
+                            // entries as they are stored: converting one would wait for its load
+                            typename Tab::elem cv[kDeep][kRows];
+                            float2 dv[kDeep];
                             u32 has = 0;  // rows that this lane's column of the footprint has, kRows bits per sample
 #pragma unroll
                             for (int b = 0; b < kDeep; ++b) {
@@ -168,14 +170,14 @@ grid_slice_kernel(const float2* __restrict__ data, const typename Tab::elem* __r
                                 for (int r = 0; r < kRows; ++r)
                                     if (unsigned(dx) < unsigned(s) && unsigned(dy + r) < unsigned(s)) {
                                         has |= 1u << (b * kRows + r);
-                                        cv[b][r] = Tab::load(ctab + (ci + r * s));
+                                        cv[b][r] = __ldg(ctab + (ci + r * s));
                                     }
                             }
 #pragma unroll
                             for (int b = 0; b < kDeep; ++b)
 #pragma unroll
                                 for (int r = 0; r < kRows; ++r)
-                                    if ((has >> (b * kRows + r)) & 1u) cmac<Tab::kReal>(acc[r], dv[b], cv[b][r]);
+                                    if ((has >> (b * kRows + r)) & 1u) cmac<Tab::kReal>(acc[r], dv[b], Tab::value(cv[b][r]));
                         }
                     }
                 }

@@ -20,12 +20,14 @@ struct TabCF16 {
     static constexpr bool kReal = false;
     using elem = __half2;
     __device__ __forceinline__ static float2 load(const elem* p) { return __half22float2(__ldg(p)); }
+    __device__ __forceinline__ static float2 value(elem u) { return __half22float2(u); }
 };
 struct TabRF16 {
     static constexpr int kMinBlocks = 4;
     static constexpr bool kReal = true;
     using elem = __half;
     __device__ __forceinline__ static float2 load(const elem* p) { return make_float2(__half2float(__ldg(p)), 0.f); }
+    __device__ __forceinline__ static float2 value(elem u) { return make_float2(__half2float(u), 0.f); }
 };
 
 // ------------------------------------------------------------------------------------------

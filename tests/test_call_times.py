@@ -121,3 +121,29 @@ def test_new_plan_of_a_short_track(tcv, cuda_ok, run, part):
 
     both, one = _us(once(plans[0]), once(plans[1]))
     assert both <= 1.1 * one, (both, one)
+
+
+@pytest.mark.parametrize("form", ["rbf16", "rf16"])
+def test_gridding_in_slices_by_table_form(tcv, cuda_ok, form):
+    """A few busy tiles are gridded in slices with several samples' entries in flight; a 16-bit entry is half
+    a float one's bytes.  Bar: a tenth over the float table's time."""
+    import numpy as np
+    import torch
+
+    from tconvolve import _lib, raw
+
+    rng, n, support, g, planes = np.random.default_rng(2), 60000, 32, 1024, 9
+    s = 2 * support + 1
+    c = torch.zeros(64 * planes * s * s, dtype=torch.complex64, device="cuda")
+    c.real.uniform_(-1.0, 1.0)
+    d = lambda a: torch.from_numpy(a.astype(np.int32)).cuda()  # noqa: E731
+    plan = raw.Plan(d(160 + rng.integers(0, 700, n)), d(128 + rng.integers(0, 700, n)),
+                    d(rng.integers(0, 64 * planes, n) * s * s), support, g, c.numel())
+    vis, grid = torch.ones(n, dtype=torch.complex64, device="cuda"), torch.zeros(g * g, dtype=torch.complex64, device="cuda")
+
+    def of(name):
+        tab, scale, _ = raw.convert_c(c, _lib.CTYPE_BY_NAME[name])
+        return lambda: plan.grid(vis, tab, _lib.CTYPE_BY_NAME[name], grid, scale)
+
+    half, full = _us(of(form), of("r32"))
+    assert half <= 1.1 * full, (half, full)
