@@ -152,12 +152,13 @@ struct tcv_plan {
 namespace tcv {
 
 // Work-unit sizes (gridding, degridding) of a plan whose both passes are sample-parallel, from the pairs
-// (of samples or footprints, with tiles) in its cells: the tuning's, or smaller where it would give less
-// than some four units per warp group of a gridding launch (888 in three CTAs per SM) or ten per CTA of a
-// degridding one (740): 77 k samples of the spectral run 129 -> 65 us gridding, 62 -> 43 degridding, 383 k
-// 177 -> 139.  Smaller still costs a unit's tile again: continuum degridding 2.07 ms with 37 footprints a
-// unit, 1.56 ms with 128.  Not below what the unit lists and partial tiles, made for the most pairs
-// that the samples can have, have room for.
+// (of samples or footprints, with tiles) in its cells: the tuning's, or smaller where it would give too few
+// units: four per warp group of a gridding launch (888 in three CTAs per SM) for footprints, one for samples,
+// ten per CTA of a degridding one (740): 77 k samples of the spectral run 129 -> 65 us gridding, 62 -> 43
+// degridding.  Smaller still costs a unit's tile again (continuum degridding 2.07 ms with 37 footprints a
+// unit, 1.56 ms with 128) and a rounding for each unit of a cell (continuum run, 218 k samples, four and one
+// per warp group: 8.2e-8 and 6.6e-8 off, 349 and 324 us).  Not below what the unit lists and partial
+// tiles, made for the most pairs that the samples can have, have room for.
 __device__ __forceinline__ void unit_sizes(const PlanGeom& g, uint32_t pairs, uint32_t* sizes)
 {
     const unsigned long long most = (unsigned long long)(g.n) * g.max_tiles;
@@ -165,7 +166,7 @@ __device__ __forceinline__ void unit_sizes(const PlanGeom& g, uint32_t pairs, ui
         const uint32_t room = uint32_t((pairs * (unsigned long long)(s) + most - 1) / most), want = pairs / units;
         return s ? max(max(32u, room), min(s, want)) : 0u;
     };
-    sizes[0] = size(uint32_t(g.split), 4096u);
+    sizes[0] = size(uint32_t(g.split), g.uniq ? 4096u : 1024u);
     sizes[1] = size(uint32_t(g.dsplit), 8192u);
 }
 

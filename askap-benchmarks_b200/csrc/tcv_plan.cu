@@ -1357,8 +1357,8 @@ PlanGeom make_geom_var(int64_t n, const int32_t* s_size, const int32_t* c_off0, 
         // there are enough samples: fewer of a track share few footprints, and pay the longer sort and the
         // lists, which look over as many cells as a footprint can touch tiles, for nothing.  us, by
         // sample and by footprint, binning, gridding, degridding: spectral run (4 tiles) 77 k samples 85
-        // 65 43 and 176 69 45, 262 k 104 102 79 and 211 102 83, 765 k 157 241 185 and 280 187 148; continuum run
-        // (15) 109 k 116 232 210 and 314 270 220, 544 k 258 600 537 and 387 605 513, 2.2 M 716 1516 1529 and
+        // 65 43 and 176 69 45, 262 k 104 101 79 and 211 102 83, 765 k 157 236 185 and 280 187 148; continuum run
+        // (15) 109 k 115 235 208 and 314 270 220, 490 k 241 594 495 and 385 576 481, 2.2 M 716 1516 1529 and
         // 620 1344 1031.  The line lies where a kept plan's passes take as long either way.
         g.u_coff_bits = bits_for(uint64_t(c_len - 1));
         g.u_rank_bits = bits_for(uint64_t(width_ranks(s_size, n_planes, nullptr) - 1));
