@@ -54,12 +54,13 @@ GridArgs make_args(const tcv_plan* p, int grp, float c_scale, float2* grid)
 // that adds its samples in order, group after group, so the sums are the same, bit for bit; per
 // update it costs more instructions, which a device that is mostly idle has to spare.
 // Whole-cell plans take it when every plane group has at most 1.2 busy tiles per SM (plan_mode_kernel):
-// 169 tiles gain (0.72 -> 0.49 ms), 289 do not (0.38 and 0.51 ms).  The samples above take 0.162 ms,
-// 160 k samples of 29^2 on 9 tiles 4.3 ms (18.8 whole).  Six samples at four CTAs an SM: eight at three
+// 169 tiles gain (0.72 -> 0.49 ms; 60 k samples of 65^2 on 144, a bfloat16 table, 0.45 -> 0.39), 289 do not
+// (0.38 and 0.51 ms).  The samples above take 0.162 ms, 160 k samples of 29^2 on 9 tiles 4.3 ms (18.8 whole).  Six samples at four CTAs an SM: eight at three
 // take 0.165 and 4.1 ms but 0.55 ms on 169 tiles, four at four 0.19, 4.7 and 0.52.
 // A kernel of its own: inside grid_tile_kernel it cost the other path 1.4 % (registers).  It is launched
 // behind the tile kernels, whose ranges are then empty, without the usual gap (it waits for them
-// itself): where it is not taken that costs 0.3 us a pass, an ordinary launch before them 4 us.
+// itself): where it is not taken that costs about 1 us a pass (65 k samples of 45^2 157.3 -> 158.4 us, 160 k
+// of 129^2 1238.1 -> 1239.3), an ordinary launch before them 4 us.
 template <class Tab, int kR, bool kVar>
 __global__ void __launch_bounds__(kTileThreads, 4)
 grid_slice_kernel(const float2* __restrict__ data, const typename Tab::elem* __restrict__ ctab,

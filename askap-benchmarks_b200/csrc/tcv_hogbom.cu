@@ -13,9 +13,9 @@
 // HogbomGolden.cc:108); that is kept.  Where it points outside the PSF (only when the PSF peak is
 // off the diagonal) the reference reads out of bounds; here those rows are skipped and counted.
 //
-// Three forms, chosen by size (tcv_hogbom_deconvolve); all give the same bits.
+// Four forms, chosen by size and image (tcv_hogbom_deconvolve); all give the same bits.
 //
-// Up to 2048 x 2048 where the device holds enough clusters (1792 here; hog_resident_kernel): the residual
+// Up to 1792 x 1792 (as many clusters as the device holds decide it; hog_resident_kernel): the residual
 // stays in registers, one cooperative launch.
 //
 // Larger images: updates are put off.  The image is cut into blocks of at least 32 x 32 pixels, and
@@ -32,11 +32,14 @@
 // (bounds, the hot blocks' loads, the exchange: 5 us at 4096^2), not a pass over the image.
 // hog_apply_kernel follows on the whole device: it brings blocks near the peak up to date, and
 // every kRing iterations and at the end all blocks (7.7 us an iteration at 4096^2, most of it the PSF
-// windows from L2).  Where many blocks stay hot, hog_pass_kernel takes over.  A pixel's updates are applied in iteration order with the reference's
-// roundings whenever they are applied, so the bits do not depend on the schedule.
+// windows from L2).  A pixel's updates are applied in iteration order with the reference's roundings
+// whenever they are applied, so the bits do not depend on the schedule.
 //
-// Beyond the block table's size (or with TCV_HOGBOM_PER_LAUNCH): a launch per iteration, which
-// subtracts the PSF over its blocks' slices of the image and scans the updated values for the
+// Where many blocks are near the peak, as in an image that an earlier cycle has cleaned, and for a few
+// iterations: a pass over the image per iteration in cooperative launches (hog_pass_kernel).
+//
+// Beyond the block table's size, for one or two iterations (or with TCV_HOGBOM_PER_LAUNCH): a launch per
+// iteration, which subtracts the PSF over its blocks' slices of the image and scans the updated values for the
 // next peak in the same pass, so an iteration reads the residual once, reads the PSF's overlap
 // once and writes the overlap once.  Each block leaves one candidate, a 64-bit key (|value| bits
 // << 32 | ~index: the largest key is the largest magnitude at the smallest index) with its signed
@@ -44,10 +47,11 @@
 // winner that the next launch reads.  The stop test (|peak| < threshold) is taken on the device:
 // later launches see the flag and return.
 //
-// Measured on one B200, us an iteration, and in brackets with one pass over the image per iteration
-// (in one cooperative launch up to 48 MiB of images, all CTAs waiting on one counter; a launch
-// each beyond): 128^2 1.15, 223^2 1.5 (8.0), 1024^2 3.2 (4.64), 1700^2 7.2 (7.4), 1900^2 6.4 (8.2), 4096^2 12.9 (27.0);
-// put-off updates with 5 sources cleaned to noise 1900^2 8.1 (8.0), 4096^2 21.7 (26.5).
+// Measured on one B200, us an iteration of 1000 (20 sources), and in brackets with one pass over the image per
+// iteration (in one cooperative launch up to 48 MiB of images, a launch each beyond): 128^2 1.11 (10.1), 223^2
+// 1.5 (7.9), 1024^2 3.2 (4.7), 1700^2 7.4 (7.4), 1900^2 6.3 (8.35), 2600^2 7.9 (15.9), 4096^2 12.8 (28.0); 5 sources cleaned
+// to noise 1900^2 8.0 (8.1), 4096^2 20.7 (26.6); an image cleaned before 1900^2 8.3 (8.05), 2048^2 8.5 (8.1), 2600^2
+// 11.7 (14.2), 4096^2 19.4 (21.9).
 #include "tcv_internal.cuh"
 
 #include <cooperative_groups.h>
@@ -414,8 +418,8 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long k)
 // Images that fit the register files: the residual stays in registers for all iterations.  Each CTA
 // owns whole rows, a thread up to kRowsT x kChunks pixels of them; an iteration loads the PSF (from
 // L2), updates, and finds the CTA's candidate; the CTAs of a cluster send theirs to its first CTA
-// through distributed shared memory, the first CTAs exchange theirs through global memory (16-18
-// words instead of one per CTA: all CTAs polling all CTAs' words kept the few L2 lines they lie on
+// through distributed shared memory, the first CTAs exchange theirs through global memory (a
+// word a cluster instead of one per CTA: all CTAs polling all CTAs' words kept the few L2 lines they lie on
 // busy and took 4 us), and each hands the winner to its cluster.
 // ------------------------------------------------------------------------------------------
 constexpr int kResThreads = 512;
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(kResThreads, 1) hog_resident_kernel(ResArgs a,
         auto on = [&](int i) { return y0 + i >= ya && y0 + i <= yb; };
         // the whole iteration's PSF values in flight at once: the later rows' by asynchronous copies to
         // this thread's own places in shared memory, the first rows' in registers
-        // (2048^2: 7.6 us an iteration with half of them loaded after the other half, 6.35 so)
+        // (half of them loaded after the other half cost a fifth more at 16 rows of four columns)
         float pv[kDirect][kChunks], top = -1.f;  // only the largest |value| is kept here
 #pragma unroll
         for (int j = 0; j < kChunks; ++j) {
