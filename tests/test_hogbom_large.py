@@ -117,3 +117,30 @@ def test_passes_take_over(tcv, orc, cuda_ok, width, bright, niters, threshold):
     psf = synthetic_psf(1051)
     dirty[200:1251, 500:1551] += np.float32(bright) * psf
     _check(orc, dirty, psf, niters, threshold)
+
+
+# a captured call replays as it ran: launches each, passes, put-off updates, passes that take over
+@pytest.mark.parametrize("width,niters,noise", [(2100, 2, 0.0), (2100, 5, 0.0), (2100, 150, 0.0), (2100, 20, 1.0), (2099, 20, 0.0)])
+def test_captured_call(tcv, cuda_ok, width, niters, noise):
+    import torch
+
+    from tconvolve.hogbom import Workspace, deconvolve_device
+    from tconvolve.workload import synthetic_psf
+
+    host = np.random.default_rng(7).standard_normal((width, width)).astype(np.float32)
+    d = torch.from_numpy((host * np.float32(noise) if noise else _bright(w=width)).ravel().copy()).cuda()
+    p = torch.from_numpy(synthetic_psf(width).ravel()).cuda()
+    m, r, ws = torch.zeros_like(d), torch.empty_like(d), Workspace(width)
+    deconvolve_device(d, width, p, width, m, r, niters, 0.1, 0.0, work=ws)
+    want = (m.clone(), r.clone())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        m.zero_()
+        deconvolve_device(d, width, p, width, m, r, niters, 0.1, 0.0, work=ws)
+    for _ in range(2):
+        m.fill_(3.0)
+        r.fill_(3.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(m, want[0]) and torch.equal(r, want[1])
+        assert ws.result()["done"] == niters
