@@ -1621,6 +1621,10 @@ tcv_status launch_passes(Passes& p, PassLimits lim, int from, int to, cudaStream
 // launch each: the cooperative launch alone takes 3 us more.
 constexpr int kFewIters = 8, kFewSingle = 3, kLeastPasses = 3;
 
+// From this width on a single iteration is a launch at the resident sizes too (alone, us: 1024^2 34 and 37 in the
+// resident form, 1500^2 38 and 41; 512^2 32 and 31).
+constexpr int kSingleWidth = 1024;
+
 // All iterations as passes, in one cooperative launch.  ran = false: nothing launched.
 tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, cudaStream_t st, bool& ran)
 {
@@ -1742,7 +1746,8 @@ tcv_status tcv_hogbom_deconvolve(const float* d_dirty, int width, const float* d
     tcv_status s = TCV_OK;
     const int few = whole_float4s(a) ? kFewIters : kFewSingle;
     const bool any = g_hog_strategy == TCV_HOGBOM_AUTO, passes = g_hog_strategy == TCV_HOGBOM_PERSISTENT;
-    if (any || passes) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
+    const bool single = any && niters == 1 && width >= kSingleWidth;
+    if ((any || passes) && !single) s = deconvolve_resident(a, w, d_dirty, niters, st, ran);
     if (s == TCV_OK && !ran && (passes || (any && niters >= kLeastPasses && niters <= few)))
         s = deconvolve_passes(a, d_dirty, niters, st, ran);
     if (s == TCV_OK && !ran && any && niters > few && width <= kDeferMaxWidth && psf_width <= kDeferMaxWidth)
