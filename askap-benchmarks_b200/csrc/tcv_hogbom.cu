@@ -1631,8 +1631,8 @@ tcv_status deconvolve_passes(const HogArgs& h, const float* dirty, int niters, c
     ran = false;
     Passes p;
     TCV_CHECK(passes_of(h, p));
-    // the arrivals reach niters x CTAs: within 32 bits
-    if (p.ctas < 1 || uint64_t(niters) * uint64_t(p.ctas) >= 1ull << 32) return TCV_OK;
+    // the arrivals reach niters x CTAs (and those withheld): within 32 bits
+    if (p.ctas < 1 || uint64_t(niters) * uint64_t(p.ctas) + g_withheld >= 1ull << 32) return TCV_OK;
     TCV_CHECK(first_scans(h, dirty, st));
     ran = true;
     return niters > 0 ? launch_passes(p, PassLimits{-1, -1, -1, -1}, 0, niters, st) : TCV_OK;

@@ -587,8 +587,8 @@ tcv_status tcv_hogbom_deconvolve(const float *d_dirty, int width, const float *d
  * cooperative launch of all iterations with the residual in registers, the CTAs meeting once per
  * iteration; larger ones with updates put off until a block of pixels could hold the next peak (a launch
  * of one cluster and a device-wide one per 16 iterations), or, where too many blocks are near the peak,
- * as cooperative launches of a pass over the image per iteration; images or PSFs over 16384 wide with one
- * launch per iteration.  PERSISTENT takes a cooperative launch of all iterations at any size, PER_LAUNCH
+ * as cooperative launches of a pass over the image per iteration; images or PSFs over 16384 wide, and one
+ * or two iterations of large images, with one launch per iteration.  PERSISTENT takes a cooperative launch of all iterations at any size, PER_LAUNCH
  * one launch per iteration.  All waits are bounded (below).  Results are identical. */
 enum { TCV_HOGBOM_AUTO = 0, TCV_HOGBOM_PER_LAUNCH = 1, TCV_HOGBOM_PERSISTENT = 2 };
 void tcv_hogbom_set_strategy(int strategy);
